@@ -241,73 +241,52 @@ __global__ void __launch_bounds__(PCG_THREADS) pcg_bsr_kernel(BsrPcgArgs<V> P) {
     rz_p = fma(bi, z, rz_p);
     bb_p = fma(bi, bi, bb_p);
   }
+  __shared__ CgScalars<A> S;
   block_partials<A>(bb_p, rz_p, 2, P.partials, S_RR, S_RZ);
-  double red[REDUCE_MAX_NV];
-  if (!grid_reduce_sync(P.bar, P.st, P.limit_ns, P.partials, P.totals, S_RR, 2, red)) return;
-  A rz = (A)red[1];
-  const double bnorm = sqrt(red[0]);
+  if (!group_reduce_apply(P.bar, P.st, P.limit_ns, P.partials, P.totals, S_RR, 2, gridDim.x,
+                          [&](const double* t) { cg_begin(S, t); }))
+    return;
   long long iters = 0;
-  double residual = bnorm;
-  int status = AXIA_OK;
-  if (bnorm >= 1e-30) {
-    for (long long it = 0; it < P.max_iter; ++it) {
-      iters = it + 1;
-      A pq_p = 0;
-      for (int base = gwarp * RPW; base < n_nodes; base += nwarps * RPW) {
-        const int a = base + grp;
-        A y0, y1, y2;
-        bsr_row<V, A, 1, L>(a, sl, P.M, P.p, y0, y1, y2);
-        if (a < n_nodes && sl == 0) {
-          P.q[3 * a] = (V)y0;
-          P.q[3 * a + 1] = (V)y1;
-          P.q[3 * a + 2] = (V)y2;
-          pq_p = fma((A)P.p[3 * a], y0, pq_p);
-          pq_p = fma((A)P.p[3 * a + 1], y1, pq_p);
-          pq_p = fma((A)P.p[3 * a + 2], y2, pq_p);
-        }
+  for (long long it = 0; !S.stop && it < P.max_iter; ++it) {
+    iters = it + 1;
+    A pq_p = 0;
+    for (int base = gwarp * RPW; base < n_nodes; base += nwarps * RPW) {
+      const int a = base + grp;
+      A y0, y1, y2;
+      bsr_row<V, A, 1, L>(a, sl, P.M, P.p, y0, y1, y2);
+      if (a < n_nodes && sl == 0) {
+        P.q[3 * a] = (V)y0;
+        P.q[3 * a + 1] = (V)y1;
+        P.q[3 * a + 2] = (V)y2;
+        pq_p = fma((A)P.p[3 * a], y0, pq_p);
+        pq_p = fma((A)P.p[3 * a + 1], y1, pq_p);
+        pq_p = fma((A)P.p[3 * a + 2], y2, pq_p);
       }
-      block_partials<A>(pq_p, A(0), 1, P.partials, S_PQ, S_PQ);
-      double red[REDUCE_MAX_NV];
-      if (!grid_reduce_sync(P.bar, P.st, P.limit_ns, P.partials, P.totals, S_PQ, 1, red)) return;
-      const A pq = (A)red[0];
-      if (!(fabs((double)pq) >= 1e-30)) {
-        status = AXIA_ERR_ZERO_PIVOT;
-        break;
-      }
-      const A alpha = rz / pq;
-      A rr_p = 0, rzn_p = 0;
-      for (int i = tid; i < nd; i += nth) {
-        P.x[i] = fma(alpha, P.p[i], P.x[i]);
-        const V ri = fma(-alpha, P.q[i], P.r[i]);
-        P.r[i] = ri;
-        rr_p = fma(ri, ri, rr_p);
-        rzn_p = fma(ri, ri * P.dinv[i], rzn_p);
-      }
-      block_partials<A>(rr_p, rzn_p, 2, P.partials, S_RR, S_RZ);
-      if (!grid_reduce_sync(P.bar, P.st, P.limit_ns, P.partials, P.totals, S_RR, 2, red)) return;
-      const A rzn = (A)red[1];
-      residual = sqrt(red[0]);
-      if (!isfinite(residual)) {
-        status = AXIA_ERR_NONFINITE;
-        break;
-      }
-      if (residual <= P.tol * bnorm) break;
-      const A beta = rzn / rz;
-      rz = rzn;
-      for (int i = tid; i < nd; i += nth) P.p[i] = fma(beta, P.p[i], P.r[i] * P.dinv[i]);
-      if (!grid_sync(P.bar, P.st, P.limit_ns)) return;
     }
-    if (status == AXIA_OK && residual > P.tol * bnorm * 10.0) status = AXIA_ERR_NOT_CONVERGED;
-  } else {
-    residual = 0.0;
+    block_partials<A>(pq_p, A(0), 1, P.partials, S_PQ, S_PQ);
+    if (!group_reduce_apply(P.bar, P.st, P.limit_ns, P.partials, P.totals, S_PQ, 1, gridDim.x,
+                            [&](const double* t) { cg_alpha(S, t); }))
+      return;
+    if (S.status != AXIA_OK) break;
+    const A alpha = S.alpha;
+    A rr_p = 0, rzn_p = 0;
+    for (int i = tid; i < nd; i += nth) {
+      P.x[i] = fma(alpha, P.p[i], P.x[i]);
+      const V ri = fma(-alpha, P.q[i], P.r[i]);
+      P.r[i] = ri;
+      rr_p = fma(ri, ri, rr_p);
+      rzn_p = fma(ri, ri * P.dinv[i], rzn_p);
+    }
+    block_partials<A>(rr_p, rzn_p, 2, P.partials, S_RR, S_RZ);
+    if (!group_reduce_apply(P.bar, P.st, P.limit_ns, P.partials, P.totals, S_RR, 2, gridDim.x,
+                            [&](const double* t) { cg_beta(S, t, P.tol); }))
+      return;
+    if (S.status != AXIA_OK || S.stop) break;
+    const A beta = S.beta;
+    for (int i = tid; i < nd; i += nth) P.p[i] = fma(beta, P.p[i], P.r[i] * P.dinv[i]);
+    if (!grid_sync(P.bar, P.st, P.limit_ns)) return;
   }
-  if (blockIdx.x == 0 && threadIdx.x == 0) {
-    P.out->iters = iters;
-    P.out->residual = residual;
-    P.out->bnorm = bnorm;
-    P.out->status = status;
-    P.out->updates = 0;
-  }
+  if (blockIdx.x == 0 && threadIdx.x == 0) cg_out(S, P.out, P.tol, iters, 0);
 }
 
 // FP32 CG on the FP32 node-block matrix with FP64 reliable updates (the
@@ -327,16 +306,19 @@ struct SolveRange {
 };
 
 // The coarse solve of the two-level preconditioner, r_c complete:
-// y = M r_c, and r_c . y reduced over the group.
+// y = M r_c, and r_c . y reduced over the group; the direction's beta (or, for
+// the first direction, the coarse part of r.z) follows on thread 0.
 __device__ __forceinline__ bool coarse_step(const BsrReliableArgs& P, const CoarseArgs& C, const SolveRange& R,
-                                            int gwarp, int nwarps, int lane, float* rz_c) {
+                                            int gwarp, int nwarps, int lane, CgScalars<float>& S, bool first) {
   __shared__ __align__(16) float s_rc[COARSE_MAX];
   const float acc = coarse_solve(C, s_rc, gwarp, nwarps, lane);
   block_partials<float>(acc, 0.f, 1, R.partials, S_RC, S_RC, R.nblk, R.rank);
-  double red[REDUCE_MAX_NV];
-  if (!group_reduce_sync(R.bar, P.st, P.limit_ns, R.partials, R.totals, S_RC, 1, R.nblk, red)) return false;
-  *rz_c = (float)red[0];
-  return true;
+  return group_reduce_apply(R.bar, P.st, P.limit_ns, R.partials, R.totals, S_RC, 1, R.nblk, [&](const double* t) {
+    if (first)
+      S.rz += (float)t[0];
+    else
+      mixed_set_beta(S, S.rzn + (float)t[0]);
+  });
 }
 
 template <int L32, int V32, int L64, int V64, bool COARSE = false, bool SYM = false>
@@ -366,28 +348,23 @@ __device__ __forceinline__ void reliable_body(const BsrReliableArgs& P, const Co
     rz_p = fmaf(ri, z, rz_p);
     bb_p = fma(bi, bi, bb_p);
   }
+  __shared__ CgScalars<float> S;
   block_partials<double>(bb_p, (double)rz_p, 2, partials, S_RR, S_RZ, R.nblk, R.rank);
-  double red[REDUCE_MAX_NV];
-  if (!group_reduce_sync(R.bar, P.st, P.limit_ns, partials, totals, S_RR, 2, R.nblk, red)) return;
-  float rz = (float)red[1];
-  const double bnorm = sqrt(red[0]);
-  double rmax = bnorm, residual = bnorm;
+  if (!group_reduce_apply(R.bar, P.st, P.limit_ns, partials, totals, S_RR, 2, R.nblk,
+                          [&](const double* t) { mixed_begin(S, t); }))
+    return;
   long long iters = 0;
-  int updates = 0, status = AXIA_OK;
-  bool converged = bnorm < 1e-30;
-  if (converged) residual = 0.0;
+  int updates = 0;
   if constexpr (COARSE) {
-    if (!converged) {  // p = D^-1 b + Z M Z^T b
-      float rz_c = 0.f;
+    if (!S.stop) {  // p = D^-1 b + Z M Z^T b
       coarse_restrict(C, P.r32, gwarp, nwarps, lane);
       if (!group_sync(R.bar, P.st, P.limit_ns, R.nblk)) return;
-      if (!coarse_step(P, C, R, gwarp, nwarps, lane, &rz_c)) return;
-      rz += rz_c;
+      if (!coarse_step(P, C, R, gwarp, nwarps, lane, S, true)) return;
       coarse_update_p(C, n0, n1, tid, nth, 0.f, P.r32, P.dinv32, P.p32, true);
       if (!group_sync(R.bar, P.st, P.limit_ns, R.nblk)) return;
     }
   }
-  for (long long it = 0; !converged && it < P.max_iter; ++it) {
+  for (long long it = 0; !S.stop && it < P.max_iter; ++it) {
     iters = it + 1;
     float pq_p = 0.f;
     {
@@ -414,14 +391,11 @@ __device__ __forceinline__ void reliable_body(const BsrReliableArgs& P, const Co
       }
     }
     block_partials<float>(pq_p, 0.f, 1, partials, S_PQ, S_PQ, R.nblk, R.rank);
-    double red[REDUCE_MAX_NV];
-    if (!group_reduce_sync(R.bar, P.st, P.limit_ns, partials, totals, S_PQ, 1, R.nblk, red)) return;
-    const float pq = (float)red[0];
-    if (!(fabsf(pq) >= 1e-30f) || !isfinite(pq)) {
-      status = isfinite(pq) ? AXIA_ERR_ZERO_PIVOT : AXIA_ERR_NONFINITE;
-      break;
-    }
-    const float alpha = rz / pq;
+    if (!group_reduce_apply(R.bar, P.st, P.limit_ns, partials, totals, S_PQ, 1, R.nblk,
+                            [&](const double* t) { mixed_alpha(S, t); }))
+      return;
+    if (S.status != AXIA_OK) break;
+    const float alpha = S.alpha;
     float rr_p = 0.f, rzn_p = 0.f;
     if constexpr (COARSE) {
       coarse_update_restrict(C, alpha, P.x32, P.p32, P.q32, P.r32, P.dinv32, gwarp, nwarps, lane, rr_p, rzn_p);
@@ -435,14 +409,13 @@ __device__ __forceinline__ void reliable_body(const BsrReliableArgs& P, const Co
       }
     }
     block_partials<float>(rr_p, rzn_p, 2, partials, S_RR, S_RZ, R.nblk, R.rank);
-    if (!group_reduce_sync(R.bar, P.st, P.limit_ns, partials, totals, S_RR, 2, R.nblk, red)) return;
-    float rzn = (float)red[1];
-    const double rnorm32 = sqrt(red[0]);
-    if (!isfinite(rnorm32)) {
-      status = AXIA_ERR_NONFINITE;
-      break;
-    }
-    if (rnorm32 <= P.delta * rmax || rnorm32 <= P.tol * bnorm) {
+    if (!group_reduce_apply(R.bar, P.st, P.limit_ns, partials, totals, S_RR, 2, R.nblk, [&](const double* t) {
+          mixed_check(S, t[0], P.tol, P.delta);
+          mixed_rz<COARSE>(S, (float)t[1], !S.update);
+        }))
+      return;
+    if (S.status != AXIA_OK) break;
+    if (S.update) {
       for (int i = i0 + tid; i < nd; i += nth) {
         P.x[i] += (double)P.x32[i];
         P.x32[i] = 0.f;
@@ -471,46 +444,29 @@ __device__ __forceinline__ void reliable_body(const BsrReliableArgs& P, const Co
         }
       }
       block_partials<double>(rr64_p, (double)rz_new_p, 2, partials, S_RR, S_RZ, R.nblk, R.rank);
-      double red[REDUCE_MAX_NV];
-      if (!group_reduce_sync(R.bar, P.st, P.limit_ns, partials, totals, S_RR, 2, R.nblk, red)) return;
+      if (!group_reduce_apply(R.bar, P.st, P.limit_ns, partials, totals, S_RR, 2, R.nblk, [&](const double* t) {
+            mixed_replaced(S, t[0], P.tol);
+            mixed_rz<COARSE>(S, (float)t[1], true);
+          }))
+        return;
       ++updates;
-      residual = sqrt(red[0]);
-      rzn = (float)red[1];
-      rmax = residual;
-      if (!isfinite(residual)) {
-        status = AXIA_ERR_NONFINITE;
-        break;
-      }
-      if (residual <= P.tol * bnorm) {
-        converged = true;
-        break;
-      }
+      if (S.status != AXIA_OK || S.stop) break;
       if constexpr (COARSE) {  // r was replaced: restrict it again
         coarse_restrict(C, P.r32, gwarp, nwarps, lane);
         if (!group_sync(R.bar, P.st, P.limit_ns, R.nblk)) return;
       }
     }
     if constexpr (COARSE) {
-      float rz_c = 0.f;
-      if (!coarse_step(P, C, R, gwarp, nwarps, lane, &rz_c)) return;
-      rzn += rz_c;
+      if (!coarse_step(P, C, R, gwarp, nwarps, lane, S, false)) return;
     }
-    const float beta = rzn / rz;
-    rz = rzn;
+    const float beta = S.beta;
     if constexpr (COARSE)
       coarse_update_p(C, n0, n1, tid, nth, beta, P.r32, P.dinv32, P.p32, false);
     else
       for (int i = i0 + tid; i < nd; i += nth) P.p32[i] = fmaf(beta, P.p32[i], P.r32[i] * P.dinv32[i]);
     if (!group_sync(R.bar, P.st, P.limit_ns, R.nblk)) return;
   }
-  if (status == AXIA_OK && residual > P.tol * bnorm * 10.0) status = AXIA_ERR_NOT_CONVERGED;
-  if (R.rank == 0 && threadIdx.x == 0) {
-    R.out->iters = iters;
-    R.out->residual = residual;
-    R.out->bnorm = bnorm;
-    R.out->status = status;
-    R.out->updates = updates;
-  }
+  if (R.rank == 0 && threadIdx.x == 0) cg_out(S, R.out, P.tol, iters, updates);
 }
 
 // FP64 reliable updates: 4 lanes per block row; 2 blocks per load where the

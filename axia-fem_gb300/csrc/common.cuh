@@ -163,13 +163,18 @@ __device__ __forceinline__ bool grid_sync(GridBarrier* bar, DevStatus* st, unsig
 
 // Grid-wide barrier that also reduces.  Every block has stored its partials of
 // nv <= 4 values at partials[(slot0 + k) * nblk + rank]; the last block to
-// arrive sums them with all its threads (one L2 round trip; thread t takes
-// blocks t, t + blockDim.x, ..., then warps and the warp sums in order: a fixed
-// order, so every run gives the same bits) and publishes totals[slot0 + k]
-// before it releases the others.  Same bounded wait as grid_sync.  With res,
-// thread 0 of every block copies the totals into shared memory and every
-// thread gets them in res[0..nv) (one L2 read per block instead of one per
-// warp on a single line); without, threads read totals[] with ld.cg.
+// arrive sums them (one L2 round trip; thread t takes blocks t, t +
+// blockDim.x, ..., then warps and the warp sums in order: a fixed order, so
+// every run gives the same bits) and publishes totals[slot0 + k] before it
+// releases the others.  Same bounded wait as grid_sync.
+//
+// What an iteration needs from the totals (step lengths, norms, branch flags)
+// is computed by `fn(totals)` on thread 0 of every block, which leaves it in
+// shared memory for the block.  Bound: GB300 issues one FP64 warp instruction
+// per SM about every 18 cycles (a dependent one every 63), so a square root and
+// a division of about 20 instructions each, executed by all 16 to 64 warps of
+// an SM, took 6 to 30 us per iteration; on one thread they take 0.6 us.
+// Likewise only the warps that hold partials join the sums.
 constexpr int REDUCE_MAX_NV = 4;
 
 // The last block's part of group_reduce_sync (every thread of the block calls
@@ -179,21 +184,24 @@ static __device__ __noinline__ void reduce_partials_last_block(const double* par
                                                         int slot0, int nv, unsigned nblk) {
   __shared__ double s_sum[REDUCE_MAX_NV][32];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nw = blockDim.x >> 5;
-  double a[REDUCE_MAX_NV];
+  const int used = min(nw, (int)((nblk + 31) >> 5));  // the other warps hold no partials
+  if (warp < used) {
+    double a[REDUCE_MAX_NV];
 #pragma unroll
-  for (int k = 0; k < REDUCE_MAX_NV; ++k) a[k] = 0.0;
-  for (int j = threadIdx.x; j < (int)nblk; j += blockDim.x) {
-    double v[REDUCE_MAX_NV];
+    for (int k = 0; k < REDUCE_MAX_NV; ++k) a[k] = 0.0;
+    for (int j = threadIdx.x; j < (int)nblk; j += blockDim.x) {
+      double v[REDUCE_MAX_NV];
 #pragma unroll
-    for (int k = 0; k < REDUCE_MAX_NV; ++k) v[k] = k < nv ? __ldcg(partials + (size_t)(slot0 + k) * nblk + j) : 0.0;
+      for (int k = 0; k < REDUCE_MAX_NV; ++k) v[k] = k < nv ? __ldcg(partials + (size_t)(slot0 + k) * nblk + j) : 0.0;
 #pragma unroll
-    for (int k = 0; k < REDUCE_MAX_NV; ++k) a[k] += v[k];
-  }
+      for (int k = 0; k < REDUCE_MAX_NV; ++k) a[k] += v[k];
+    }
 #pragma unroll
-  for (int k = 0; k < REDUCE_MAX_NV; ++k) {
-    if (k < nv) {
-      a[k] = warp_sum(a[k]);
-      if (lane == 0) s_sum[k][warp] = a[k];
+    for (int k = 0; k < REDUCE_MAX_NV; ++k) {
+      if (k < nv) {
+        a[k] = warp_sum(a[k]);
+        if (lane == 0) s_sum[k][warp] = a[k];
+      }
     }
   }
   __syncthreads();
@@ -201,7 +209,7 @@ static __device__ __noinline__ void reduce_partials_last_block(const double* par
 #pragma unroll
     for (int k = 0; k < REDUCE_MAX_NV; ++k) {
       if (k < nv) {
-        double t = lane < nw ? s_sum[k][lane] : 0.0;
+        double t = lane < used ? s_sum[k][lane] : 0.0;
         t = warp_sum(t);
         if (lane == 0) {
           totals[slot0 + k] = t;
@@ -212,9 +220,10 @@ static __device__ __noinline__ void reduce_partials_last_block(const double* par
   }
 }
 
-__device__ __forceinline__ bool group_reduce_sync(GridBarrier* bar, DevStatus* st, unsigned long long limit_ns,
-                                                  const double* partials, double* totals, int slot0, int nv,
-                                                  unsigned nblk, double* res = nullptr) {
+template <typename F>
+__device__ __forceinline__ bool group_reduce_apply(GridBarrier* bar, DevStatus* st, unsigned long long limit_ns,
+                                                   const double* partials, double* totals, int slot0, int nv,
+                                                   unsigned nblk, F&& fn) {
   __shared__ int s_last, s_ok2;
   __shared__ unsigned s_gen;
   __shared__ double s_tot[REDUCE_MAX_NV];
@@ -225,28 +234,39 @@ __device__ __forceinline__ bool group_reduce_sync(GridBarrier* bar, DevStatus* s
     s_last = last;
   }
   __syncthreads();
-  int ok = 1;
-  if (s_last) {
-    reduce_partials_last_block(partials, totals, s_tot, slot0, nv, nblk);
-    if (threadIdx.x == 0) {
+  if (s_last) reduce_partials_last_block(partials, totals, s_tot, slot0, nv, nblk);
+  if (threadIdx.x == 0) {
+    int ok = 1;
+    if (s_last) {
       __threadfence();
       barrier_release(bar, s_gen);
+    } else {
+      ok = barrier_wait(bar, st, limit_ns, s_gen);
+      if (ok)
+        for (int k = 0; k < nv; ++k) s_tot[k] = __ldcg(totals + slot0 + k);
     }
-  } else if (threadIdx.x == 0) {
-    ok = barrier_wait(bar, st, limit_ns, s_gen);
-    if (ok && res)
-      for (int k = 0; k < nv; ++k) s_tot[k] = __ldcg(totals + slot0 + k);
+    s_ok2 = ok;
+    if (ok) fn(s_tot);
   }
-  if (threadIdx.x == 0) s_ok2 = ok;
   __syncthreads();
-  if (res)
-    for (int k = 0; k < nv; ++k) res[k] = s_tot[k];
   return s_ok2 != 0;
+}
+
+// The same, every thread getting the totals themselves in res[0 .. nv).
+__device__ __forceinline__ bool group_reduce_sync(GridBarrier* bar, DevStatus* st, unsigned long long limit_ns,
+                                                  const double* partials, double* totals, int slot0, int nv,
+                                                  unsigned nblk, double* res) {
+  __shared__ double s_res[REDUCE_MAX_NV];
+  const bool ok = group_reduce_apply(bar, st, limit_ns, partials, totals, slot0, nv, nblk, [&](const double* t) {
+    for (int k = 0; k < nv; ++k) s_res[k] = t[k];
+  });
+  for (int k = 0; k < nv; ++k) res[k] = s_res[k];
+  return ok;
 }
 
 __device__ __forceinline__ bool grid_reduce_sync(GridBarrier* bar, DevStatus* st, unsigned long long limit_ns,
                                                  const double* partials, double* totals, int slot0, int nv,
-                                                 double* res = nullptr) {
+                                                 double* res) {
   return group_reduce_sync(bar, st, limit_ns, partials, totals, slot0, nv, gridDim.x, res);
 }
 

@@ -61,70 +61,49 @@ __global__ void __launch_bounds__(PCG_THREADS) pcg_kernel(PcgArgs<V> P) {
     rz_p = fma(bi, z, rz_p);
     bb_p = fma(bi, bi, bb_p);
   }
+  __shared__ CgScalars<A> S;
   block_partials<A>(bb_p, rz_p, 2, P.partials, S_RR, S_RZ);
-  double red[REDUCE_MAX_NV];
-  if (!grid_reduce_sync(P.bar, P.st, P.limit_ns, P.partials, P.totals, S_RR, 2, red)) return;
-  A rz = (A)red[1];
-  const double bnorm = sqrt(red[0]);
+  if (!group_reduce_apply(P.bar, P.st, P.limit_ns, P.partials, P.totals, S_RR, 2, gridDim.x,
+                          [&](const double* t) { cg_begin(S, t); }))
+    return;
   long long iters = 0;
-  double residual = bnorm;
-  int status = AXIA_OK;
-  if (bnorm >= 1e-30) {
-    for (long long it = 0; it < P.max_iter; ++it) {
-      iters = it + 1;
-      // q = K p, p.q
-      A pq_p = 0;
-      for (int base = gwarp * RPW; base < n; base += nwarps * RPW) {
-        const int row = base + grp;
-        const A s = csr_row_dot<V, A, L>(row, n, sl, P.rowptr, P.col, P.val, P.p);
-        if (row < n && sl == 0) {
-          P.q[row] = (V)s;
-          pq_p = fma((A)P.p[row], s, pq_p);
-        }
+  for (long long it = 0; !S.stop && it < P.max_iter; ++it) {
+    iters = it + 1;
+    // q = K p, p.q
+    A pq_p = 0;
+    for (int base = gwarp * RPW; base < n; base += nwarps * RPW) {
+      const int row = base + grp;
+      const A s = csr_row_dot<V, A, L>(row, n, sl, P.rowptr, P.col, P.val, P.p);
+      if (row < n && sl == 0) {
+        P.q[row] = (V)s;
+        pq_p = fma((A)P.p[row], s, pq_p);
       }
-      block_partials<A>(pq_p, A(0), 1, P.partials, S_PQ, S_PQ);
-      double red[REDUCE_MAX_NV];
-      if (!grid_reduce_sync(P.bar, P.st, P.limit_ns, P.partials, P.totals, S_PQ, 1, red)) return;
-      const A pq = (A)red[0];
-      if (!(fabs((double)pq) >= 1e-30)) {
-        status = AXIA_ERR_ZERO_PIVOT;
-        break;
-      }
-      const A alpha = rz / pq;
-      // x += alpha p, r -= alpha q, r.r, r.z
-      A rr_p = 0, rzn_p = 0;
-      for (int i = tid; i < n; i += nth) {
-        P.x[i] = fma(alpha, P.p[i], P.x[i]);
-        const V ri = fma(-alpha, P.q[i], P.r[i]);
-        P.r[i] = ri;
-        rr_p = fma(ri, ri, rr_p);
-        rzn_p = fma(ri, ri * P.dinv[i], rzn_p);
-      }
-      block_partials<A>(rr_p, rzn_p, 2, P.partials, S_RR, S_RZ);
-      if (!grid_reduce_sync(P.bar, P.st, P.limit_ns, P.partials, P.totals, S_RR, 2, red)) return;
-      const A rzn = (A)red[1];
-      residual = sqrt(red[0]);
-      if (!isfinite(residual)) {
-        status = AXIA_ERR_NONFINITE;
-        break;
-      }
-      if (residual <= P.tol * bnorm) break;
-      const A beta = rzn / rz;
-      rz = rzn;
-      for (int i = tid; i < n; i += nth) P.p[i] = fma(beta, P.p[i], P.r[i] * P.dinv[i]);
-      if (!grid_sync(P.bar, P.st, P.limit_ns)) return;
     }
-    if (status == AXIA_OK && residual > P.tol * bnorm * 10.0) status = AXIA_ERR_NOT_CONVERGED;
-  } else {
-    residual = 0.0;
+    block_partials<A>(pq_p, A(0), 1, P.partials, S_PQ, S_PQ);
+    if (!group_reduce_apply(P.bar, P.st, P.limit_ns, P.partials, P.totals, S_PQ, 1, gridDim.x,
+                            [&](const double* t) { cg_alpha(S, t); }))
+      return;
+    if (S.status != AXIA_OK) break;
+    const A alpha = S.alpha;
+    // x += alpha p, r -= alpha q, r.r, r.z
+    A rr_p = 0, rzn_p = 0;
+    for (int i = tid; i < n; i += nth) {
+      P.x[i] = fma(alpha, P.p[i], P.x[i]);
+      const V ri = fma(-alpha, P.q[i], P.r[i]);
+      P.r[i] = ri;
+      rr_p = fma(ri, ri, rr_p);
+      rzn_p = fma(ri, ri * P.dinv[i], rzn_p);
+    }
+    block_partials<A>(rr_p, rzn_p, 2, P.partials, S_RR, S_RZ);
+    if (!group_reduce_apply(P.bar, P.st, P.limit_ns, P.partials, P.totals, S_RR, 2, gridDim.x,
+                            [&](const double* t) { cg_beta(S, t, P.tol); }))
+      return;
+    if (S.status != AXIA_OK || S.stop) break;
+    const A beta = S.beta;
+    for (int i = tid; i < n; i += nth) P.p[i] = fma(beta, P.p[i], P.r[i] * P.dinv[i]);
+    if (!grid_sync(P.bar, P.st, P.limit_ns)) return;
   }
-  if (blockIdx.x == 0 && threadIdx.x == 0) {
-    P.out->iters = iters;
-    P.out->residual = residual;
-    P.out->bnorm = bnorm;
-    P.out->status = status;
-    P.out->updates = 0;
-  }
+  if (blockIdx.x == 0 && threadIdx.x == 0) cg_out(S, P.out, P.tol, iters, 0);
 }
 
 // ---------------------------------------------------------------------------
@@ -178,18 +157,14 @@ __global__ void __launch_bounds__(PCG_THREADS, 4) pcg_reliable_kernel(ReliableAr
     rz_p = fmaf(ri, z, rz_p);
     bb_p = fma(bi, bi, bb_p);
   }
+  __shared__ CgScalars<float> S;
   block_partials<double>(bb_p, (double)rz_p, 2, P.partials, S_RR, S_RZ);
-  double red[REDUCE_MAX_NV];
-  if (!grid_reduce_sync(P.bar, P.st, P.limit_ns, P.partials, P.totals, S_RR, 2, red)) return;
-  float rz = (float)red[1];
-  const double bnorm = sqrt(red[0]);
-  double rmax = bnorm;       // residual norm at the last update
-  double residual = bnorm;   // FP64 residual norm at the last update
+  if (!group_reduce_apply(P.bar, P.st, P.limit_ns, P.partials, P.totals, S_RR, 2, gridDim.x,
+                          [&](const double* t) { mixed_begin(S, t); }))
+    return;
   long long iters = 0;
-  int updates = 0, status = AXIA_OK;
-  bool converged = bnorm < 1e-30;
-  if (converged) residual = 0.0;
-  for (long long it = 0; !converged && it < P.max_iter; ++it) {
+  int updates = 0;
+  for (long long it = 0; !S.stop && it < P.max_iter; ++it) {
     iters = it + 1;
     float pq_p = 0.f;
     {
@@ -205,14 +180,11 @@ __global__ void __launch_bounds__(PCG_THREADS, 4) pcg_reliable_kernel(ReliableAr
       }
     }
     block_partials<float>(pq_p, 0.f, 1, P.partials, S_PQ, S_PQ);
-    double red[REDUCE_MAX_NV];
-    if (!grid_reduce_sync(P.bar, P.st, P.limit_ns, P.partials, P.totals, S_PQ, 1, red)) return;
-    const float pq = (float)red[0];
-    if (!(fabsf(pq) >= 1e-30f) || !isfinite(pq)) {
-      status = isfinite(pq) ? AXIA_ERR_ZERO_PIVOT : AXIA_ERR_NONFINITE;
-      break;
-    }
-    const float alpha = rz / pq;
+    if (!group_reduce_apply(P.bar, P.st, P.limit_ns, P.partials, P.totals, S_PQ, 1, gridDim.x,
+                            [&](const double* t) { mixed_alpha(S, t); }))
+      return;
+    if (S.status != AXIA_OK) break;
+    const float alpha = S.alpha;
     float rr_p = 0.f, rzn_p = 0.f;
     for (int i = tid; i < n; i += nth) {
       P.x32[i] = fmaf(alpha, P.p32[i], P.x32[i]);
@@ -222,14 +194,14 @@ __global__ void __launch_bounds__(PCG_THREADS, 4) pcg_reliable_kernel(ReliableAr
       rzn_p = fmaf(ri, ri * P.dinv32[i], rzn_p);
     }
     block_partials<float>(rr_p, rzn_p, 2, P.partials, S_RR, S_RZ);
-    if (!grid_reduce_sync(P.bar, P.st, P.limit_ns, P.partials, P.totals, S_RR, 2, red)) return;
-    float rzn = (float)red[1];
-    const double rnorm32 = sqrt(red[0]);
-    if (!isfinite(rnorm32)) {
-      status = AXIA_ERR_NONFINITE;
-      break;
-    }
-    if (rnorm32 <= P.delta * rmax || rnorm32 <= P.tol * bnorm) {
+    if (!group_reduce_apply(P.bar, P.st, P.limit_ns, P.partials, P.totals, S_RR, 2, gridDim.x,
+                            [&](const double* t) {
+                              mixed_check(S, t[0], P.tol, P.delta);
+                              mixed_rz<false>(S, (float)t[1], !S.update);
+                            }))
+      return;
+    if (S.status != AXIA_OK) break;
+    if (S.update) {
       // reliable update: x += x32 (FP64), r = b - K x (FP64), r32 = r
       for (int i = tid; i < n; i += nth) {
         P.x[i] += (double)P.x32[i];
@@ -255,34 +227,20 @@ __global__ void __launch_bounds__(PCG_THREADS, 4) pcg_reliable_kernel(ReliableAr
         }
       }
       block_partials<double>(rr64_p, (double)rz_new_p, 2, P.partials, S_RR, S_RZ);
-      double red[REDUCE_MAX_NV];
-      if (!grid_reduce_sync(P.bar, P.st, P.limit_ns, P.partials, P.totals, S_RR, 2, red)) return;
+      if (!group_reduce_apply(P.bar, P.st, P.limit_ns, P.partials, P.totals, S_RR, 2, gridDim.x,
+                              [&](const double* t) {
+                                mixed_replaced(S, t[0], P.tol);
+                                mixed_rz<false>(S, (float)t[1], true);
+                              }))
+        return;
       ++updates;
-      residual = sqrt(red[0]);
-      rzn = (float)red[1];
-      rmax = residual;
-      if (!isfinite(residual)) {
-        status = AXIA_ERR_NONFINITE;
-        break;
-      }
-      if (residual <= P.tol * bnorm) {
-        converged = true;
-        break;
-      }
+      if (S.status != AXIA_OK || S.stop) break;
     }
-    const float beta = rzn / rz;
-    rz = rzn;
+    const float beta = S.beta;
     for (int i = tid; i < n; i += nth) P.p32[i] = fmaf(beta, P.p32[i], P.r32[i] * P.dinv32[i]);
     if (!grid_sync(P.bar, P.st, P.limit_ns)) return;
   }
-  if (status == AXIA_OK && residual > P.tol * bnorm * 10.0) status = AXIA_ERR_NOT_CONVERGED;
-  if (blockIdx.x == 0 && threadIdx.x == 0) {
-    P.out->iters = iters;
-    P.out->residual = residual;
-    P.out->bnorm = bnorm;
-    P.out->status = status;
-    P.out->updates = updates;
-  }
+  if (blockIdx.x == 0 && threadIdx.x == 0) cg_out(S, P.out, P.tol, iters, updates);
 }
 
 // ---------------------------------------------------------------------------

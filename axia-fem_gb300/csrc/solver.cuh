@@ -48,37 +48,145 @@ __device__ __forceinline__ T group_sum(T v) {
 }
 
 // block-reduce up to two values and store them as this block's partials
-// (block `rank` of a group of nblk blocks; the whole grid by default)
+// (block `rank` of a group of nblk blocks; the whole grid by default).
+// FP64 values go through shared memory: a warp sum costs every warp five
+// dependent FP64 additions per value, and GB300 issues one FP64 warp
+// instruction per SM about every 18 cycles, so 16 warps and two values take
+// 1.5 us per block; four warps per value adding up a quarter of the warps'
+// lanes each, then one warp, need 8 + 3 + 5 instead of 160 of them.
 template <typename A>
 __device__ __forceinline__ void block_partials(A v0, A v1, int nv, double* partials, int slot0, int slot1,
                                                unsigned nblk = 0, unsigned rank = 0) {
-  __shared__ A s_red[2][32];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nw = blockDim.x >> 5;
-  v0 = warp_sum(v0);
-  if (nv > 1) v1 = warp_sum(v1);
-  if (lane == 0) {
-    s_red[0][warp] = v0;
-    s_red[1][warp] = v1;
+  if (nblk == 0) {
+    nblk = gridDim.x;
+    rank = blockIdx.x;
   }
-  __syncthreads();
-  if (warp == 0) {
-    A a0 = lane < nw ? s_red[0][lane] : A(0);
-    A a1 = lane < nw ? s_red[1][lane] : A(0);
-    a0 = warp_sum(a0);
-    if (nv > 1) a1 = warp_sum(a1);
+  if constexpr (sizeof(A) == sizeof(double)) {
+    constexpr int Q = 4;
+    __shared__ A s_all[2][PCG_THREADS];
+    __shared__ A s_part[2][Q][32];
+    s_all[0][threadIdx.x] = v0;
+    if (nv > 1) s_all[1][threadIdx.x] = v1;
+    __syncthreads();
+    for (int t = warp; t < Q * nv; t += nw) {
+      const int k = t / Q, g = t % Q;
+      A a = A(0);
+      for (int w = g; w < nw; w += Q) a += s_all[k][32 * w + lane];
+      s_part[k][g][lane] = a;
+    }
+    __syncthreads();
+    for (int k = warp; k < nv; k += nw) {
+      const A a = warp_sum((s_part[k][0][lane] + s_part[k][1][lane]) + (s_part[k][2][lane] + s_part[k][3][lane]));
+      if (lane == 0) partials[(k == 0 ? slot0 : slot1) * nblk + rank] = a;
+    }
+  } else {
+    __shared__ A s_red[2][32];
+    v0 = warp_sum(v0);
+    if (nv > 1) v1 = warp_sum(v1);
     if (lane == 0) {
-      if (nblk == 0) {
-        nblk = gridDim.x;
-        rank = blockIdx.x;
+      s_red[0][warp] = v0;
+      s_red[1][warp] = v1;
+    }
+    __syncthreads();
+    if (warp == 0) {
+      A a0 = lane < nw ? s_red[0][lane] : A(0);
+      A a1 = lane < nw ? s_red[1][lane] : A(0);
+      a0 = warp_sum(a0);
+      if (nv > 1) a1 = warp_sum(a1);
+      if (lane == 0) {
+        partials[slot0 * nblk + rank] = (double)a0;
+        if (nv > 1) partials[slot1 * nblk + rank] = (double)a1;
       }
-      partials[slot0 * nblk + rank] = (double)a0;
-      if (nv > 1) partials[slot1 * nblk + rank] = (double)a1;
     }
   }
 }
 
+// What one iteration of a persistent CG needs from its reductions, computed
+// by thread 0 of each block and read by the block from shared memory.
+template <typename A>
+struct CgScalars {
+  A rz, rzn;                     // r.z of the current direction; of the new r, its diagonal part
+  A alpha, beta;
+  double bnorm, rmax, residual;  // ||b||, ||r|| at the last update, final residual
+  int status;                    // axia_status that ends the loop
+  int update;                    // mixed: replace the residual now
+  int stop;                      // converged
+};
+
 __device__ __forceinline__ double total(const double* totals, int slot) { return __ldcg(totals + slot); }
 
+
+// The scalar steps of the FP32 CG with FP64 reliable updates, on thread 0 of
+// each block.  beta is r.z (new) / r.z (old), with the replaced r after an update.
+__device__ __forceinline__ void mixed_begin(CgScalars<float>& S, const double* t) {
+  S.rz = (float)t[1];
+  S.bnorm = S.rmax = S.residual = sqrt(t[0]);
+  S.status = AXIA_OK;
+  S.update = 0;
+  S.stop = S.bnorm < 1e-30;
+  if (S.stop) S.residual = 0.0;
+}
+__device__ __forceinline__ void mixed_alpha(CgScalars<float>& S, const double* t) {
+  const float pq = (float)t[0];
+  if (!(fabsf(pq) >= 1e-30f) || !isfinite(pq)) S.status = isfinite(pq) ? AXIA_ERR_ZERO_PIVOT : AXIA_ERR_NONFINITE;
+  S.alpha = S.rz / pq;
+}
+__device__ __forceinline__ void mixed_set_beta(CgScalars<float>& S, float rzn) {
+  S.beta = rzn / S.rz;
+  S.rz = rzn;
+}
+__device__ __forceinline__ void mixed_check(CgScalars<float>& S, double rr, double tol, double delta) {
+  const double rnorm32 = sqrt(rr);
+  if (!isfinite(rnorm32)) S.status = AXIA_ERR_NONFINITE;
+  S.update = rnorm32 <= delta * S.rmax || rnorm32 <= tol * S.bnorm;
+}
+__device__ __forceinline__ void mixed_replaced(CgScalars<float>& S, double rr, double tol) {
+  S.residual = S.rmax = sqrt(rr);
+  if (!isfinite(S.residual)) S.status = AXIA_ERR_NONFINITE;
+  S.stop = S.residual <= tol * S.bnorm;
+}
+// the diagonal part of the new r.z: beta at once with the diagonal
+// preconditioner, after the coarse part is known with the two-level one
+template <bool COARSE>
+__device__ __forceinline__ void mixed_rz(CgScalars<float>& S, float rzn, bool last) {
+  if constexpr (COARSE)
+    S.rzn = rzn;
+  else if (last)
+    mixed_set_beta(S, rzn);
+}
+// The same steps of the one-precision CG (linalg.rs:199-259).
+template <typename A>
+__device__ __forceinline__ void cg_begin(CgScalars<A>& S, const double* t) {
+  S.rz = (A)t[1];
+  S.bnorm = S.residual = sqrt(t[0]);
+  S.status = AXIA_OK;
+  S.stop = !(S.bnorm >= 1e-30);
+  if (S.stop) S.residual = 0.0;
+}
+template <typename A>
+__device__ __forceinline__ void cg_alpha(CgScalars<A>& S, const double* t) {
+  const A pq = (A)t[0];
+  if (!(fabs((double)pq) >= 1e-30)) S.status = AXIA_ERR_ZERO_PIVOT;
+  S.alpha = S.rz / pq;
+}
+template <typename A>
+__device__ __forceinline__ void cg_beta(CgScalars<A>& S, const double* t, double tol) {
+  const A rzn = (A)t[1];
+  S.residual = sqrt(t[0]);
+  if (!isfinite(S.residual)) S.status = AXIA_ERR_NONFINITE;
+  S.stop = S.residual <= tol * S.bnorm;
+  S.beta = rzn / S.rz;
+  S.rz = rzn;
+}
+template <typename A>
+__device__ __forceinline__ void cg_out(const CgScalars<A>& S, PcgOut* out, double tol, long long iters, int updates) {
+  out->iters = iters;
+  out->residual = S.residual;
+  out->bnorm = S.bnorm;
+  out->status = S.status == AXIA_OK && S.residual > tol * S.bnorm * 10.0 ? AXIA_ERR_NOT_CONVERGED : S.status;
+  out->updates = updates;
+}
 
 // ---------------------------------------------------------------------------
 // Node-block (3x3) matrix and the mixed-precision argument pack (bsr.cu)
