@@ -271,11 +271,12 @@ __global__ void __launch_bounds__(PCG_THREADS) pcg_bsr_kernel(BsrPcgArgs<V> P) {
     const A alpha = S.alpha;
     A rr_p = 0, rzn_p = 0;
     for (int i = tid; i < nd; i += nth) {
-      P.x[i] = fma(alpha, P.p[i], P.x[i]);
-      const V ri = fma(-alpha, P.q[i], P.r[i]);
+      const V pi = P.p[i], xi = P.x[i], qi = P.q[i], r0 = P.r[i], di = __ldg(P.dinv + i);
+      P.x[i] = fma(alpha, pi, xi);
+      const V ri = fma(-alpha, qi, r0);
       P.r[i] = ri;
       rr_p = fma(ri, ri, rr_p);
-      rzn_p = fma(ri, ri * P.dinv[i], rzn_p);
+      rzn_p = fma(ri, ri * di, rzn_p);
     }
     block_partials<A>(rr_p, rzn_p, 2, P.partials, S_RR, S_RZ);
     if (!group_reduce_apply(P.bar, P.st, P.limit_ns, P.partials, P.totals, S_RR, 2, gridDim.x,
@@ -331,6 +332,9 @@ __device__ __forceinline__ void reliable_body(const BsrReliableArgs& P, const Co
   M64.n_nodes = n1;
   const int tid = R.rank * blockDim.x + threadIdx.x, nth = R.nblk * blockDim.x;
   const int gwarp = tid >> 5, nwarps = nth >> 5;
+  // restriction chunks go to the warps of different blocks first: a small
+  // system has fewer chunks than warps
+  const int cwarp = (threadIdx.x >> 5) * R.nblk + R.rank;
   const int lane = threadIdx.x & 31;
   const int nd = 3 * n1;  // vector loops run over [i0, 3 n1)
   double* const partials = R.partials;
@@ -357,7 +361,7 @@ __device__ __forceinline__ void reliable_body(const BsrReliableArgs& P, const Co
   int updates = 0;
   if constexpr (COARSE) {
     if (!S.stop) {  // p = D^-1 b + Z M Z^T b
-      coarse_restrict(C, P.r32, gwarp, nwarps, lane);
+      coarse_restrict(C, P.r32, cwarp, nwarps, lane);
       if (!group_sync(R.bar, P.st, P.limit_ns, R.nblk)) return;
       if (!coarse_step(P, C, R, gwarp, nwarps, lane, S, true)) return;
       coarse_update_p(C, n0, n1, tid, nth, 0.f, P.r32, P.dinv32, P.p32, true);
@@ -381,12 +385,13 @@ __device__ __forceinline__ void reliable_body(const BsrReliableArgs& P, const Co
           bsr_row<float, float, V32, L32>(a, sl, M32, P.p32, y0, y1, y2);
         }
         if (a < n1 && sl == 0) {
+          const float p0 = P.p32[3 * a], p1 = P.p32[3 * a + 1], p2 = P.p32[3 * a + 2];
           P.q32[3 * a] = y0;
           P.q32[3 * a + 1] = y1;
           P.q32[3 * a + 2] = y2;
-          pq_p = fmaf(P.p32[3 * a], y0, pq_p);
-          pq_p = fmaf(P.p32[3 * a + 1], y1, pq_p);
-          pq_p = fmaf(P.p32[3 * a + 2], y2, pq_p);
+          pq_p = fmaf(p0, y0, pq_p);
+          pq_p = fmaf(p1, y1, pq_p);
+          pq_p = fmaf(p2, y2, pq_p);
         }
       }
     }
@@ -398,14 +403,15 @@ __device__ __forceinline__ void reliable_body(const BsrReliableArgs& P, const Co
     const float alpha = S.alpha;
     float rr_p = 0.f, rzn_p = 0.f;
     if constexpr (COARSE) {
-      coarse_update_restrict(C, alpha, P.x32, P.p32, P.q32, P.r32, P.dinv32, gwarp, nwarps, lane, rr_p, rzn_p);
+      coarse_update_restrict(C, alpha, P.x32, P.p32, P.q32, P.r32, P.dinv32, cwarp, nwarps, lane, rr_p, rzn_p);
     } else {
       for (int i = i0 + tid; i < nd; i += nth) {
-        P.x32[i] = fmaf(alpha, P.p32[i], P.x32[i]);
-        const float ri = fmaf(-alpha, P.q32[i], P.r32[i]);
+        const float pi = P.p32[i], xi = P.x32[i], qi = P.q32[i], r0 = P.r32[i], di = __ldg(P.dinv32 + i);
+        P.x32[i] = fmaf(alpha, pi, xi);
+        const float ri = fmaf(-alpha, qi, r0);
         P.r32[i] = ri;
         rr_p = fmaf(ri, ri, rr_p);
-        rzn_p = fmaf(ri, ri * P.dinv32[i], rzn_p);
+        rzn_p = fmaf(ri, ri * di, rzn_p);
       }
     }
     block_partials<float>(rr_p, rzn_p, 2, partials, S_RR, S_RZ, R.nblk, R.rank);
@@ -452,7 +458,7 @@ __device__ __forceinline__ void reliable_body(const BsrReliableArgs& P, const Co
       ++updates;
       if (S.status != AXIA_OK || S.stop) break;
       if constexpr (COARSE) {  // r was replaced: restrict it again
-        coarse_restrict(C, P.r32, gwarp, nwarps, lane);
+        coarse_restrict(C, P.r32, cwarp, nwarps, lane);
         if (!group_sync(R.bar, P.st, P.limit_ns, R.nblk)) return;
       }
     }

@@ -82,9 +82,9 @@ __device__ __forceinline__ void coarse_chunk_finish(const CoarseArgs& C, int c, 
 }
 
 // r_c = Z^T r over the chunks (after an FP64 residual replaced r, and at the start)
-__device__ __forceinline__ void coarse_restrict(const CoarseArgs& C, const float* r, int gwarp, int nwarps,
+__device__ __forceinline__ void coarse_restrict(const CoarseArgs& C, const float* r, int cwarp, int nwarps,
                                                 int lane) {
-  for (int c = C.chunk_lo + gwarp; c < C.chunk_hi; c += nwarps) {
+  for (int c = C.chunk_lo + cwarp; c < C.chunk_hi; c += nwarps) {
     const int4 ch = C.chunk[c];
     float v[6] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
 #pragma unroll 4
@@ -100,26 +100,39 @@ __device__ __forceinline__ void coarse_restrict(const CoarseArgs& C, const float
 
 // The CG update x += alpha p, r -= alpha q node by node in subdomain order,
 // with the partial sums of r.r and r.D^-1 r and the restriction of the new r.
+// A node's 15 values are all requested before its six stores (the stores may
+// alias the loads as far as the compiler knows, so a load after a store waits
+// a memory round trip).
 __device__ __forceinline__ void coarse_update_restrict(const CoarseArgs& C, float alpha, float* x, const float* p,
-                                                       const float* q, float* r, const float* dinv, int gwarp,
+                                                       const float* q, float* r, const float* dinv, int cwarp,
                                                        int nwarps, int lane, float& rr_p, float& rz_p) {
-  for (int c = C.chunk_lo + gwarp; c < C.chunk_hi; c += nwarps) {
+  for (int c = C.chunk_lo + cwarp; c < C.chunk_hi; c += nwarps) {
     const int4 ch = C.chunk[c];
     float v[6] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
-#pragma unroll 4
-    for (int k = ch.y + lane; k < ch.z; k += 32) {
-      const int a = __ldg(C.sub_node + k);
+    int k = ch.y + lane;
+    int a = k < ch.z ? __ldg(C.sub_node + k) : 0;
+    while (k < ch.z) {
       const float4 g = __ldg(C.geo + a);
-      const unsigned m = geo_bits(g);
-      float rv[3];
+      const int i = 3 * a;
+      float xv[3], pv[3], qv[3], rv[3], dv[3];
 #pragma unroll
       for (int d = 0; d < 3; ++d) {
-        const int i = 3 * a + d;
-        x[i] = fmaf(alpha, p[i], x[i]);
-        const float ri = fmaf(-alpha, q[i], r[i]);
-        r[i] = ri;
+        pv[d] = p[i + d];
+        xv[d] = x[i + d];
+        qv[d] = q[i + d];
+        rv[d] = r[i + d];
+        dv[d] = __ldg(dinv + i + d);
+      }
+      k += 32;
+      a = k < ch.z ? __ldg(C.sub_node + k) : 0;
+      const unsigned m = geo_bits(g);
+#pragma unroll
+      for (int d = 0; d < 3; ++d) {
+        x[i + d] = fmaf(alpha, pv[d], xv[d]);
+        const float ri = fmaf(-alpha, qv[d], rv[d]);
+        r[i + d] = ri;
         rr_p = fmaf(ri, ri, rr_p);
-        rz_p = fmaf(ri, ri * dinv[i], rz_p);
+        rz_p = fmaf(ri, ri * dv[d], rz_p);
         rv[d] = ((m >> d) & 1u) ? ri : 0.f;
       }
       zt_add(g, rv[0], rv[1], rv[2], v);
@@ -164,9 +177,18 @@ __device__ __forceinline__ float coarse_solve(const CoarseArgs& C, float* s_rc, 
 // subdomain's six y per node, then its three DOFs (beta = 0, add = true: p += Z y).
 __device__ __forceinline__ void coarse_update_p(const CoarseArgs& C, int n0, int n1, int tid, int nth, float beta,
                                                 const float* r, const float* dinv, float* p, bool add_only) {
-#pragma unroll 2
   for (int a = n0 + tid; a < n1; a += nth) {
     const float4 g = __ldg(C.geo + a);
+    const int i = 3 * a;
+    float pv[3], rv[3], dv[3];
+#pragma unroll
+    for (int c = 0; c < 3; ++c) {
+      pv[c] = p[i + c];
+      if (!add_only) {
+        rv[c] = r[i + c];
+        dv[c] = __ldg(dinv + i + c);
+      }
+    }
     const unsigned m = geo_bits(g);
     const float* y = C.yc + 6 * (m >> 3);
     const float y0 = y[0], y1 = y[1], y2 = y[2], y3 = y[3], y4 = y[4], y5 = y[5];
@@ -174,12 +196,7 @@ __device__ __forceinline__ void coarse_update_p(const CoarseArgs& C, int n0, int
                          (m & 2u) ? fmaf(-g.z, y3, fmaf(g.x, y5, y1)) : 0.f,
                          (m & 4u) ? fmaf(g.y, y3, fmaf(-g.x, y4, y2)) : 0.f};
 #pragma unroll
-    for (int c = 0; c < 3; ++c) {
-      const int i = 3 * a + c;
-      if (add_only)
-        p[i] += zc[c];
-      else
-        p[i] = fmaf(beta, p[i], fmaf(r[i], dinv[i], zc[c]));
-    }
+    for (int c = 0; c < 3; ++c)
+      p[i + c] = add_only ? pv[c] + zc[c] : fmaf(beta, pv[c], fmaf(rv[c], dv[c], zc[c]));
   }
 }

@@ -88,11 +88,12 @@ __global__ void __launch_bounds__(PCG_THREADS) pcg_kernel(PcgArgs<V> P) {
     // x += alpha p, r -= alpha q, r.r, r.z
     A rr_p = 0, rzn_p = 0;
     for (int i = tid; i < n; i += nth) {
-      P.x[i] = fma(alpha, P.p[i], P.x[i]);
-      const V ri = fma(-alpha, P.q[i], P.r[i]);
+      const V pi = P.p[i], xi = P.x[i], qi = P.q[i], r0 = P.r[i], di = __ldg(P.dinv + i);
+      P.x[i] = fma(alpha, pi, xi);
+      const V ri = fma(-alpha, qi, r0);
       P.r[i] = ri;
       rr_p = fma(ri, ri, rr_p);
-      rzn_p = fma(ri, ri * P.dinv[i], rzn_p);
+      rzn_p = fma(ri, ri * di, rzn_p);
     }
     block_partials<A>(rr_p, rzn_p, 2, P.partials, S_RR, S_RZ);
     if (!group_reduce_apply(P.bar, P.st, P.limit_ns, P.partials, P.totals, S_RR, 2, gridDim.x,
@@ -187,11 +188,12 @@ __global__ void __launch_bounds__(PCG_THREADS, 4) pcg_reliable_kernel(ReliableAr
     const float alpha = S.alpha;
     float rr_p = 0.f, rzn_p = 0.f;
     for (int i = tid; i < n; i += nth) {
-      P.x32[i] = fmaf(alpha, P.p32[i], P.x32[i]);
-      const float ri = fmaf(-alpha, P.q32[i], P.r32[i]);
+      const float pi = P.p32[i], xi = P.x32[i], qi = P.q32[i], r0 = P.r32[i], di = __ldg(P.dinv32 + i);
+      P.x32[i] = fmaf(alpha, pi, xi);
+      const float ri = fmaf(-alpha, qi, r0);
       P.r32[i] = ri;
       rr_p = fmaf(ri, ri, rr_p);
-      rzn_p = fmaf(ri, ri * P.dinv32[i], rzn_p);
+      rzn_p = fmaf(ri, ri * di, rzn_p);
     }
     block_partials<float>(rr_p, rzn_p, 2, P.partials, S_RR, S_RZ);
     if (!group_reduce_apply(P.bar, P.st, P.limit_ns, P.partials, P.totals, S_RR, 2, gridDim.x,
