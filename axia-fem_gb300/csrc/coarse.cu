@@ -53,7 +53,9 @@ struct CoarseBlk {
 };
 
 struct CoarseState {
-  int nodes_target = 0;
+  int nodes_target = 0;          // nodes per subdomain; 0: default_subdomains
+  int fewer = 0;                 // automatic size: how often it was coarsened
+  bool row_overflow = false;     // a node row reaches more subdomains than its item list holds
   bool per_mesh = false;         // one block per mesh
   std::vector<CoarseBlk> blk;
   CoarseBlk* d_blk = nullptr;    // [n_blocks]
@@ -860,6 +862,26 @@ int grid_for(const axia_ctx* ctx, int64_t n, int threads) {
   return (int)std::max<int64_t>(1, std::min<int64_t>((n + threads - 1) / threads, (int64_t)ctx->sm_count * 16));
 }
 
+// Default number of subdomains of a mesh: 0.38 nodes^0.55 (times the mean
+// blocks per node row over C3D8's 27), at least 50 nodes each, at most 512.
+// More subdomains cut the iterations, but the dense inverse grows with their
+// cube.  Measured, assembly + solve: C3D8 12^3 1 subdomain 3.6 ms, 27 1.8;
+// 20^3 8 3.6, 64 2.4, 125 2.5; 30^3 27 5.3, 125 4.3, 343 5.3; 45^3 125 7.8,
+// 216 7.8, 512 9.1; 65^3 216 16.9, 512 16.8; 80^3 216 30.1, 512 27.4; C3D20
+// 15^3 48 7.3, 150 6.1, 252 6.4; 25^3 125 16.1, 343 14.9, 648 17.0; C3D10
+// 13x11x12 27 6.5, 120 4.6.  64 cubes of 10 to 40 edges, solve: 232 in all
+// 187 ms, 1071 104, 3085 77, 4899 77 (and 5 ms more for the inverse).
+// `fewer` counts fallbacks to larger subdomains: a quarter each time, at
+// the last step of 500 nodes (13,500 blocks) and 1/512 of the mesh at least.
+constexpr int DEFAULT_SUBDOMAIN_STEPS = 3;
+int64_t default_subdomains(double nodes, double blocks_per_row, int fewer) {
+  const double dense = std::max(blocks_per_row, 1.0) / 27.0;
+  double v = std::min(0.38 * std::pow(std::max(nodes, 1.0), 0.55) * std::max(dense, 1.0), nodes / 50.0);
+  for (int k = 0; k < fewer; ++k) v *= 0.25;
+  if (fewer >= DEFAULT_SUBDOMAIN_STEPS) v = std::min(v, nodes / std::max(500.0 / dense, nodes / 512.0));
+  return std::max<int64_t>(1, (int64_t)std::min(512.0, v));
+}
+
 // subdomains, chunks, geo and T for the current mesh and constraints
 int build_space(axia_ctx* ctx, CoarseState* S) {
   const int64_t n = ctx->n_nodes;
@@ -873,7 +895,9 @@ int build_space(axia_ctx* ctx, CoarseState* S) {
   std::vector<int64_t> target(nm);
   int64_t tsum = 0;
   for (int k = 0; k < nm; ++k) {
-    target[k] = std::max<int64_t>(1, (mesh_a1(k) - mesh_a0(k)) / std::max(1, S->nodes_target));
+    const int64_t nk = mesh_a1(k) - mesh_a0(k);
+    target[k] = S->nodes_target > 0 ? std::max<int64_t>(1, nk / S->nodes_target)
+                                    : default_subdomains((double)nk, (double)ctx->n_adj / (double)n, S->fewer);
     tsum += target[k];
   }
   if (!S->per_mesh) {
@@ -1129,7 +1153,10 @@ int build_item_structure(axia_ctx* ctx, CoarseState* S) {
     k_row_count<<<grid_for(ctx, (int64_t)n * 32, 256), 256, 0, ctx->stream>>>(n, ctx->d_qptr, ctx->d_qadj, A.geo,
                                                                              d_cnt, ctx->d_status);
     ctx->launches++;
-    if ((st = read_status(ctx, "a node row touches more than 32 subdomains (raise coarse_nodes)"))) break;
+    if ((st = read_status(ctx, "a node row touches more than 32 subdomains (raise coarse_nodes)"))) {
+      S->row_overflow = st == AXIA_ERR_INVALID_ARG;
+      break;
+    }
     size_t tb = 0;
     cub::DeviceScan::ExclusiveSum(nullptr, tb, d_cnt, S->off, n + 1, ctx->stream);
     if ((st = dev_alloc(ctx, &d_temp, std::max<size_t>(tb, 16)))) break;
@@ -1289,44 +1316,42 @@ void coarse_release(axia_ctx* ctx) {
 // The coarse space of the current mesh (built on first use, or when the
 // requested subdomain size changes) and its operator for the current
 // assembly (rebuilt after every assembly).
-// Default subdomain size: about 512 subdomains (8^3 for a cube; the dense
-// inverse then costs about 4 ms), but no fewer than about 13,500 matrix node
-// blocks per subdomain -- 500 nodes for C3D8 (27 blocks per node row), about
-// 250 for C3D20 (about 55).  Measured per step: C3D20 50^3 350 iterations
-// and 147 ms with 216 subdomains, 271 and 127 ms with 512; SIMP C3D8
-// 100x50x50 236 iterations and 31.1 ms with 125 subdomains, 167 and 26.9 ms
-// with 512; the C3D8 100^3 headline keeps its 512.
-static int default_nodes_target(const axia_ctx* ctx) {
-  if (ctx->n_adj <= 0 || ctx->n_nodes <= 0) return 2000;
-  const double floor_nodes = 500.0 * 27.0 * (double)ctx->n_nodes / (double)ctx->n_adj;
-  const double v = std::max(floor_nodes, (double)ctx->n_nodes / 512.0);
-  return (int)std::min(1.0e6, std::max(16.0, v));
-}
-
 int coarse_prepare(axia_ctx* ctx, int nodes_target, CoarseArgs* out, bool per_mesh) {
   if (!ctx->have_bsr64) return set_error(ctx, AXIA_ERR_STATE, "coarse space needs the FP64 node-block matrix");
-  if (nodes_target <= 0) nodes_target = default_nodes_target(ctx);
+  nodes_target = std::max(nodes_target, 0);
   per_mesh = per_mesh && ctx->mesh_node0.size() >= 3;  // two or more meshes
   auto* S = static_cast<CoarseState*>(ctx->coarse);
   if (S && (S->nodes_target != nodes_target || S->per_mesh != per_mesh)) {
     coarse_release(ctx);
     S = nullptr;
   }
-  if (!S) {
-    S = new CoarseState();
-    S->nodes_target = nodes_target;
-    S->per_mesh = per_mesh;
-    ++ctx->coarse_gen;
-    ctx->coarse = S;
-    const int st = build_space(ctx, S);
-    if (st) {
-      coarse_release(ctx);
-      return st;
+  for (int fewer = 0;; ++fewer) {
+    if (!S) {
+      S = new CoarseState();
+      S->nodes_target = nodes_target;
+      S->per_mesh = per_mesh;
+      S->fewer = fewer;
+      ++ctx->coarse_gen;
+      ctx->coarse = S;
+      const int st = build_space(ctx, S);
+      if (st) {
+        coarse_release(ctx);
+        return st;
+      }
     }
-  }
-  if (S->op_gen != ctx->assemble_gen) {
-    AXIA_TRY(build_operator(ctx, S));
-    S->op_gen = ctx->assemble_gen;
+    if (S->op_gen == ctx->assemble_gen) break;
+    const int st = build_operator(ctx, S);
+    if (st == AXIA_OK) {
+      S->op_gen = ctx->assemble_gen;
+      break;
+    }
+    // very flat elements or hub nodes: a node row reaches more subdomains than
+    // an item list holds; the automatic size then falls back to larger ones
+    const bool retry = S->row_overflow && nodes_target == 0 && fewer < DEFAULT_SUBDOMAIN_STEPS;
+    coarse_release(ctx);  // a half-built operator is not reused
+    S = nullptr;
+    if (!retry) return st;
+    ctx->last_error.clear();
   }
   // arrival counters of the restriction (a stopped solve may leave them set)
   AXIA_CUDA(ctx, cudaMemsetAsync(S->cnt, 0, (size_t)S->args.n_sub * sizeof(int), ctx->stream));
