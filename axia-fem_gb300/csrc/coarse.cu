@@ -862,8 +862,9 @@ int grid_for(const axia_ctx* ctx, int64_t n, int threads) {
   return (int)std::max<int64_t>(1, std::min<int64_t>((n + threads - 1) / threads, (int64_t)ctx->sm_count * 16));
 }
 
-// Default number of subdomains of a mesh: 0.38 nodes^0.55 (times the mean
-// blocks per node row over C3D8's 27), at least 50 nodes each, at most 512.
+// Default number of subdomains of a mesh: 0.46 nodes^0.55 (times the mean
+// blocks per node row over C3D8's 27), at least 50 nodes each, at most 512;
+// the grid of boxes then has at most so many cells.
 // More subdomains cut the iterations, but the dense inverse grows with their
 // cube.  Measured, assembly + solve: C3D8 12^3 1 subdomain 3.6 ms, 27 1.8;
 // 20^3 8 3.6, 64 2.4, 125 2.5; 30^3 27 5.3, 125 4.3, 343 5.3; 45^3 125 7.8,
@@ -876,7 +877,7 @@ int grid_for(const axia_ctx* ctx, int64_t n, int threads) {
 constexpr int DEFAULT_SUBDOMAIN_STEPS = 3;
 int64_t default_subdomains(double nodes, double blocks_per_row, int fewer) {
   const double dense = std::max(blocks_per_row, 1.0) / 27.0;
-  double v = std::min(0.38 * std::pow(std::max(nodes, 1.0), 0.55) * std::max(dense, 1.0), nodes / 50.0);
+  double v = std::min(0.46 * std::pow(std::max(nodes, 1.0), 0.55) * std::max(dense, 1.0), nodes / 50.0);
   for (int k = 0; k < fewer; ++k) v *= 0.25;
   if (fewer >= DEFAULT_SUBDOMAIN_STEPS) v = std::min(v, nodes / std::max(500.0 / dense, nodes / 512.0));
   return std::max<int64_t>(1, (int64_t)std::min(512.0, v));

@@ -676,7 +676,7 @@ def main():
     ap.add_argument("--delta", type=float, default=0.01, help="reliable-update residual reduction")
     ap.add_argument("--coarse-nodes", type=int, default=0,
                     help="nodes per subdomain of the coarse space (0: the library default, about "
-                         "0.38 nodes^0.55 subdomains, 512 at most)")
+                         "0.46 nodes^0.55 subdomains, 512 at most)")
     ap.add_argument("--fp64-updates", action="store_true",
                     help="--only batch: FP64 reliable updates inside the kernel (no FP32 low parts)")
     ap.add_argument("--only", choices=["mixed", "coarse", "fp64", "spmv", "batch", "assemble"], default=None,

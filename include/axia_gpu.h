@@ -131,7 +131,7 @@ typedef struct axia_solve_opts {
   int32_t spmv_vec;        /* node-block form: blocks per lane load (1, 2, 4; 0 = automatic) */
   int32_t preconditioner;  /* axia_preconditioner (0 = Jacobi) */
   int32_t coarse_nodes;    /* AXIA_PRECOND_COARSE: nodes per subdomain (0 = chosen by the mesh: about
-                              0.38 nodes^0.55 subdomains, more for denser rows, 512 at most; at most
+                              0.46 nodes^0.55 subdomains, more for denser rows, 512 at most; at most
                               682 subdomains per system, in a multi-mesh solve per mesh) */
   int32_t krylov;          /* axia_krylov: batched load cases only (0 = one recurrence per case) */
   int32_t reserved;        /* zero */
