@@ -129,6 +129,7 @@ void free_mesh_state(axia_ctx* ctx) {
   dev_release(ctx, ctx->d_qf32);
   dev_release(ctx, ctx->d_zf32);
   ctx->full_capacity = 0;
+  dev_release(ctx, ctx->d_row_order);
   dev_release(ctx, ctx->d_mB);
   dev_release(ctx, ctx->d_mX);
   dev_release(ctx, ctx->d_mX32);

@@ -19,6 +19,8 @@
 #include "coarse.cuh"
 #include "dword.cuh"
 
+#include <cub/cub.cuh>
+
 namespace {
 
 constexpr int NR = 32;   // load cases per column block
@@ -121,10 +123,10 @@ __device__ __forceinline__ void stc(float* p, const float (&v)[TC]) {
 }
 
 // values of block s: from the row's staging (staged) or the matrix planes
-template <int TC, int TU, bool STAGED>
+template <int NC, int TC, int TU, bool STAGED>
 __device__ __forceinline__ void row_tile(int a, int len, int lane, const RowStage* st, const BsrMatM<float>& M,
                                          const float* X, float (&y)[3][TC]) {
-  constexpr int LG = NR / TC, G = 32 / LG;
+  constexpr int LG = NC / TC, G = 32 / LG;
   const int cl = lane % LG, grp = lane / LG;
   const int beg = STAGED ? 0 : __ldg(M.adj_ptr + a);
 #pragma unroll
@@ -139,7 +141,7 @@ __device__ __forceinline__ void row_tile(int a, int len, int lane, const RowStag
       if (s < len) {
         const int b = STAGED ? st->adj[s] : ld_stream(M.adj + beg + s);
 #pragma unroll
-        for (int j = 0; j < 3; ++j) ldc<TC>(X + (size_t)(3 * b + j) * NR + TC * cl, x[u][j]);
+        for (int j = 0; j < 3; ++j) ldc<TC>(X + (size_t)(3 * b + j) * NC + TC * cl, x[u][j]);
       } else {
 #pragma unroll
         for (int j = 0; j < 3; ++j)
@@ -173,22 +175,24 @@ __device__ __forceinline__ void row_tile(int a, int len, int lane, const RowStag
 // Y[3a+i][4 cl + 2 h + c], c = 0, 1: two of the lane's four load cases in FP64.
 // The FP64 residual of a reliable update runs in two such halves so that the
 // kernel fits the register budget of two blocks per SM.
+template <int NC>
 __device__ __forceinline__ void bsr_row_multi_half(int a, int lane, const BsrMatM<double>& M, const double* X, int h,
                                                    double y[3][2]) {
-  const int cl = lane % LPG, grp = lane / LPG;
+  constexpr int LG = NC / CPL;
+  const int cl = lane % LG, grp = lane / LG;
 #pragma unroll
   for (int i = 0; i < 3; ++i) y[i][0] = y[i][1] = 0.0;
   const int beg = __ldg(M.adj_ptr + a), end = __ldg(M.adj_ptr + a + 1);
   int b = beg + grp < end ? ld_stream(M.adj + beg + grp) : 0;
-  for (int s = beg + grp; s < end; s += 32 / LPG) {
-    const int b_next = s + 32 / LPG < end ? ld_stream(M.adj + s + 32 / LPG) : 0;
+  for (int s = beg + grp; s < end; s += 32 / LG) {
+    const int b_next = s + 32 / LG < end ? ld_stream(M.adj + s + 32 / LG) : 0;
     double v[9];
 #pragma unroll
     for (int k = 0; k < 9; ++k) v[k] = ld_stream(M.val + (long long)k * M.nb + s);
     double x[3][2];
 #pragma unroll
     for (int j = 0; j < 3; ++j) {
-      const double2 t = *reinterpret_cast<const double2*>(X + (size_t)(3 * b + j) * NR + CPL * cl + 2 * h);
+      const double2 t = *reinterpret_cast<const double2*>(X + (size_t)(3 * b + j) * NC + CPL * cl + 2 * h);
       x[j][0] = t.x;
       x[j][1] = t.y;
     }
@@ -202,79 +206,91 @@ __device__ __forceinline__ void bsr_row_multi_half(int a, int lane, const BsrMat
 #pragma unroll
   for (int i = 0; i < 3; ++i)
 #pragma unroll
-    for (int c = 0; c < 2; ++c) {
-      y[i][c] += __shfl_xor_sync(0xffffffffu, y[i][c], 8);
-      y[i][c] += __shfl_xor_sync(0xffffffffu, y[i][c], 16);
-    }
+    for (int c = 0; c < 2; ++c)
+#pragma unroll
+      for (int o = LG; o < 32; o <<= 1) y[i][c] += __shfl_xor_sync(0xffffffffu, y[i][c], o);
 }
 
 // Per-column partial sums of this block: v[c] is this thread's contribution
-// to column TC*(tid % (32/TC))+c (TC = 4: the float4 layout of the vector
+// to column TC*(tid % (NC/TC))+c (TC = 4: the float4 layout of the vector
 // phases).  Written to partials[(slot0 + col) * G + block].
-// one scratch for every instantiation of block_partials_cols (a __shared__
-// array inside the template is allocated once per instantiation: 8 KB each)
-__device__ __forceinline__ double (*cols_scratch())[NR] {
-  __shared__ double s_cols[PCG_THREADS / 32][NR];
-  return s_cols;
+// The sums run in FP64 through shared memory: 63 FP64 warp instructions per
+// block.  (Shuffling converted values in every warp took 208, and GB300
+// issues one per SM about every 18 cycles: 3.6 us per call for two blocks.)
+// FP32 values become FP64 by integer operations (a conversion is an FP64-pipe
+// instruction too).
+struct __align__(16) ColsScratch {
+  union {
+    float f[PCG_THREADS * CPL];
+    double d[PCG_THREADS * 2];  // FP64 inputs: 64 values of a warp at a time
+  };
+  double warp[PCG_THREADS / 32][NR];
+  double quarter[4][NR];
+};
+__device__ __forceinline__ ColsScratch& cols_scratch() {
+  __shared__ ColsScratch s;
+  return s;
 }
+__device__ __forceinline__ double to_f64(float v) { return f32_to_f64_exact(v); }
+__device__ __forceinline__ double to_f64(double v) { return v; }
 
-template <typename A, int TC = CPL>
+template <int NC, int TC, typename A>
 __device__ __forceinline__ void block_partials_cols(const A (&v)[TC], double* partials, int slot0) {
-  constexpr int LG = NR / TC;
-  double (*s_cols)[NR] = cols_scratch();
+  ColsScratch& s = cols_scratch();
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nw = blockDim.x >> 5;
-  double t[TC];
+  // a warp's 32 TC values in order: value e is one of column e % NC, so lane l
+  // adds up values of column l % NC
+  if constexpr (sizeof(A) == sizeof(float)) {
+    stc<TC>(s.f + threadIdx.x * TC, v);
+    __syncthreads();
+    double t = to_f64(s.f[32 * TC * warp + lane]);
 #pragma unroll
-  for (int c = 0; c < TC; ++c) {
-    t[c] = (double)v[c];
+    for (int g = 1; g < TC; ++g) t += to_f64(s.f[32 * (TC * warp + g) + lane]);
+    s.warp[warp][lane] = t;
+  } else {
+    double t = 0.0;
 #pragma unroll
-    for (int o = LG; o < 32; o <<= 1) t[c] += __shfl_xor_sync(0xffffffffu, t[c], o);
-  }
-  if (lane < LG) {
+    for (int h = 0; h < TC; h += 2) {  // 64 of the warp's values at a time
+      const int first = 32 * h;
+      if (lane * TC >= first && lane * TC < first + 64)
 #pragma unroll
-    for (int c = 0; c < TC; ++c) s_cols[warp][TC * lane + c] = t[c];
+        for (int c = 0; c < TC; ++c) s.d[64 * warp + lane * TC + c - first] = v[c];
+      __syncwarp();
+      t += s.d[64 * warp + lane] + s.d[64 * warp + 32 + lane];
+      __syncwarp();
+    }
+    s.warp[warp][lane] = t;
   }
   __syncthreads();
-  if (threadIdx.x < NR) {
-    double s = 0.0;
-    for (int w = 0; w < nw; ++w) s += s_cols[w][threadIdx.x];
-    partials[(size_t)(slot0 + threadIdx.x) * gridDim.x + blockIdx.x] = s;
+  if (warp < 4) {
+    double t = 0.0;
+    for (int w = warp; w < nw; w += 4) t += s.warp[w][lane];
+    s.quarter[warp][lane] = t;
+  }
+  __syncthreads();
+  if (warp == 0) {
+    double t = (s.quarter[0][lane] + s.quarter[1][lane]) + (s.quarter[2][lane] + s.quarter[3][lane]);
+#pragma unroll
+    for (int o = NC; o < 32; o <<= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
+    if (lane < NC) partials[(size_t)(slot0 + lane) * gridDim.x + blockIdx.x] = t;
   }
 }
 
-// Reduce-and-sync over nv partial slots; the last block to arrive sums them
-// (one warp per slot, ascending block order) and publishes totals[slot0..].
+// Reduce-and-sync over nv partial slots: after a barrier the slots are shared
+// out over the blocks, one warp per slot (ascending block order), and a second
+// barrier publishes totals[slot0..].  One block alone would add 64 x 304 FP64
+// values, 9 us on its SM.
 __device__ __forceinline__ bool grid_reduce_sync_wide(GridBarrier* bar, DevStatus* st, unsigned long long limit_ns,
                                                       const double* partials, double* totals, int slot0, int nv) {
-  __shared__ int s_last, s_ok;
-  __shared__ unsigned s_gen;
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    int last;
-    s_gen = barrier_arrive(bar, gridDim.x, &last);
-    s_last = last;
+  if (!grid_sync(bar, st, limit_ns)) return false;
+  const int lane = threadIdx.x & 31;
+  for (int k = blockIdx.x + (int)gridDim.x * (int)(threadIdx.x >> 5); k < nv; k += gridDim.x * (blockDim.x >> 5)) {
+    const int cnt = lane < (int)gridDim.x ? ((int)gridDim.x - lane + 31) / 32 : 0;
+    double a = ldcg_sum(partials + (size_t)(slot0 + k) * gridDim.x + lane, 32, cnt);
+    a = warp_sum(a);
+    if (lane == 0) totals[slot0 + k] = a;
   }
-  __syncthreads();
-  int ok = 1;
-  if (s_last) {
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nw = blockDim.x >> 5;
-    for (int k = warp; k < nv; k += nw) {
-      const int cnt = lane < (int)gridDim.x ? ((int)gridDim.x - lane + 31) / 32 : 0;
-      double a = ldcg_sum(partials + (size_t)(slot0 + k) * gridDim.x + lane, 32, cnt);
-      a = warp_sum(a);
-      if (lane == 0) totals[slot0 + k] = a;
-    }
-    __syncthreads();
-    if (threadIdx.x == 0) {
-      __threadfence();
-      barrier_release(bar, s_gen);
-    }
-  } else if (threadIdx.x == 0) {
-    ok = barrier_wait(bar, st, limit_ns, s_gen);
-  }
-  if (threadIdx.x == 0) s_ok = ok;
-  __syncthreads();
-  return s_ok != 0;
+  return grid_sync(bar, st, limit_ns);
 }
 
 struct MultiOut {
@@ -299,6 +315,7 @@ struct BatchState {
 };
 
 struct MultiArgs {
+  const int* order;     // [n_nodes] block rows in the order the SpMV takes them (batch_row_order)
   BsrMatM<float> M32;
   BsrMatM<double> M64;
   int nd;
@@ -324,7 +341,7 @@ struct MultiArgs {
   int resume = 0;       // start from state, after an update whose |r|^2 and r.D^-1 r are in totals
 };
 
-constexpr int SL_A = 0, SL_B = NR;  // two banks of NR slots
+constexpr int SL_A = 0;  // two banks of NC slots: SL_A .. and NC ..
 
 // ---------------------------------------------------------------------------
 // Two-level preconditioner for 32 columns (the single-column form is in
@@ -334,83 +351,114 @@ constexpr int SL_A = 0, SL_B = NR;  // two banks of NR slots
 // y = M r_c as tasks (row, column quad) with lanes over the coarse unknowns;
 // the prolongation inside the search-direction update.
 // ---------------------------------------------------------------------------
-__device__ __forceinline__ void coarse_restrict_m(const CoarseArgs& C, const float* R, int gwarp, int nwarps,
-                                                  int lane) {
-  const int cl = lane % LPG, grp = lane / LPG;
-  for (int ci = C.chunk_lo + gwarp; ci < C.chunk_hi; ci += nwarps) {
+// Chunk ci of subdomain I is summed in part_m; the warp that finishes the last
+// chunk of I adds the chunk sums in chunk order into r_c.
+template <int NC>
+__device__ __forceinline__ void coarse_chunk_finish_m(const CoarseArgs& C, int I, int lane) {
+  __threadfence();
+  __syncwarp();
+  const int c0 = __ldg(C.chunk_ptr + I), c1 = __ldg(C.chunk_ptr + I + 1);
+  int last = 0;
+  if (lane == 0) last = atomicAdd(C.cnt + I, 1) == c1 - c0 - 1;
+  last = __shfl_sync(0xffffffffu, last, 0);
+  if (last) {
+    __threadfence();
+    for (int e = lane; e < 6 * NC; e += 32)
+      C.rc_m[(size_t)6 * I * NC + e] = ldcg_sum(C.part_m + (size_t)c0 * 6 * NC + e, (size_t)6 * NC, c1 - c0);
+    if (lane == 0) atomicExch(C.cnt + I, 0);
+  }
+}
+
+// The restriction of R over the chunks; with UPDATE, the CG update r -= alpha q
+// in the same pass with the per-case sums of r.r and r.D^-1 r.  A lane takes
+// two load cases of a node (32 cases: 16 lanes per node, two nodes per warp and step): a
+// node's rows are contiguous, so the subdomain order costs no bandwidth, and
+// the registers hold a whole node's loads.
+template <int NC, bool UPDATE>
+__device__ __forceinline__ void coarse_restrict_m(const CoarseArgs& C, const float* s_alpha, float* R, const float* Q,
+                                                  const float* dinv, int cwarp, int nwarps, int lane, float (&rr)[2],
+                                                  float (&rz)[2]) {
+  constexpr int LG = NC / 2, NS = 32 / LG;  // lanes per node, nodes per step
+  const int c0 = 2 * (lane % LG), grp = lane / LG;
+  for (int ci = C.chunk_lo + cwarp; ci < C.chunk_hi; ci += nwarps) {
     const int4 ch = C.chunk[ci];
-    float v[6][CPL];
+    float v[6][2];
 #pragma unroll
-    for (int i = 0; i < 6; ++i)
-#pragma unroll
-      for (int c = 0; c < CPL; ++c) v[i][c] = 0.f;
-#pragma unroll 2
-    for (int k = ch.y + grp; k < ch.z; k += 32 / LPG) {
-      const int a = __ldg(C.sub_node + k);
+    for (int i = 0; i < 6; ++i) v[i][0] = v[i][1] = 0.f;
+    int k = ch.y + grp;
+    int a = k < ch.z ? __ldg(C.sub_node + k) : 0;
+    while (k < ch.z) {
       const float4 g = __ldg(C.geo + a);
       const unsigned m = geo_bits(g);
-      float r[3][CPL];
+      float2 r[3], q[3];
+      float di[3];
+      const size_t o = (size_t)(3 * a) * NC + c0;
 #pragma unroll
       for (int d = 0; d < 3; ++d) {
-        if ((m >> d) & 1u) {
-          ld4(R + (size_t)(3 * a + d) * NR + CPL * cl, r[d]);
-        } else {
-#pragma unroll
-          for (int c = 0; c < CPL; ++c) r[d][c] = 0.f;
+        r[d] = *reinterpret_cast<const float2*>(R + o + d * NC);
+        if (UPDATE) {
+          q[d] = *reinterpret_cast<const float2*>(Q + o + d * NC);
+          di[d] = __ldg(dinv + 3 * a + d);
         }
       }
+      k += NS;
+      a = k < ch.z ? __ldg(C.sub_node + k) : 0;
 #pragma unroll
-      for (int c = 0; c < CPL; ++c) {
-        v[0][c] += r[0][c];
-        v[1][c] += r[1][c];
-        v[2][c] += r[2][c];
-        v[3][c] = fmaf(g.y, r[2][c], fmaf(-g.z, r[1][c], v[3][c]));
-        v[4][c] = fmaf(g.z, r[0][c], fmaf(-g.x, r[2][c], v[4][c]));
-        v[5][c] = fmaf(g.x, r[1][c], fmaf(-g.y, r[0][c], v[5][c]));
+      for (int d = 0; d < 3; ++d) {
+        if (UPDATE) {
+          r[d].x = fmaf(-s_alpha[c0], q[d].x, r[d].x);
+          r[d].y = fmaf(-s_alpha[c0 + 1], q[d].y, r[d].y);
+          *reinterpret_cast<float2*>(R + o + d * NC) = r[d];
+          rr[0] = fmaf(r[d].x, r[d].x, rr[0]);
+          rr[1] = fmaf(r[d].y, r[d].y, rr[1]);
+          rz[0] = fmaf(r[d].x, r[d].x * di[d], rz[0]);
+          rz[1] = fmaf(r[d].y, r[d].y * di[d], rz[1]);
+        }
+        if (!((m >> d) & 1u)) r[d] = make_float2(0.f, 0.f);
+      }
+#pragma unroll
+      for (int c = 0; c < 2; ++c) {
+        const float x = c ? r[0].y : r[0].x, y = c ? r[1].y : r[1].x, z = c ? r[2].y : r[2].x;
+        v[0][c] += x;
+        v[1][c] += y;
+        v[2][c] += z;
+        v[3][c] = fmaf(g.y, z, fmaf(-g.z, y, v[3][c]));
+        v[4][c] = fmaf(g.z, x, fmaf(-g.x, z, v[4][c]));
+        v[5][c] = fmaf(g.x, y, fmaf(-g.y, x, v[5][c]));
       }
     }
 #pragma unroll
-    for (int i = 0; i < 6; ++i)
+    for (int i = 0; i < 6; ++i) {
 #pragma unroll
-      for (int c = 0; c < CPL; ++c) {
-        v[i][c] += __shfl_xor_sync(0xffffffffu, v[i][c], 8);
-        v[i][c] += __shfl_xor_sync(0xffffffffu, v[i][c], 16);
+      for (int o = LG; o < 32; o <<= 1) {
+        v[i][0] += __shfl_xor_sync(0xffffffffu, v[i][0], o);
+        v[i][1] += __shfl_xor_sync(0xffffffffu, v[i][1], o);
       }
-    if (grp == 0)
-#pragma unroll
-      for (int i = 0; i < 6; ++i) st4(C.part_m + ((size_t)ci * 6 + i) * NR + CPL * cl, v[i]);
-    __threadfence();
-    __syncwarp();
-    const int I = ch.x, c0 = __ldg(C.chunk_ptr + I), c1 = __ldg(C.chunk_ptr + I + 1);
-    int last = 0;
-    if (lane == 0) last = atomicAdd(C.cnt + I, 1) == c1 - c0 - 1;
-    last = __shfl_sync(0xffffffffu, last, 0);
-    if (last) {
-      __threadfence();
-#pragma unroll
-      for (int i = 0; i < 6; ++i)
-        C.rc_m[(size_t)(6 * I + i) * NR + lane] =
-            ldcg_sum(C.part_m + ((size_t)c0 * 6 + i) * NR + lane, (size_t)6 * NR, c1 - c0);
-      if (lane == 0) atomicExch(C.cnt + I, 0);
+      if (grp == 0) *reinterpret_cast<float2*>(C.part_m + ((size_t)ci * 6 + i) * NC + c0) = make_float2(v[i][0], v[i][1]);
     }
+    coarse_chunk_finish_m<NC>(C, ch.x, lane);
   }
 }
 
 // Y = M R_c; per column r_c . y into partials[(slot0 + col) * G + block].
-// Tasks of 16 rows go to the blocks in turn; a thread owns one (row, load
-// case).  The task walks the columns of M in tiles of 64: the tile of R_c
-// (64 x 32, contiguous) and the 16 x 64 tile of M are copied into a 3-stage
-// shared-memory ring with cp.async, two tiles ahead of the one being summed,
-// so a task keeps ~24 KB in flight instead of waiting one memory round trip
-// per tile.  `ring` is COARSE_RING_FLOATS of 16-byte aligned shared memory.
-// The per-column sums run over the block's tasks and rows in a fixed order.
-constexpr int CS_TJ = 64;                          // columns of M per tile
-constexpr int CS_TR = PCG_THREADS / NR;            // rows per task (16)
-constexpr int CS_STAGE = CS_TJ * NR + CS_TR * CS_TJ;  // floats per stage: R_c tile + M tile
-constexpr int COARSE_RING_FLOATS = 3 * CS_STAGE;
+// Tasks of 16 rows of Y go to the blocks in turn.  The 16 warps of a block
+// share out the columns of M; each streams its columns (M is symmetric: row k,
+// columns i0 ..) and rows of R_c through its own 3-stage cp.async ring, 4
+// columns a stage, and a lane owns 2 rows x NC / 4 cases (32 cases: 16
+// multiply-adds for five shared loads).  The warps' partial tiles are added in warp order.
+// Bound: L2 latency over the ring.  Measured with its barriers at 3072
+// unknowns: one output per thread from block-wide tiles (two shared loads per
+// multiply-add) 94 us, the loads straight to registers 61 us.
+constexpr int CS_TR = 16;                                   // rows per task
+constexpr int CS_WARPS = PCG_THREADS / 32;
+constexpr int CS_K = 4;                                     // columns per stage
+constexpr int CS_STAGE = CS_K * (NR + CS_TR);               // floats: R_c rows, M rows
+constexpr int CS_RING = 3 * CS_STAGE;                       // per warp; holds its partial tile at the end
+static_assert(CS_RING >= CS_TR * NR, "the partial tile reuses the warp's ring");
+constexpr int COARSE_RING_FLOATS = CS_WARPS * CS_RING;
 
 // dynamic shared memory of the 32-case kernel: the row staging of the SpMV
-// phase and the coarse solve's ring take turns in it
+// phase and the coarse solve's tiles take turns in it
 constexpr size_t DYN_BYTES =
     STAGE_BYTES > COARSE_RING_FLOATS * sizeof(float) ? STAGE_BYTES : COARSE_RING_FLOATS * sizeof(float);
 
@@ -419,61 +467,89 @@ __device__ __forceinline__ void cp_async16(float* smem, const float* gmem) {
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(s), "l"(gmem) : "memory");
 }
 
+template <int NC>
 __device__ __forceinline__ void coarse_solve_m(const CoarseArgs& C, float* ring, double* partials, int slot0) {
   __shared__ float s_prod[PCG_THREADS];
-  __shared__ float s_cc[NR];
-  const int r = threadIdx.x / NR, c = threadIdx.x % NR;
-  if (threadIdx.x < NR) s_cc[threadIdx.x] = 0.f;
+  __shared__ float s_cc[NC];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  constexpr int W = NC / 4;  // cases per lane
+  constexpr int STAGE = CS_K * (NC + CS_TR);
+  const int r2 = 2 * (lane & 7), cw = W * (lane >> 3);
+  if (threadIdx.x < NC) s_cc[threadIdx.x] = 0.f;
   const int ntask = (C.nc + CS_TR - 1) / CS_TR;
-  const int nt = C.ldm / CS_TJ;  // tiles per row of M (ldm is a multiple of 64; zero past nc)
+  const int kw = C.ldm / CS_WARPS, nt = kw / CS_K;  // ldm is a multiple of 64; M and R_c are zero past nc
+  float* const wr = ring + warp * CS_RING;
   for (int task = blockIdx.x; task < ntask; task += gridDim.x) {
     const int i0 = task * CS_TR;
-    // thread t copies 16 bytes of the R_c tile and (t < 256) 16 bytes of the M tile
+    float y[2][W];
+#pragma unroll
+    for (int q = 0; q < W; ++q) y[0][q] = y[1][q] = 0.f;
+    const float* m = C.minv + (size_t)(warp * kw + (lane >> 2)) * C.ldm + i0 + 4 * (lane & 3);
+    const float* rc = C.rc_m + (size_t)(warp * kw) * NC + 4 * lane;
     auto issue = [&](int t) {
       if (t < nt) {
-        float* st = ring + (t % 3) * CS_STAGE;
-        const int jj = threadIdx.x >> 3, cc = 4 * (threadIdx.x & 7);
-        cp_async16(st + jj * NR + cc, C.rc_m + (size_t)(t * CS_TJ + jj) * NR + cc);
-        if (threadIdx.x < CS_TR * CS_TJ / 4) {
-          const int rr = threadIdx.x >> 4, kk = 4 * (threadIdx.x & 15);
-          cp_async16(st + CS_TJ * NR + rr * CS_TJ + kk, C.minv + (size_t)(i0 + rr) * C.ldm + t * CS_TJ + kk);
-        }
+        float* st = wr + (t % 3) * STAGE;
+        if (lane < CS_K * NC / 4) cp_async16(st + 4 * lane, rc + (size_t)t * CS_K * NC);
+        if (lane < CS_K * CS_TR / 4) cp_async16(st + CS_K * NC + 4 * lane, m + (size_t)t * CS_K * C.ldm);
       }
-      asm volatile("cp.async.commit_group;" ::: "memory");
+      cp_async_commit();
     };
-    __syncthreads();  // the ring is free (the previous task's readers are done)
+    __syncthreads();  // the rings (the previous task's partial tiles) are read
     issue(0);
     issue(1);
-    float y = 0.f;
     for (int t = 0; t < nt; ++t) {
-      asm volatile("cp.async.wait_group 1;" ::: "memory");  // tile t has landed
-      __syncthreads();
-      issue(t + 2);  // into the stage tile t - 1 used; every thread is past it
-      const float* st = ring + (t % 3) * CS_STAGE;
-      const float* mt = st + CS_TJ * NR + r * CS_TJ;
-#pragma unroll 8
-      for (int jj = 0; jj < CS_TJ; ++jj) y = fmaf(mt[jj], st[jj * NR + c], y);
+      issue(t + 2);
+      cp_async_wait<2>();  // stage t has landed
+      __syncwarp();
+      const float* st = wr + (t % 3) * STAGE;
+#pragma unroll
+      for (int k = 0; k < CS_K; ++k) {
+        const float2 mv = *reinterpret_cast<const float2*>(st + CS_K * NC + k * CS_TR + r2);
+        float v[W];
+#pragma unroll
+        for (int q = 0; q < W; q += 2) {
+          const float2 f = *reinterpret_cast<const float2*>(st + k * NC + cw + q);
+          v[q] = f.x;
+          v[q + 1] = f.y;
+        }
+#pragma unroll
+        for (int q = 0; q < W; ++q) {
+          y[0][q] = fmaf(mv.x, v[q], y[0][q]);
+          y[1][q] = fmaf(mv.y, v[q], y[1][q]);
+        }
+      }
+      __syncwarp();  // stage t is read before stage t + 3 lands on it
     }
-    asm volatile("cp.async.wait_group 0;" ::: "memory");
-    const int i = i0 + r;
-    float prod = 0.f;
-    if (i < C.nc) {
-      C.yc_m[(size_t)i * NR + c] = y;
-      prod = __ldcg(C.rc_m + (size_t)i * NR + c) * y;
+    cp_async_wait<0>();
+    __syncwarp();
+#pragma unroll
+    for (int h = 0; h < 2; ++h)
+#pragma unroll
+      for (int q = 0; q < W; q += 2)
+        *reinterpret_cast<float2*>(wr + (r2 + h) * NC + cw + q) = make_float2(y[h][q], y[h][q + 1]);
+    __syncthreads();
+    const int i = i0 + threadIdx.x / NC, c = threadIdx.x % NC;
+    float s = 0.f, prod = 0.f;
+    if (threadIdx.x < CS_TR * NC && i < C.nc) {
+#pragma unroll
+      for (int w = 0; w < CS_WARPS; ++w) s += ring[w * CS_RING + threadIdx.x];
+      C.yc_m[(size_t)i * NC + c] = s;
+      prod = __ldcg(C.rc_m + (size_t)i * NC + c) * s;
     }
     s_prod[threadIdx.x] = prod;
     __syncthreads();
-    if (threadIdx.x < NR) {
+    if (threadIdx.x < NC) {
       float sum = s_cc[threadIdx.x];
-      for (int q = 0; q < CS_TR; ++q) sum += s_prod[q * NR + threadIdx.x];
+      for (int q = 0; q < CS_TR; ++q) sum += s_prod[q * NC + threadIdx.x];
       s_cc[threadIdx.x] = sum;
     }
   }
   __syncthreads();
-  if (threadIdx.x < NR) partials[(size_t)(slot0 + threadIdx.x) * gridDim.x + blockIdx.x] = (double)s_cc[threadIdx.x];
+  if (threadIdx.x < NC) partials[(size_t)(slot0 + threadIdx.x) * gridDim.x + blockIdx.x] = to_f64(s_cc[threadIdx.x]);
 }
 
 // coarse part of z at DOF row `row`, columns c0..c0+3
+template <int NC>
 __device__ __forceinline__ void coarse_prolong_m(const CoarseArgs& C, long long row, int c0, float zc[CPL]) {
   const int a = (int)(row / 3), d = (int)(row - 3LL * a);
   const float4 g = __ldg(C.geo + a);
@@ -481,30 +557,36 @@ __device__ __forceinline__ void coarse_prolong_m(const CoarseArgs& C, long long 
 #pragma unroll
   for (int c = 0; c < CPL; ++c) zc[c] = 0.f;
   if (!((m >> d) & 1u)) return;
-  const float* Y = C.yc_m + (size_t)(6 * (m >> 3)) * NR + c0;
+  const float* Y = C.yc_m + (size_t)(6 * (m >> 3)) * NC + c0;
   float t[CPL], u[CPL], w[CPL];
   float cu, cw;
   if (d == 0) {
-    ld4(Y, t), ld4(Y + 4 * NR, u), ld4(Y + 5 * NR, w), cu = g.z, cw = -g.y;
+    ld4(Y, t), ld4(Y + 4 * NC, u), ld4(Y + 5 * NC, w), cu = g.z, cw = -g.y;
   } else if (d == 1) {
-    ld4(Y + NR, t), ld4(Y + 3 * NR, u), ld4(Y + 5 * NR, w), cu = -g.z, cw = g.x;
+    ld4(Y + NC, t), ld4(Y + 3 * NC, u), ld4(Y + 5 * NC, w), cu = -g.z, cw = g.x;
   } else {
-    ld4(Y + 2 * NR, t), ld4(Y + 3 * NR, u), ld4(Y + 4 * NR, w), cu = g.y, cw = -g.x;
+    ld4(Y + 2 * NC, t), ld4(Y + 3 * NC, u), ld4(Y + 4 * NC, w), cu = g.y, cw = -g.x;
   }
 #pragma unroll
   for (int c = 0; c < CPL; ++c) zc[c] = fmaf(cu, u[c], fmaf(cw, w[c], t[c]));
 }
 
-// the coarse half of the preconditioner for the current R32: restriction,
-// barrier, Y = M R_c and the per-column r . Z y reduced into totals[SL_A..]
-__device__ __forceinline__ bool coarse_step_m(const MultiArgs& P, int gwarp, int nwarps, int lane, float* ring) {
-  coarse_restrict_m(P.C, P.R32, gwarp, nwarps, lane);
-  if (!grid_sync(P.bar, P.st, P.limit_ns)) return false;
-  coarse_solve_m(P.C, ring, P.partials, SL_A);
-  return grid_reduce_sync_wide(P.bar, P.st, P.limit_ns, P.partials, P.totals, SL_A, NR);
+// the coarse half of the preconditioner for the current R32: restriction and a
+// barrier (unless the update did them), Y = M R_c and the per-column r . Z y
+// reduced into totals[SL_A..]
+template <int NC>
+__device__ __forceinline__ bool coarse_step_m(const MultiArgs& P, bool restricted, int cwarp, int nwarps, int lane,
+                                              float* ring) {
+  if (!restricted) {
+    float none[2];
+    coarse_restrict_m<NC, false>(P.C, nullptr, P.R32, nullptr, nullptr, cwarp, nwarps, lane, none, none);
+    if (!grid_sync(P.bar, P.st, P.limit_ns)) return false;
+  }
+  coarse_solve_m<NC>(P.C, ring, P.partials, SL_A);
+  return grid_reduce_sync_wide(P.bar, P.st, P.limit_ns, P.partials, P.totals, SL_A, NC);
 }
 
-template <bool COARSE, int TC, int TU>
+template <bool COARSE, int NC, int TC, int TU>
 __global__ void __launch_bounds__(PCG_THREADS, 2) pcg_bsr_multi_kernel(MultiArgs P) {
   extern __shared__ __align__(16) RowStage s_stage[];  // DYN_BYTES: row staging, or the coarse solve's ring
   float* const ring = reinterpret_cast<float*>(s_stage);
@@ -513,12 +595,15 @@ __global__ void __launch_bounds__(PCG_THREADS, 2) pcg_bsr_multi_kernel(MultiArgs
   __shared__ int s_active[NR], s_flag, s_restart[NR];
   __shared__ double s_rrec[NR];  // recurrence |r| of each case when the last update was triggered
   __shared__ long long s_citers[NR];
+  constexpr int LG4 = NC / CPL;  // float4 chunks of a vector row
+  constexpr int SL_B = NC;
   const int nd = P.nd, n_nodes = P.M32.n_nodes;
   const int tid = blockIdx.x * blockDim.x + threadIdx.x, nth = gridDim.x * blockDim.x;
   const int lane = threadIdx.x & 31;
   const int gwarp = tid >> 5, nwarps = nth >> 5;
-  const int cq = tid % LPG;            // this thread's column quad in the vector phases
-  const long long nq = (long long)nd * LPG;  // float4 chunks of an [nd][NR] vector
+  // restriction chunks go to the warps of different blocks first
+  const int cwarp = (int)(threadIdx.x >> 5) * (int)gridDim.x + (int)blockIdx.x;
+  const long long nq = (long long)nd * LG4;  // float4 chunks of an [nd][NC] vector
   // the bookkeeping after a reliable update whose |r|^2 (slots SL_A) is in
   // totals.  A case whose true residual came back more than twice its
   // recurrence residual restarts its search direction (beta = 0): the
@@ -527,7 +612,7 @@ __global__ void __launch_bounds__(PCG_THREADS, 2) pcg_bsr_multi_kernel(MultiArgs
   // converging.
   auto after_update = [&](int& updates) {
     ++updates;
-    if (threadIdx.x < NR) {
+    if (threadIdx.x < NC) {
       const int c = threadIdx.x;
       const double rn = sqrt(__ldcg(P.totals + SL_A + c));
       s_restart[c] = 0;
@@ -541,11 +626,13 @@ __global__ void __launch_bounds__(PCG_THREADS, 2) pcg_bsr_multi_kernel(MultiArgs
     __syncthreads();
   };
   // the end of an iteration: the coarse correction of r, beta, p = z + beta p
-  auto iteration_tail = [&]() -> bool {
+  // and, with add_x, x += alpha p for the old p (the x / r update leaves it to
+  // this pass, which reads p anyway)
+  auto iteration_tail = [&](bool add_x) -> bool {
     if constexpr (COARSE) {
-      if (!coarse_step_m(P, gwarp, nwarps, lane, ring)) return false;
+      if (!coarse_step_m<NC>(P, add_x, cwarp, nwarps, lane, ring)) return false;
     }
-    if (threadIdx.x < NR) {
+    if (threadIdx.x < NC) {
       const int c = threadIdx.x;
       double rzn = __ldcg(P.totals + SL_B + c);
       if constexpr (COARSE) rzn += __ldcg(P.totals + SL_A + c);
@@ -555,12 +642,19 @@ __global__ void __launch_bounds__(PCG_THREADS, 2) pcg_bsr_multi_kernel(MultiArgs
     }
     __syncthreads();
     for (long long q = tid; q < nq; q += nth) {
-      const long long row = q / LPG;
-      const int c0 = CPL * (int)(q % LPG);
+      const long long row = q / LG4;
+      const int c0 = CPL * (int)(q % LG4);
       float p[CPL], r[CPL], zc[CPL] = {0.f, 0.f, 0.f, 0.f};
       ld4(P.P32 + q * CPL, p);
       ld4(P.R32 + q * CPL, r);
-      if constexpr (COARSE) coarse_prolong_m(P.C, row, c0, zc);
+      if (add_x) {
+        float x[CPL];
+        ld4(P.X32 + q * CPL, x);
+#pragma unroll
+        for (int c = 0; c < CPL; ++c) x[c] = fmaf(s_alpha[c0 + c], p[c], x[c]);
+        st4(P.X32 + q * CPL, x);
+      }
+      if constexpr (COARSE) coarse_prolong_m<NC>(P.C, row, c0, zc);
       const float di = P.dinv32[row];
 #pragma unroll
       for (int c = 0; c < CPL; ++c)
@@ -588,14 +682,20 @@ __global__ void __launch_bounds__(PCG_THREADS, 2) pcg_bsr_multi_kernel(MultiArgs
     updates0 = P.state->updates;
     __syncthreads();
     after_update(updates0);
-    if (!iteration_tail()) return;
+    if (!iteration_tail(false)) return;
   }
   // init: x = 0, r32 = b, p = z = r32 / diag, per-column r.z and b.b
   if (!P.resume) {
+    if (threadIdx.x < NR) {  // columns past NC stay idle
+      const int c = threadIdx.x;
+      s_rz[c] = s_bnorm[c] = s_rmax[c] = s_res[c] = s_rrec[c] = 0.0;
+      s_active[c] = s_restart[c] = 0;
+      s_citers[c] = 0;
+    }
     float rz_p[CPL] = {0, 0, 0, 0};
     double bb_p[CPL] = {0, 0, 0, 0};
     for (long long q = tid; q < nq; q += nth) {
-      const long long row = q / LPG;
+      const long long row = q / LG4;
       double bv[CPL];
       ld4(P.B + q * CPL, bv);
       const float di = P.dinv32[row];
@@ -614,13 +714,13 @@ __global__ void __launch_bounds__(PCG_THREADS, 2) pcg_bsr_multi_kernel(MultiArgs
       st4(P.R32 + q * CPL, r);
       st4(P.P32 + q * CPL, z);
     }
-    block_partials_cols<double>(bb_p, P.partials, SL_A);
+    block_partials_cols<NC, CPL>(bb_p, P.partials, SL_A);
     __syncthreads();
-    block_partials_cols<float>(rz_p, P.partials, SL_B);
+    block_partials_cols<NC, CPL>(rz_p, P.partials, SL_B);
   }
   if (!P.resume) {
-  if (!grid_reduce_sync_wide(P.bar, P.st, P.limit_ns, P.partials, P.totals, 0, 2 * NR)) return;
-  if (threadIdx.x < NR) {
+  if (!grid_reduce_sync_wide(P.bar, P.st, P.limit_ns, P.partials, P.totals, 0, 2 * NC)) return;
+  if (threadIdx.x < NC) {
     const int c = threadIdx.x;
     s_bnorm[c] = sqrt(__ldcg(P.totals + SL_A + c));
     s_rz[c] = __ldcg(P.totals + SL_B + c);
@@ -634,12 +734,12 @@ __global__ void __launch_bounds__(PCG_THREADS, 2) pcg_bsr_multi_kernel(MultiArgs
   }
   __syncthreads();
   if constexpr (COARSE) {  // P = D^-1 B + Z M Z^T B
-    if (!coarse_step_m(P, gwarp, nwarps, lane, ring)) return;
-    if (threadIdx.x < NR) s_rz[threadIdx.x] += __ldcg(P.totals + SL_A + threadIdx.x);
+    if (!coarse_step_m<NC>(P, false, cwarp, nwarps, lane, ring)) return;
+    if (threadIdx.x < NC) s_rz[threadIdx.x] += __ldcg(P.totals + SL_A + threadIdx.x);
     for (long long q = tid; q < nq; q += nth) {
       float p[CPL], zc[CPL];
       ld4(P.P32 + q * CPL, p);
-      coarse_prolong_m(P.C, q / LPG, CPL * (int)(q % LPG), zc);
+      coarse_prolong_m<NC>(P.C, q / LG4, CPL * (int)(q % LG4), zc);
 #pragma unroll
       for (int c = 0; c < CPL; ++c) p[c] += zc[c];
       st4(P.P32 + q * CPL, p);
@@ -651,7 +751,7 @@ __global__ void __launch_bounds__(PCG_THREADS, 2) pcg_bsr_multi_kernel(MultiArgs
   int updates = updates0, status = AXIA_OK;
   for (long long it = it0; it < P.max_iter; ++it) {
     int any = 0;
-    for (int c = 0; c < NR; ++c) any |= s_active[c];
+    for (int c = 0; c < NC; ++c) any |= s_active[c];
     if (!any) break;
     iters = it + 1;
     // Q = K P (FP32) and per-column p.q
@@ -659,36 +759,47 @@ __global__ void __launch_bounds__(PCG_THREADS, 2) pcg_bsr_multi_kernel(MultiArgs
 #pragma unroll
     for (int c = 0; c < TC; ++c) pq_p[c] = 0.f;
     RowStage* const stg = s_stage + 2 * (threadIdx.x >> 5);
-    stage_row(gwarp, lane, P.M32, stg);
+    // the blocks take tiles of 16 or 64 rows of the space-filling order in
+    // turn, a warp every 16th row of a tile (16: a mesh of few tiles per block
+    // would leave blocks idle in the last round)
+    const int nw = blockDim.x >> 5, lt = n_nodes >= 32 * nwarps ? 2 : 0;
+    auto row_index = [&](int j) {  // this warp's j-th row
+      return ((((j >> lt) * (int)gridDim.x + (int)blockIdx.x) << lt) + (j & ((1 << lt) - 1))) * nw +
+             (int)(threadIdx.x >> 5);
+    };
+    int a = row_index(0) < n_nodes ? __ldg(P.order + row_index(0)) : n_nodes;
+    stage_row(a, lane, P.M32, stg);
     int kb = 0;
-    for (int a = gwarp; a < n_nodes; a += nwarps, kb ^= 1) {
-      stage_row(a + nwarps, lane, P.M32, stg + (kb ^ 1));
+    for (int j = 0; row_index(j) < n_nodes; ++j, kb ^= 1) {
+      const int next = row_index(j + 1) < n_nodes ? __ldg(P.order + row_index(j + 1)) : n_nodes;
+      stage_row(next, lane, P.M32, stg + (kb ^ 1));
       cp_async_wait<1>();  // this row's copies (all but the group just opened)
       __syncwarp();
       float y[3][TC];
       const int len = __ldg(P.M32.adj_ptr + a + 1) - __ldg(P.M32.adj_ptr + a);
       if (len <= STAGE_B)
-        row_tile<TC, TU, true>(a, len, lane, stg + kb, P.M32, P.P32, y);
+        row_tile<NC, TC, TU, true>(a, len, lane, stg + kb, P.M32, P.P32, y);
       else
-        row_tile<TC, TU, false>(a, len, lane, stg + kb, P.M32, P.P32, y);
+        row_tile<NC, TC, TU, false>(a, len, lane, stg + kb, P.M32, P.P32, y);
       __syncwarp();  // every lane is done with stg[kb] before it is refilled
-      if (lane < NR / TC) {
+      if (lane < NC / TC) {
 #pragma unroll
-        for (int i = 0; i < 3; ++i) {
-          const size_t off = (size_t)(3 * a + i) * NR + TC * lane;
+        for (int d = 0; d < 3; ++d) {
+          const size_t off = (size_t)(3 * a + d) * NC + TC * lane;
           float p[TC];
           ldc<TC>(P.P32 + off, p);
-          stc<TC>(P.Q32 + off, y[i]);
+          stc<TC>(P.Q32 + off, y[d]);
 #pragma unroll
-          for (int c = 0; c < TC; ++c) pq_p[c] = fmaf(p[c], y[i][c], pq_p[c]);
+          for (int c = 0; c < TC; ++c) pq_p[c] = fmaf(p[c], y[d][c], pq_p[c]);
         }
       }
+      a = next;
     }
     cp_async_wait<0>();  // the last (empty or unused) group
-    // lanes 0 .. 32/TC - 1 hold the columns TC lane .. TC lane + TC - 1 of their warp
-    block_partials_cols<float, TC>(pq_p, P.partials, SL_A);
-    if (!grid_reduce_sync_wide(P.bar, P.st, P.limit_ns, P.partials, P.totals, SL_A, NR)) return;
-    if (threadIdx.x < NR) {
+    // lanes 0 .. NC/TC - 1 hold the columns TC lane .. TC lane + TC - 1 of their warp
+    block_partials_cols<NC, TC>(pq_p, P.partials, SL_A);
+    if (!grid_reduce_sync_wide(P.bar, P.st, P.limit_ns, P.partials, P.totals, SL_A, NC)) return;
+    if (threadIdx.x < NC) {
       const int c = threadIdx.x;
       const double pq = __ldcg(P.totals + SL_A + c);
       float al = 0.f;
@@ -704,45 +815,55 @@ __global__ void __launch_bounds__(PCG_THREADS, 2) pcg_bsr_multi_kernel(MultiArgs
       s_alpha[c] = al;
     }
     __syncthreads();
-    float rr_p[CPL] = {0, 0, 0, 0}, rzn_p[CPL] = {0, 0, 0, 0};
-    for (long long q = tid; q < nq; q += nth) {
-      const long long row = q / LPG;
-      const int c0 = CPL * (int)(q % LPG);
-      float x[CPL], r[CPL], p[CPL], qq[CPL];
-      ld4(P.X32 + q * CPL, x);
-      ld4(P.R32 + q * CPL, r);
-      ld4(P.P32 + q * CPL, p);
-      ld4(P.Q32 + q * CPL, qq);
-      const float di = P.dinv32[row];
+    if constexpr (COARSE) {
+      float rr_p[2] = {0.f, 0.f}, rzn_p[2] = {0.f, 0.f};
+      coarse_restrict_m<NC, true>(P.C, s_alpha, P.R32, P.Q32, P.dinv32, cwarp, nwarps, lane, rr_p, rzn_p);
+      block_partials_cols<NC, 2>(rr_p, P.partials, SL_A);
+      __syncthreads();  // the scratch is read
+      block_partials_cols<NC, 2>(rzn_p, P.partials, SL_B);
+    } else {
+      float rr_p[CPL] = {0, 0, 0, 0}, rzn_p[CPL] = {0, 0, 0, 0};
+      for (long long q = tid; q < nq; q += nth) {
+        const int c0 = CPL * (int)(q % LG4);
+        float r[CPL], qq[CPL];
+        ld4(P.R32 + q * CPL, r);
+        ld4(P.Q32 + q * CPL, qq);
+        const float di = __ldg(P.dinv32 + q / LG4);
 #pragma unroll
-      for (int c = 0; c < CPL; ++c) {
-        const float al = s_alpha[c0 + c];
-        x[c] = fmaf(al, p[c], x[c]);
-        r[c] = fmaf(-al, qq[c], r[c]);
-        rr_p[c] = fmaf(r[c], r[c], rr_p[c]);
-        rzn_p[c] = fmaf(r[c], r[c] * di, rzn_p[c]);
+        for (int c = 0; c < CPL; ++c) {
+          r[c] = fmaf(-s_alpha[c0 + c], qq[c], r[c]);
+          rr_p[c] = fmaf(r[c], r[c], rr_p[c]);
+          rzn_p[c] = fmaf(r[c], r[c] * di, rzn_p[c]);
+        }
+        st4(P.R32 + q * CPL, r);
       }
-      st4(P.X32 + q * CPL, x);
-      st4(P.R32 + q * CPL, r);
+      block_partials_cols<NC, CPL>(rr_p, P.partials, SL_A);
+      __syncthreads();  // the scratch is read
+      block_partials_cols<NC, CPL>(rzn_p, P.partials, SL_B);
     }
-    block_partials_cols<float>(rr_p, P.partials, SL_A);
-    __syncthreads();
-    block_partials_cols<float>(rzn_p, P.partials, SL_B);
-    if (!grid_reduce_sync_wide(P.bar, P.st, P.limit_ns, P.partials, P.totals, 0, 2 * NR)) return;
-    if (threadIdx.x == 0) {
-      int all_dropped = 1, candidate = 0, seen = 0;
-      for (int c = 0; c < NR; ++c) {
-        if (!s_active[c]) continue;
-        seen = 1;
-        const double rn = sqrt(__ldcg(P.totals + SL_A + c));
-        s_rrec[c] = rn;
-        if (!isfinite(rn)) candidate = 1;
-        if (rn > P.delta * s_rmax[c]) all_dropped = 0;
-        if (rn <= P.tol * s_bnorm[c]) candidate = 1;
-      }
-      s_flag = seen && (all_dropped || candidate);
+    if (!grid_reduce_sync_wide(P.bar, P.st, P.limit_ns, P.partials, P.totals, 0, 2 * NC)) return;
+    if (threadIdx.x < 32) {  // one lane per case
+      const int c = threadIdx.x;
+      const bool on = c < NC && s_active[c];
+      const double rn = on ? sqrt(__ldcg(P.totals + SL_A + c)) : 0.0;
+      if (on) s_rrec[c] = rn;
+      const bool dropped = !on || rn <= P.delta * s_rmax[c];
+      const bool candidate = on && (!isfinite(rn) || rn <= P.tol * s_bnorm[c]);
+      const int all_dropped = __all_sync(0xffffffffu, dropped || (on && !isfinite(rn)));
+      const int any_candidate = __any_sync(0xffffffffu, candidate), seen = __any_sync(0xffffffffu, on);
+      if (c == 0) s_flag = seen && (all_dropped || any_candidate);
     }
     __syncthreads();
+    if (s_flag)  // the update needs x complete
+      for (long long q = tid; q < nq; q += nth) {
+        const int c0 = CPL * (int)(q % LG4);
+        float x[CPL], p[CPL];
+        ld4(P.X32 + q * CPL, x);
+        ld4(P.P32 + q * CPL, p);
+#pragma unroll
+        for (int c = 0; c < CPL; ++c) x[c] = fmaf(s_alpha[c0 + c], p[c], x[c]);
+        st4(P.X32 + q * CPL, x);
+      }
     if (s_flag && P.split) {  // the update runs as its own launches; resume from the state
       if (blockIdx.x == 0) {
         if (threadIdx.x < NR) {
@@ -784,11 +905,11 @@ __global__ void __launch_bounds__(PCG_THREADS, 2) pcg_bsr_multi_kernel(MultiArgs
 #pragma unroll
         for (int h = 0; h < 2; ++h) {
           double y[3][2];
-          bsr_row_multi_half(a, lane, P.M64, P.X, h, y);
-          if (lane < LPG) {
+          bsr_row_multi_half<NC>(a, lane, P.M64, P.X, h, y);
+          if (lane < LG4) {
 #pragma unroll
             for (int i = 0; i < 3; ++i) {
-              const size_t off = (size_t)(3 * a + i) * NR + CPL * lane + 2 * h;
+              const size_t off = (size_t)(3 * a + i) * NC + CPL * lane + 2 * h;
               const double2 bv = *reinterpret_cast<const double2*>(P.B + off);
               const float di = P.dinv32[3 * a + i];
               const double rv0 = bv.x - y[i][0], rv1 = bv.y - y[i][1];
@@ -802,22 +923,22 @@ __global__ void __launch_bounds__(PCG_THREADS, 2) pcg_bsr_multi_kernel(MultiArgs
           }
         }
       }
-      block_partials_cols<double>(rr64, P.partials, SL_A);
+      block_partials_cols<NC, CPL>(rr64, P.partials, SL_A);
       __syncthreads();
-      block_partials_cols<float>(rz2, P.partials, SL_B);
-      if (!grid_reduce_sync_wide(P.bar, P.st, P.limit_ns, P.partials, P.totals, 0, 2 * NR)) return;
+      block_partials_cols<NC, CPL>(rz2, P.partials, SL_B);
+      if (!grid_reduce_sync_wide(P.bar, P.st, P.limit_ns, P.partials, P.totals, 0, 2 * NC)) return;
       after_update(updates);
     }
-    if (!iteration_tail()) return;
+    if (!iteration_tail(!s_flag)) return;
   }
   int any_active = 0, broke = 0;
-  for (int c = 0; c < NR; ++c) {
+  for (int c = 0; c < NC; ++c) {
     any_active |= s_active[c];
     broke |= s_res[c] < 0.0;
   }
   if (broke) status = AXIA_ERR_ZERO_PIVOT;
   else if (any_active) status = AXIA_ERR_NOT_CONVERGED;
-  if (blockIdx.x == 0 && threadIdx.x < NR) {
+  if (blockIdx.x == 0 && threadIdx.x < NC) {
     const int c = threadIdx.x;
     P.out->bnorm[c] = s_bnorm[c];
     P.out->residual[c] = s_res[c];
@@ -852,19 +973,23 @@ __global__ void k_batch_fold(long long n, double* X, float* X32, float* Xh, floa
   }
 }
 
-template <bool DW>
-__global__ void __launch_bounds__(256) k_batch_resid(BsrMatM<float> M32, const float* __restrict__ lo32,
+template <bool DW, int NC>
+__global__ void __launch_bounds__(256) k_batch_resid(const int* __restrict__ order, BsrMatM<float> M32, const float* __restrict__ lo32,
                                                     BsrMatM<double> M64, const double* __restrict__ B,
                                                     const double* __restrict__ X, const float* __restrict__ Xh,
                                                     const float* __restrict__ Xl, const float* __restrict__ dinv32,
                                                     float* R32, double* part, unsigned cases) {
-  __shared__ double s_rr[8][NR], s_rz[8][NR];
+  __shared__ double s_rr[8][32], s_rz[8][32];
+  constexpr int RPW = 32 / NC;  // rows per warp
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-  const bool on = (cases >> lane) & 1u;  // the cases (lanes) this pass computes
+  const int c = lane % NC, grp = lane / NC;
+  const bool on = (cases >> c) & 1u;  // the cases this pass computes
   const int n = M32.n_nodes;
   const long long nb = M32.nb;
   double rr = 0.0, rz = 0.0;
-  for (int a = blockIdx.x * 8 + w; on && a < n; a += gridDim.x * 8) {
+  const int per = (n + (int)gridDim.x - 1) / (int)gridDim.x, i1 = min(n, ((int)blockIdx.x + 1) * per);
+  for (int i0 = blockIdx.x * per + w * RPW + grp; on && i0 < i1; i0 += 8 * RPW) {
+    const int a = __ldg(order + i0);
     const int beg = __ldg(M32.adj_ptr + a), end = __ldg(M32.adj_ptr + a + 1);
     double y[3];
     if constexpr (DW) {
@@ -874,7 +999,7 @@ __global__ void __launch_bounds__(256) k_batch_resid(BsrMatM<float> M32, const f
         dw xv[3];
 #pragma unroll
         for (int j = 0; j < 3; ++j) {
-          const size_t o = (size_t)(3 * b + j) * NR + lane;
+          const size_t o = (size_t)(3 * b + j) * NC + c;
           xv[j] = dw{Xh[o], Xl[o]};
         }
 #pragma unroll
@@ -889,14 +1014,14 @@ __global__ void __launch_bounds__(256) k_batch_resid(BsrMatM<float> M32, const f
         const int b = __ldg(M64.adj + s);
         double xv[3];
 #pragma unroll
-        for (int j = 0; j < 3; ++j) xv[j] = X[(size_t)(3 * b + j) * NR + lane];
+        for (int j = 0; j < 3; ++j) xv[j] = X[(size_t)(3 * b + j) * NC + c];
 #pragma unroll
         for (int p = 0; p < 9; ++p) y[p / 3] = fma(__ldg(M64.val + p * nb + s), xv[p % 3], y[p / 3]);
       }
     }
 #pragma unroll
     for (int i = 0; i < 3; ++i) {
-      const size_t o = (size_t)(3 * a + i) * NR + lane;
+      const size_t o = (size_t)(3 * a + i) * NC + c;
       const double r = B[o] - y[i];
       rr = fma(r, r, rr);
       const float r32 = (float)r;
@@ -907,15 +1032,16 @@ __global__ void __launch_bounds__(256) k_batch_resid(BsrMatM<float> M32, const f
   s_rr[w][lane] = rr;
   s_rz[w][lane] = rz;
   __syncthreads();
-  if (w == 0 && on) {  // the other cases keep the partials of an earlier pass
+  if (w == 0 && lane < NC && on) {  // the other cases keep the partials of an earlier pass
     double a = 0.0, b = 0.0;
+    for (int k = 0; k < 8; ++k)
 #pragma unroll
-    for (int k = 0; k < 8; ++k) {
-      a += s_rr[k][lane];
-      b += s_rz[k][lane];
-    }
+      for (int g = 0; g < RPW; ++g) {
+        a += s_rr[k][g * NC + lane];
+        b += s_rz[k][g * NC + lane];
+      }
     part[(size_t)lane * gridDim.x + blockIdx.x] = a;
-    part[(size_t)(NR + lane) * gridDim.x + blockIdx.x] = b;
+    part[(size_t)(NC + lane) * gridDim.x + blockIdx.x] = b;
   }
 }
 
@@ -929,7 +1055,7 @@ struct CaseList {
   int c[NR];
 };
 
-template <int KP>
+template <int KP, int NC>
 __global__ void __launch_bounds__(256) k_batch_resid64_cases(BsrMatM<double> M64, const double* __restrict__ B,
                                                             const double* __restrict__ X,
                                                             const float* __restrict__ dinv32, float* R32,
@@ -952,13 +1078,13 @@ __global__ void __launch_bounds__(256) k_batch_resid64_cases(BsrMatM<double> M64
       const int b = __ldg(M64.adj + s);
       double xv[3];
 #pragma unroll
-      for (int j = 0; j < 3; ++j) xv[j] = X[(size_t)(3 * b + j) * NR + c];
+      for (int j = 0; j < 3; ++j) xv[j] = X[(size_t)(3 * b + j) * NC + c];
 #pragma unroll
       for (int p = 0; p < 9; ++p) y[p / 3] = fma(__ldg(M64.val + p * nb + s), xv[p % 3], y[p / 3]);
     }
 #pragma unroll
     for (int i = 0; i < 3; ++i) {
-      const size_t o = (size_t)(3 * a + i) * NR + c;
+      const size_t o = (size_t)(3 * a + i) * NC + c;
       const double r = B[o] - y[i];
       rr = fma(r, r, rr);
       const float r32 = (float)r;
@@ -983,14 +1109,14 @@ __global__ void __launch_bounds__(256) k_batch_resid64_cases(BsrMatM<double> M64
       b += s_rz[k][lane];
     }
     part[(size_t)list.c[lane] * gridDim.x + blockIdx.x] = a;
-    part[(size_t)(NR + list.c[lane]) * gridDim.x + blockIdx.x] = b;
+    part[(size_t)(NC + list.c[lane]) * gridDim.x + blockIdx.x] = b;
   }
 }
 
 // totals[k] = sum over the g blocks of part[k][.], ascending block order (one warp per slot)
-__global__ void k_batch_resid_sum(const double* part, int g, double* totals) {
+__global__ void k_batch_resid_sum(const double* part, int g, int slots, double* totals) {
   const int lane = threadIdx.x & 31, k = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
-  if (k >= 2 * NR) return;
+  if (k >= slots) return;
   double a = 0.0;
   for (int b = lane; b < g; b += 32) a += part[(size_t)k * g + b];
   a = warp_sum(a);
@@ -998,21 +1124,22 @@ __global__ void k_batch_resid_sum(const double* part, int g, double* totals) {
 }
 
 // B[d][c] = f_c[d] - K_fp u0 (free d), 0 (prescribed d); columns >= nrhs zero
-__global__ void k_batch_rhs(int64_t nd, int nrhs, const int32_t* ind_of, const double* F, const double* kfu0,
+__global__ void k_batch_rhs(int64_t nd, int width, int nrhs, const int32_t* ind_of, const double* F, const double* kfu0,
                             double* B) {
-  for (int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; t < nd * NR; t += (int64_t)gridDim.x * blockDim.x) {
-    const int64_t d = t / NR;
-    const int c = (int)(t % NR);
+  for (int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; t < nd * width; t += (int64_t)gridDim.x * blockDim.x) {
+    const int64_t d = t / width;
+    const int c = (int)(t % width);
     const int r = ind_of[d];
     B[t] = (c < nrhs && r >= 0) ? F[(int64_t)c * nd + d] - kfu0[r] : 0.0;
   }
 }
 // U_c[d] = u0[d] + X[d][c] on free DOFs
-__global__ void k_batch_out(int64_t nd, int nrhs, const int32_t* ind_of, const double* u0, const double* X, double* U) {
+__global__ void k_batch_out(int64_t nd, int width, int nrhs, const int32_t* ind_of, const double* u0, const double* X,
+                            double* U) {
   for (int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; t < nd * nrhs; t += (int64_t)gridDim.x * blockDim.x) {
     const int c = (int)(t / nd);
     const int64_t d = t % nd;
-    U[t] = ind_of[d] >= 0 ? u0[d] + X[d * NR + c] : u0[d];
+    U[t] = ind_of[d] >= 0 ? u0[d] + X[d * width + c] : u0[d];
   }
 }
 
@@ -1045,7 +1172,7 @@ __global__ void __launch_bounds__(BT) k_blk_spmm(BsrMatM<float> M, const float* 
   for (int a = gwarp; a < M.n_nodes; a += nwarps) {
     const int len = __ldg(M.adj_ptr + a + 1) - __ldg(M.adj_ptr + a);
     float y[3][2];
-    row_tile<2, 4, false>(a, len, lane, nullptr, M, P, y);
+    row_tile<NR, 2, 4, false>(a, len, lane, nullptr, M, P, y);
     if (lane < 16) {
 #pragma unroll
       for (int i = 0; i < 3; ++i) stc<2>(Q + (size_t)(3 * a + i) * NR + 2 * lane, y[i]);
@@ -1179,7 +1306,7 @@ __global__ void __launch_bounds__(BT) k_blk_precond(int64_t nd, const float* din
     const int64_t row = q / LPG;
     float r[CPL], zc[CPL] = {0.f, 0.f, 0.f, 0.f};
     ld4(R + q * CPL, r);
-    if constexpr (COARSE) coarse_prolong_m(C, row, CPL * (int)(q % LPG), zc);
+    if constexpr (COARSE) coarse_prolong_m<NR>(C, row, CPL * (int)(q % LPG), zc);
     const float di = dinv[row];
 #pragma unroll
     for (int c = 0; c < CPL; ++c) zc[c] = fmaf(r[c], di, zc[c]);
@@ -1187,15 +1314,16 @@ __global__ void __launch_bounds__(BT) k_blk_precond(int64_t nd, const float* din
   }
 }
 
-__global__ void __launch_bounds__(BT) k_blk_restrict(CoarseArgs C, const float* R) {
+__global__ void __launch_bounds__(BT) k_blk_restrict(CoarseArgs C, float* R) {
   const int lane = threadIdx.x & 31;
   const int gwarp = (blockIdx.x * BT + threadIdx.x) >> 5, nwarps = (gridDim.x * BT) >> 5;
-  coarse_restrict_m(C, R, gwarp, nwarps, lane);
+  float none[2];
+  coarse_restrict_m<NR, false>(C, nullptr, R, nullptr, nullptr, gwarp, nwarps, lane, none, none);
 }
 
 __global__ void __launch_bounds__(PCG_THREADS) k_blk_coarse_solve(CoarseArgs C, double* scratch) {
   extern __shared__ __align__(16) float s_ring[];  // COARSE_RING_FLOATS
-  coarse_solve_m(C, s_ring, scratch, 0);
+  coarse_solve_m<NR>(C, s_ring, scratch, 0);
 }
 
 // X += X32 (FP64), X32 = 0
@@ -1355,18 +1483,29 @@ struct BatchTile {
 };
 // ((4, 2) is left out: it spills about 100 bytes of registers with the coarse space.)
 constexpr BatchTile kBatchTiles[] = {{4, 1}, {2, 2}, {2, 4}, {1, 4}, {1, 8}};
-constexpr BatchTile kBatchDefault = {2, 4};
+constexpr BatchTile kBatchDefault = {4, 1};
 
 template <bool COARSE>
 const void* batch_kernel(BatchTile t) {
   switch (t.tc * 100 + t.tu) {
-    case 401: return (const void*)pcg_bsr_multi_kernel<COARSE, 4, 1>;
-    case 202: return (const void*)pcg_bsr_multi_kernel<COARSE, 2, 2>;
-    case 204: return (const void*)pcg_bsr_multi_kernel<COARSE, 2, 4>;
-    case 104: return (const void*)pcg_bsr_multi_kernel<COARSE, 1, 4>;
-    case 108: return (const void*)pcg_bsr_multi_kernel<COARSE, 1, 8>;
+    case 401: return (const void*)pcg_bsr_multi_kernel<COARSE, NR, 4, 1>;
+    case 202: return (const void*)pcg_bsr_multi_kernel<COARSE, NR, 2, 2>;
+    case 204: return (const void*)pcg_bsr_multi_kernel<COARSE, NR, 2, 4>;
+    case 104: return (const void*)pcg_bsr_multi_kernel<COARSE, NR, 1, 4>;
+    case 108: return (const void*)pcg_bsr_multi_kernel<COARSE, NR, 1, 8>;
     default: return nullptr;
   }
+}
+
+// Columns of a launch that solves nc load cases: 8, 16 or 32, so a few cases
+// (or the remainder of a list) do not pay for 32 columns of every vector and
+// of the products.
+int batch_width(int nc) { return nc <= 8 ? 8 : nc <= 16 ? 16 : NR; }
+
+template <bool COARSE>
+const void* narrow_kernel(int width) {
+  return width == 8 ? (const void*)pcg_bsr_multi_kernel<COARSE, 8, 2, 2>
+                    : (const void*)pcg_bsr_multi_kernel<COARSE, 16, 4, 1>;
 }
 
 bool valid_tile(int tc, int tu) {
@@ -1375,7 +1514,110 @@ bool valid_tile(int tc, int tu) {
   return false;
 }
 
+// ---------------------------------------------------------------------------
+// The order in which the 32-case SpMV takes the block rows: the nodes along a
+// Morton curve through the mesh's bounding box, so that the rows a block works
+// on at one time are neighbours in space.  A row gathers 27 vector rows of 384
+// bytes (C3D8); 64 neighbouring rows share about 220 of their 1,728, which the
+// L1 then serves, where 64 consecutive rows of a grid numbered line by line
+// share 600.
+// ---------------------------------------------------------------------------
+__device__ __forceinline__ unsigned long long ordered_bits(double x) {
+  const unsigned long long u = (unsigned long long)__double_as_longlong(x);
+  return u >> 63 ? ~u : u | (1ull << 63);
+}
+__device__ __forceinline__ double from_ordered_bits(unsigned long long u) {
+  return __longlong_as_double((long long)(u >> 63 ? u & ~(1ull << 63) : ~u));
+}
+// box[0..2] minima (start ~0), box[3..5] maxima (start 0), as ordered bits
+__global__ void k_order_box(int n, const double* __restrict__ xyz, unsigned long long* box) {
+  unsigned long long lo[3] = {~0ull, ~0ull, ~0ull}, hi[3] = {0, 0, 0};
+  for (int a = blockIdx.x * blockDim.x + threadIdx.x; a < n; a += gridDim.x * blockDim.x)
+#pragma unroll
+    for (int d = 0; d < 3; ++d) {
+      const unsigned long long u = ordered_bits(xyz[3LL * a + d]);
+      lo[d] = min(lo[d], u);
+      hi[d] = max(hi[d], u);
+    }
+#pragma unroll
+  for (int d = 0; d < 3; ++d) {
+    for (int o = 16; o > 0; o >>= 1) {
+      lo[d] = min(lo[d], __shfl_xor_sync(0xffffffffu, lo[d], o));
+      hi[d] = max(hi[d], __shfl_xor_sync(0xffffffffu, hi[d], o));
+    }
+    if ((threadIdx.x & 31) == 0) {
+      atomicMin(box + d, lo[d]);
+      atomicMax(box + 3 + d, hi[d]);
+    }
+  }
+}
+__device__ __forceinline__ unsigned spread3(unsigned v) {  // bit k of v (10 bits) to bit 3 k
+  v = (v | v << 16) & 0x030000ffu;
+  v = (v | v << 8) & 0x0300f00fu;
+  v = (v | v << 4) & 0x030c30c3u;
+  return (v | v << 2) & 0x09249249u;
+}
+__global__ void k_order_keys(int n, const double* __restrict__ xyz, const unsigned long long* box, unsigned* key,
+                             int* iota) {
+  double ext = 0.0, lo[3];
+#pragma unroll
+  for (int d = 0; d < 3; ++d) {
+    lo[d] = from_ordered_bits(box[d]);
+    ext = fmax(ext, from_ordered_bits(box[3 + d]) - lo[d]);
+  }
+  const float scale = ext > 0.0 ? (float)(1023.0 / ext) : 0.f;
+  for (int a = blockIdx.x * blockDim.x + threadIdx.x; a < n; a += gridDim.x * blockDim.x) {
+    unsigned k = 0;
+#pragma unroll
+    for (int d = 0; d < 3; ++d) {
+      const float t = (float)(xyz[3LL * a + d] - lo[d]) * scale;
+      k |= spread3(t > 0.f ? min((unsigned)t, 1023u) : 0u) << d;
+    }
+    key[a] = k;
+    iota[a] = a;
+  }
+}
+
+int ensure_row_order(axia_ctx* ctx) {
+  if (ctx->d_row_order) return AXIA_OK;
+  const int n = (int)ctx->n_nodes;
+  int *iota = nullptr, *order = nullptr;
+  unsigned *key = nullptr, *key_out = nullptr;
+  unsigned long long* box = nullptr;
+  unsigned char* temp = nullptr;
+  int st = AXIA_OK;
+  do {
+    if ((st = dev_alloc(ctx, &iota, (size_t)n))) break;
+    if ((st = dev_alloc(ctx, &order, (size_t)n))) break;
+    if ((st = dev_alloc(ctx, &key, (size_t)n))) break;
+    if ((st = dev_alloc(ctx, &key_out, (size_t)n))) break;
+    if ((st = dev_alloc(ctx, &box, (size_t)6))) break;
+    AXIA_CUDA(ctx, cudaMemsetAsync(box, 0xff, 3 * sizeof(*box), ctx->stream));
+    AXIA_CUDA(ctx, cudaMemsetAsync(box + 3, 0, 3 * sizeof(*box), ctx->stream));
+    const int grid = std::max(1, std::min((n + 255) / 256, ctx->sm_count * 4));
+    k_order_box<<<grid, 256, 0, ctx->stream>>>(n, ctx->d_coords, box);
+    k_order_keys<<<grid, 256, 0, ctx->stream>>>(n, ctx->d_coords, box, key, iota);
+    ctx->launches += 2;
+    size_t tb = 0;
+    cub::DeviceRadixSort::SortPairs(nullptr, tb, key, key_out, iota, order, n, 0, 30, ctx->stream);
+    if ((st = dev_alloc(ctx, &temp, std::max<size_t>(tb, 16)))) break;
+    AXIA_CUDA(ctx, cub::DeviceRadixSort::SortPairs(temp, tb, key, key_out, iota, order, n, 0, 30, ctx->stream));
+    AXIA_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
+  } while (false);
+  dev_release(ctx, iota);
+  dev_release(ctx, key);
+  dev_release(ctx, key_out);
+  dev_release(ctx, box);
+  dev_release(ctx, temp);
+  if (st)
+    dev_release(ctx, order);
+  else
+    ctx->d_row_order = order;
+  return st;
+}
+
 int ensure_batch_buffers(axia_ctx* ctx) {
+  AXIA_TRY(ensure_row_order(ctx));
   const size_t blk = (size_t)ctx->ndof * NR;
   if (ctx->batch_capacity < blk) {
     AXIA_TRY(dev_alloc(ctx, &ctx->d_mB, blk));
@@ -1398,13 +1640,15 @@ int ensure_batch_buffers(axia_ctx* ctx) {
 int batch_grid(axia_ctx* ctx, const void* kern, int* grid) {
   // static + staging shared memory is above the 48 KB a block gets without opting in
   AXIA_CUDA(ctx, cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)DYN_BYTES));
-  AXIA_TRY(coop_grid(ctx, kern, (int)std::min<int64_t>(ctx->ndof, INT32_MAX), grid, DYN_BYTES));
+  // a thread per float4 chunk of a vector, a warp per block row: more blocks
+  // than the single system's DOF count asks for
+  AXIA_TRY(coop_grid(ctx, kern, (int)std::min<int64_t>(ctx->ndof * 8, INT32_MAX), grid, DYN_BYTES));
   if ((size_t)*grid * 2 * NR > ctx->partial_slots) *grid = (int)(ctx->partial_slots / (2 * NR));
   return AXIA_OK;
 }
 
 MultiArgs multi_args(axia_ctx* ctx, double rtol, double delta, long long max_iter, const CoarseArgs& cargs) {
-  return MultiArgs{BsrMatM<float>{(int)ctx->n_nodes, ctx->d_qptr, ctx->d_qadj, ctx->d_bval32, (long long)ctx->nbq},
+  return MultiArgs{ctx->d_row_order, BsrMatM<float>{(int)ctx->n_nodes, ctx->d_qptr, ctx->d_qadj, ctx->d_bval32, (long long)ctx->nbq},
                    BsrMatM<double>{(int)ctx->n_nodes, ctx->d_qptr, ctx->d_qadj, ctx->d_bval64, (long long)ctx->nbq},
                    (int)ctx->ndof, ctx->d_bdinv32, ctx->d_mB, ctx->d_mX, ctx->d_mX32, ctx->d_mR32, ctx->d_mP32,
                    ctx->d_mQ32, ctx->d_partials, ctx->d_totals, ctx->d_bar, ctx->d_status, (MultiOut*)ctx->d_mout,
@@ -1595,7 +1839,7 @@ struct BlockRun {
     count(1);
   }
   // Z = M R (diagonal, plus the coarse part)
-  void precond(const float* R, float* Z) {
+  void precond(float* R, float* Z) {
     if (coarse) {
       k_blk_restrict<<<g_row, BT, 0, s>>>(C, R);
       k_blk_coarse_solve<<<ctx->sm_count * 2, PCG_THREADS, COARSE_RING_FLOATS * sizeof(float), s>>>(C, part());
@@ -1658,7 +1902,7 @@ int batch_block_solve(axia_ctx* ctx, int nrhs, const double* d_F, double* d_U, c
   const int64_t n = B.nd * NR;
   for (int c0 = 0; c0 < nrhs && st == AXIA_OK; c0 += NR) {
     const int nc = std::min(NR, nrhs - c0);
-    k_batch_rhs<<<ctx->sm_count * 8, 256, 0, B.s>>>(B.nd, nc, ctx->d_ind_of, d_F + (int64_t)c0 * B.nd, ctx->d_kfu0,
+    k_batch_rhs<<<ctx->sm_count * 8, 256, 0, B.s>>>(B.nd, NR, nc, ctx->d_ind_of, d_F + (int64_t)c0 * B.nd, ctx->d_kfu0,
                                                    ctx->d_mB);
     cudaEventRecord(ev0, B.s);
     k_blk_init<<<B.g_row, BT, 0, B.s>>>(n, ctx->d_mB, ctx->d_mX, ctx->d_mX32, ctx->d_mR32, B.part());
@@ -1745,7 +1989,7 @@ int batch_block_solve(axia_ctx* ctx, int nrhs, const double* d_F, double* d_U, c
       st = set_error(ctx, AXIA_ERR_NOT_CONVERGED, "block CG did not converge in " + std::to_string(iters) + " iterations");
       break;
     }
-    k_batch_out<<<ctx->sm_count * 8, 256, 0, B.s>>>(B.nd, nc, ctx->d_ind_of, ctx->d_u0, ctx->d_mX,
+    k_batch_out<<<ctx->sm_count * 8, 256, 0, B.s>>>(B.nd, NR, nc, ctx->d_ind_of, ctx->d_u0, ctx->d_mX,
                                                    d_U + (int64_t)c0 * B.nd);
     ctx->launches++;
     if (cudaGetLastError() != cudaSuccess) st = set_error(ctx, AXIA_ERR_CUDA, "block CG launch");
@@ -1781,11 +2025,12 @@ int ensure_segment_buffers(axia_ctx* ctx) {
 // the double-word error floor (about 2^-47 sum |K| |X|) is reached and the
 // updates are FP64 from then on.  Then the kernel resumes (phase 0 when it
 // finishes).
+template <int NC>
 int run_segmented(axia_ctx* ctx, const void* kern, int grid, MultiArgs& P) {
   const int64_t nd = ctx->ndof;
-  const long long n = (long long)nd * NR;
+  const long long n = (long long)nd * NC;
   const int g_res = (int)std::min<int64_t>((ctx->n_nodes + 7) / 8, (int64_t)ctx->sm_count * 8);
-  if ((size_t)g_res * 2 * NR > ctx->partial_slots) return set_error(ctx, AXIA_ERR_TOO_LARGE, "partials area too small");
+  if ((size_t)g_res * 2 * NC > ctx->partial_slots) return set_error(ctx, AXIA_ERR_TOO_LARGE, "partials area too small");
   const BsrMatM<float> M32{(int)ctx->n_nodes, ctx->d_qptr, ctx->d_qadj, ctx->d_bval32, (long long)ctx->nbq};
   const BsrMatM<double> M64{(int)ctx->n_nodes, ctx->d_qptr, ctx->d_qadj, ctx->d_bval64, (long long)ctx->nbq};
   BatchState hs;
@@ -1801,14 +2046,14 @@ int run_segmented(axia_ctx* ctx, const void* kern, int grid, MultiArgs& P) {
     if (hs.phase != 1) return AXIA_OK;  // finished, or stopped early (status / barrier limit)
     auto residual = [&](bool dwr, unsigned cases) -> int {
       if (dwr)
-        k_batch_resid<true><<<g_res, 256, 0, ctx->stream>>>(M32, ctx->d_bval32lo, M64, ctx->d_mB, ctx->d_mX,
+        k_batch_resid<true, NC><<<g_res, 256, 0, ctx->stream>>>(P.order, M32, ctx->d_bval32lo, M64, ctx->d_mB, ctx->d_mX,
                                                              ctx->d_mXh, ctx->d_mXl, ctx->d_bdinv32, ctx->d_mR32,
                                                              ctx->d_partials, cases);
       else
-        k_batch_resid<false><<<g_res, 256, 0, ctx->stream>>>(M32, ctx->d_bval32lo, M64, ctx->d_mB, ctx->d_mX,
+        k_batch_resid<false, NC><<<g_res, 256, 0, ctx->stream>>>(P.order, M32, ctx->d_bval32lo, M64, ctx->d_mB, ctx->d_mX,
                                                               ctx->d_mXh, ctx->d_mXl, ctx->d_bdinv32, ctx->d_mR32,
                                                               ctx->d_partials, cases);
-      k_batch_resid_sum<<<2, NR * 32, 0, ctx->stream>>>(ctx->d_partials, g_res, ctx->d_totals);
+      k_batch_resid_sum<<<2, NC * 32, 0, ctx->stream>>>(ctx->d_partials, g_res, 2 * NC, ctx->d_totals);
       ctx->launches += 2;
       AXIA_CUDA(ctx, cudaGetLastError());
       return AXIA_OK;
@@ -1818,20 +2063,20 @@ int run_segmented(axia_ctx* ctx, const void* kern, int grid, MultiArgs& P) {
     ctx->launches++;
     AXIA_TRY(residual(!fp64_only, ~0u));
     if (!fp64_only) {
-      double tot[NR];
+      double tot[NC];
       AXIA_CUDA(ctx, cudaMemcpyAsync(tot, ctx->d_totals, sizeof(tot), cudaMemcpyDeviceToHost, ctx->stream));
       AXIA_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
       // the cases whose double-word residual meets tol or stalled: FP64 for them
       unsigned check = 0;
-      for (int c = 0; c < NR; ++c) {
+      for (int c = 0; c < NC; ++c) {
         if (!hs.active[c]) continue;
         const double rn = std::sqrt(tot[c]);
         if (rn <= P.tol * hs.bnorm[c] || !(rn <= 0.5 * hs.rmax[c])) check |= 1u << c;
       }
       if (check) {
-        double t64[NR];
+        double t64[NC];
         CaseList list{};
-        for (int c = 0; c < NR; ++c)
+        for (int c = 0; c < NC; ++c)
           if ((check >> c) & 1u) list.c[list.n++] = c;
         int kp = 1;
         while (kp < list.n) kp <<= 1;
@@ -1840,20 +2085,20 @@ int run_segmented(axia_ctx* ctx, const void* kern, int grid, MultiArgs& P) {
                                                ctx->d_partials, list);
         };
         switch (kp) {
-          case 1: sub(k_batch_resid64_cases<1>); break;
-          case 2: sub(k_batch_resid64_cases<2>); break;
-          case 4: sub(k_batch_resid64_cases<4>); break;
-          case 8: sub(k_batch_resid64_cases<8>); break;
-          case 16: sub(k_batch_resid64_cases<16>); break;
-          default: sub(k_batch_resid64_cases<32>); break;
+          case 1: sub(k_batch_resid64_cases<1, NC>); break;
+          case 2: sub(k_batch_resid64_cases<2, NC>); break;
+          case 4: sub(k_batch_resid64_cases<4, NC>); break;
+          case 8: sub(k_batch_resid64_cases<8, NC>); break;
+          case 16: sub(k_batch_resid64_cases<16, NC>); break;
+          default: sub(k_batch_resid64_cases<32, NC>); break;
         }
-        k_batch_resid_sum<<<2, NR * 32, 0, ctx->stream>>>(ctx->d_partials, g_res, ctx->d_totals);
+        k_batch_resid_sum<<<2, NC * 32, 0, ctx->stream>>>(ctx->d_partials, g_res, 2 * NC, ctx->d_totals);
         ctx->launches += 2;
         AXIA_CUDA(ctx, cudaGetLastError());
         AXIA_CUDA(ctx, cudaMemcpyAsync(t64, ctx->d_totals, sizeof(t64), cudaMemcpyDeviceToHost, ctx->stream));
         AXIA_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
         // double-word and FP64 residuals apart by more than 10 %: the floor is reached
-        for (int c = 0; c < NR; ++c) {
+        for (int c = 0; c < NC; ++c) {
           if (!((check >> c) & 1u)) continue;
           const double a = std::sqrt(tot[c]), b = std::sqrt(t64[c]);
           if (!(std::fabs(a - b) <= 0.1 * b)) fp64_only = true;
@@ -1880,9 +2125,6 @@ int batch_solve(axia_ctx* ctx, int nrhs, const double* d_F, double* d_U, const a
   const double delta = opts->inner_rtol > 0 && opts->inner_rtol < 1 ? opts->inner_rtol : 0.01;
   const BatchTile tile = valid_tile(ctx->tuned_btc, ctx->tuned_btu) ? BatchTile{ctx->tuned_btc, ctx->tuned_btu}
                                                                      : kBatchDefault;
-  const void* kern = coarse ? batch_kernel<true>(tile) : batch_kernel<false>(tile);
-  int grid = 0;
-  AXIA_TRY(batch_grid(ctx, kern, &grid));
   // with the FP32 low parts assembled the reliable updates run in double words
   // between segments of the kernel
   const bool split = ctx->have_bsr32lo;
@@ -1891,9 +2133,13 @@ int batch_solve(axia_ctx* ctx, int nrhs, const double* d_F, double* d_U, const a
   info->outer_iters = 0;
   double worst = 0.0;
   for (int c0 = 0; c0 < nrhs; c0 += NR) {
-    const int nc = std::min(NR, nrhs - c0);
+    const int nc = std::min(NR, nrhs - c0), width = batch_width(nc);
+    const void* kern = width < NR ? (coarse ? narrow_kernel<true>(width) : narrow_kernel<false>(width))
+                                  : (coarse ? batch_kernel<true>(tile) : batch_kernel<false>(tile));
+    int grid = 0;
+    AXIA_TRY(batch_grid(ctx, kern, &grid));
     AXIA_TRY(reset_dev_status(ctx));
-    k_batch_rhs<<<ctx->sm_count * 8, 256, 0, ctx->stream>>>(nd, nc, ctx->d_ind_of, d_F + (int64_t)c0 * nd, ctx->d_kfu0,
+    k_batch_rhs<<<ctx->sm_count * 8, 256, 0, ctx->stream>>>(nd, width, nc, ctx->d_ind_of, d_F + (int64_t)c0 * nd, ctx->d_kfu0,
                                                            ctx->d_mB);
     ctx->launches++;
     AXIA_CUDA(ctx, cudaMemsetAsync(ctx->d_bar, 0, sizeof(GridBarrier), ctx->stream));
@@ -1901,7 +2147,10 @@ int batch_solve(axia_ctx* ctx, int nrhs, const double* d_F, double* d_U, const a
     if (split) {
       P.state = static_cast<BatchState*>(ctx->d_mstate);
       P.split = 1;
-      AXIA_TRY(timed_launch(ctx, info, [&]() -> int { return run_segmented(ctx, kern, grid, P); }));
+      AXIA_TRY(timed_launch(ctx, info, [&]() -> int {
+        return width == 8 ? run_segmented<8>(ctx, kern, grid, P)
+                          : width == 16 ? run_segmented<16>(ctx, kern, grid, P) : run_segmented<NR>(ctx, kern, grid, P);
+      }));
     } else {
       AXIA_TRY(timed_launch(ctx, info, [&]() -> int { return launch_batch(ctx, kern, grid, P); }));
     }
@@ -1922,7 +2171,7 @@ int batch_solve(axia_ctx* ctx, int nrhs, const double* d_F, double* d_U, const a
       if (o.status == AXIA_ERR_ZERO_PIVOT) return set_error(ctx, o.status, "batched CG: zero pivot in a load case");
       return set_error(ctx, o.status, "batched CG did not converge in " + std::to_string(o.iters) + " iterations");
     }
-    k_batch_out<<<ctx->sm_count * 8, 256, 0, ctx->stream>>>(nd, nc, ctx->d_ind_of, ctx->d_u0, ctx->d_mX,
+    k_batch_out<<<ctx->sm_count * 8, 256, 0, ctx->stream>>>(nd, width, nc, ctx->d_ind_of, ctx->d_u0, ctx->d_mX,
                                                            d_U + (int64_t)c0 * nd);
     ctx->launches++;
     AXIA_CUDA(ctx, cudaGetLastError());

@@ -391,6 +391,7 @@ struct axia_ctx {
   double *d_mB = nullptr, *d_mX = nullptr;
   float *d_mX32 = nullptr, *d_mR32 = nullptr, *d_mP32 = nullptr, *d_mQ32 = nullptr;
   void* d_mout = nullptr;
+  int* d_row_order = nullptr;   // [n_nodes] block rows in the SpMV's order (batch.cu)
   // segmented batched solve (double-word reliable updates): X as FP32 pairs and the kernel's state
   float *d_mXh = nullptr, *d_mXl = nullptr;
   size_t seg_capacity = 0;
