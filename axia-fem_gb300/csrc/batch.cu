@@ -75,16 +75,27 @@ __device__ __forceinline__ void cp_async_wait() {
   asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory");
 }
 
-// Starts the copy of row a into st (nothing for a >= n_nodes or a long row)
-// and closes the lane's copy group.
-__device__ __forceinline__ void stage_row(int a, int lane, const BsrMatM<float>& M, RowStage* st) {
+// A block row on its way through a warp's loop: node (n_nodes: none), first
+// block, blocks.
+struct RowRef {
+  int a, beg, len;
+};
+__device__ __forceinline__ RowRef row_ref(int a, const BsrMatM<float>& M) {
+  RowRef r{a, 0, 0};
   if (a < M.n_nodes) {
-    const int beg = __ldg(M.adj_ptr + a), len = __ldg(M.adj_ptr + a + 1) - beg;
-    if (len <= STAGE_B && lane < len) {
+    r.beg = __ldg(M.adj_ptr + a);
+    r.len = __ldg(M.adj_ptr + a + 1) - r.beg;
+  }
+  return r;
+}
+
+// Starts the copy of a row into st (nothing for none or a long row) and closes
+// the lane's copy group.
+__device__ __forceinline__ void stage_row(const RowRef& r, int lane, const BsrMatM<float>& M, RowStage* st) {
+  if (r.len <= STAGE_B && lane < r.len) {
 #pragma unroll
-      for (int k = 0; k < 9; ++k) cp_async4(&st->v[k][lane], M.val + (long long)k * M.nb + beg + lane);
-      cp_async4(&st->adj[lane], M.adj + beg + lane);
-    }
+    for (int k = 0; k < 9; ++k) cp_async4(&st->v[k][lane], M.val + (long long)k * M.nb + r.beg + lane);
+    cp_async4(&st->adj[lane], M.adj + r.beg + lane);
   }
   cp_async_commit();
 }
@@ -767,20 +778,25 @@ __global__ void __launch_bounds__(PCG_THREADS, 2) pcg_bsr_multi_kernel(MultiArgs
       return ((((j >> lt) * (int)gridDim.x + (int)blockIdx.x) << lt) + (j & ((1 << lt) - 1))) * nw +
              (int)(threadIdx.x >> 5);
     };
-    int a = row_index(0) < n_nodes ? __ldg(P.order + row_index(0)) : n_nodes;
-    stage_row(a, lane, P.M32, stg);
+    // pipelined: row j is computed while row j + 1 is copied, the bounds of row
+    // j + 2 and the node of row j + 3 are loaded
+    auto node_at = [&](int j) { return row_index(j) < n_nodes ? __ldg(P.order + row_index(j)) : n_nodes; };
+    RowRef cur = row_ref(node_at(0), P.M32), nxt = row_ref(node_at(1), P.M32);
+    int a2 = node_at(2);
+    stage_row(cur, lane, P.M32, stg);
     int kb = 0;
-    for (int j = 0; row_index(j) < n_nodes; ++j, kb ^= 1) {
-      const int next = row_index(j + 1) < n_nodes ? __ldg(P.order + row_index(j + 1)) : n_nodes;
-      stage_row(next, lane, P.M32, stg + (kb ^ 1));
+    for (int j = 0; cur.a < n_nodes; ++j, kb ^= 1) {
+      stage_row(nxt, lane, P.M32, stg + (kb ^ 1));
+      const RowRef after = row_ref(a2, P.M32);
+      a2 = node_at(j + 3);
       cp_async_wait<1>();  // this row's copies (all but the group just opened)
       __syncwarp();
       float y[3][TC];
-      const int len = __ldg(P.M32.adj_ptr + a + 1) - __ldg(P.M32.adj_ptr + a);
-      if (len <= STAGE_B)
-        row_tile<NC, TC, TU, true>(a, len, lane, stg + kb, P.M32, P.P32, y);
+      const int a = cur.a;
+      if (cur.len <= STAGE_B)
+        row_tile<NC, TC, TU, true>(a, cur.len, lane, stg + kb, P.M32, P.P32, y);
       else
-        row_tile<NC, TC, TU, false>(a, len, lane, stg + kb, P.M32, P.P32, y);
+        row_tile<NC, TC, TU, false>(a, cur.len, lane, stg + kb, P.M32, P.P32, y);
       __syncwarp();  // every lane is done with stg[kb] before it is refilled
       if (lane < NC / TC) {
 #pragma unroll
@@ -793,7 +809,8 @@ __global__ void __launch_bounds__(PCG_THREADS, 2) pcg_bsr_multi_kernel(MultiArgs
           for (int c = 0; c < TC; ++c) pq_p[c] = fmaf(p[c], y[d][c], pq_p[c]);
         }
       }
-      a = next;
+      cur = nxt;
+      nxt = after;
     }
     cp_async_wait<0>();  // the last (empty or unused) group
     // lanes 0 .. NC/TC - 1 hold the columns TC lane .. TC lane + TC - 1 of their warp
