@@ -1010,18 +1010,30 @@ __global__ void __launch_bounds__(256) k_batch_resid(const int* __restrict__ ord
     const int beg = __ldg(M32.adj_ptr + a), end = __ldg(M32.adj_ptr + a + 1);
     double y[3];
     if constexpr (DW) {
+      // four blocks at a time (rows are padded to four): a plane's values of the
+      // four are one 16-byte load; scalar loads of 18 planes per block took
+      // 3.97 ms at 80^3 with 32 cases
       dw_acc acc[3];
-      for (int s = beg; s < end; ++s) {
-        const int b = __ldg(M32.adj + s);
-        dw xv[3];
+      for (int s = beg; s < end; s += 4) {
+        const int4 b4 = __ldg(reinterpret_cast<const int4*>(M32.adj + s));
+        const int b[4] = {b4.x, b4.y, b4.z, b4.w};
+        dw xv[4][3];
 #pragma unroll
-        for (int j = 0; j < 3; ++j) {
-          const size_t o = (size_t)(3 * b + j) * NC + c;
-          xv[j] = dw{Xh[o], Xl[o]};
+        for (int t = 0; t < 4; ++t)
+#pragma unroll
+          for (int j = 0; j < 3; ++j) {
+            const size_t o = (size_t)(3 * b[t] + j) * NC + c;
+            xv[t][j] = dw{__ldg(Xh + o), __ldg(Xl + o)};
+          }
+#pragma unroll
+        for (int p = 0; p < 9; ++p) {
+          const float4 h = __ldg(reinterpret_cast<const float4*>(M32.val + p * nb + s));
+          const float4 l = __ldg(reinterpret_cast<const float4*>(lo32 + p * nb + s));
+          dw_fma(acc[p / 3], dw{h.x, l.x}, xv[0][p % 3]);
+          dw_fma(acc[p / 3], dw{h.y, l.y}, xv[1][p % 3]);
+          dw_fma(acc[p / 3], dw{h.z, l.z}, xv[2][p % 3]);
+          dw_fma(acc[p / 3], dw{h.w, l.w}, xv[3][p % 3]);
         }
-#pragma unroll
-        for (int p = 0; p < 9; ++p)
-          dw_fma(acc[p / 3], dw{__ldg(M32.val + p * nb + s), __ldg(lo32 + p * nb + s)}, xv[p % 3]);
       }
 #pragma unroll
       for (int i = 0; i < 3; ++i) y[i] = dw_to_double(dw_value(acc[i]));
@@ -2036,12 +2048,13 @@ int ensure_segment_buffers(axia_ctx* ctx) {
 }
 
 // The batched kernel in segments: it stops at each reliable update (phase 1);
-// X is folded and R = B - K X computed in double words, then in FP64 for the
-// cases whose double-word residual meets its tolerance (the FP64 one decides
-// convergence) or has not dropped below half of its previous update's.  If the two residuals of a case then differ by more than 10 %,
-// the double-word error floor (about 2^-47 sum |K| |X|) is reached and the
-// updates are FP64 from then on.  Then the kernel resumes (phase 0 when it
-// finishes).
+// X is folded and R = B - K X computed: in FP64 for the cases whose recurrence
+// residual meets its tolerance, in double words for the others, and then in
+// FP64 for those whose double-word residual meets the tolerance (the FP64 one
+// decides convergence) or has not dropped below half of its previous update's.
+// If the two residuals of a case differ by more than 10 %, the double-word
+// error floor (about 2^-47 sum |K| |X|) is reached and the updates are FP64
+// from then on.  Then the kernel resumes (phase 0 when it finishes).
 template <int NC>
 int run_segmented(axia_ctx* ctx, const void* kern, int grid, MultiArgs& P) {
   const int64_t nd = ctx->ndof;
@@ -2078,17 +2091,28 @@ int run_segmented(axia_ctx* ctx, const void* kern, int grid, MultiArgs& P) {
     k_batch_fold<<<ctx->sm_count * 8, 256, 0, ctx->stream>>>(n, ctx->d_mX, ctx->d_mX32, ctx->d_mXh, ctx->d_mXl,
                                                             fp64_only ? 0 : 1);
     ctx->launches++;
-    AXIA_TRY(residual(!fp64_only, ~0u));
+    // the cases whose recurrence residual meets tol go to FP64 at once, without
+    // a double-word pass
+    unsigned direct = 0, active = 0;
+    for (int c = 0; c < NC; ++c) {
+      if (!hs.active[c]) continue;
+      active |= 1u << c;
+      if (hs.rrec[c] <= P.tol * hs.bnorm[c]) direct |= 1u << c;
+    }
+    const bool dw_pass = !fp64_only && (active & ~direct) != 0;
+    if (fp64_only || dw_pass) AXIA_TRY(residual(!fp64_only, fp64_only ? ~0u : ~direct));
     if (!fp64_only) {
       double tot[NC];
-      AXIA_CUDA(ctx, cudaMemcpyAsync(tot, ctx->d_totals, sizeof(tot), cudaMemcpyDeviceToHost, ctx->stream));
-      AXIA_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
       // the cases whose double-word residual meets tol or stalled: FP64 for them
-      unsigned check = 0;
-      for (int c = 0; c < NC; ++c) {
-        if (!hs.active[c]) continue;
-        const double rn = std::sqrt(tot[c]);
-        if (rn <= P.tol * hs.bnorm[c] || !(rn <= 0.5 * hs.rmax[c])) check |= 1u << c;
+      unsigned check = direct;
+      if (dw_pass) {
+        AXIA_CUDA(ctx, cudaMemcpyAsync(tot, ctx->d_totals, sizeof(tot), cudaMemcpyDeviceToHost, ctx->stream));
+        AXIA_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
+        for (int c = 0; c < NC; ++c) {
+          if (!(((active & ~direct) >> c) & 1u)) continue;
+          const double rn = std::sqrt(tot[c]);
+          if (rn <= P.tol * hs.bnorm[c] || !(rn <= 0.5 * hs.rmax[c])) check |= 1u << c;
+        }
       }
       if (check) {
         double t64[NC];
@@ -2106,8 +2130,8 @@ int run_segmented(axia_ctx* ctx, const void* kern, int grid, MultiArgs& P) {
           case 2: sub(k_batch_resid64_cases<2, NC>); break;
           case 4: sub(k_batch_resid64_cases<4, NC>); break;
           case 8: sub(k_batch_resid64_cases<8, NC>); break;
-          case 16: sub(k_batch_resid64_cases<16, NC>); break;
-          default: sub(k_batch_resid64_cases<32, NC>); break;
+          case 16: sub(k_batch_resid64_cases<NC < 16 ? NC : 16, NC>); break;
+          default: sub(k_batch_resid64_cases<NC, NC>); break;  // kp is at most NC
         }
         k_batch_resid_sum<<<2, NC * 32, 0, ctx->stream>>>(ctx->d_partials, g_res, 2 * NC, ctx->d_totals);
         ctx->launches += 2;
@@ -2116,7 +2140,7 @@ int run_segmented(axia_ctx* ctx, const void* kern, int grid, MultiArgs& P) {
         AXIA_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
         // double-word and FP64 residuals apart by more than 10 %: the floor is reached
         for (int c = 0; c < NC; ++c) {
-          if (!((check >> c) & 1u)) continue;
+          if (!(((check & ~direct) >> c) & 1u)) continue;
           const double a = std::sqrt(tot[c]), b = std::sqrt(t64[c]);
           if (!(std::fabs(a - b) <= 0.1 * b)) fp64_only = true;
         }
