@@ -46,7 +46,7 @@ const int kXi[20][3] = {{-1, -1, -1}, {1, -1, -1}, {1, 1, -1}, {-1, 1, -1}, {-1,
                         {-1, 0, 1},   {-1, -1, 0}, {1, -1, 0}, {1, 1, 0},   {-1, 1, 0}};
 
 constexpr int kRec = 9;  // per (element, node): 6 stresses, 3 forces
-constexpr int kGp = 15;  // per Gauss point in shared memory: w*cofactor (9), sigma (6)
+constexpr int kGp = 15;  // per Gauss point in shared memory: w * cofactor rows times sigma (9), sigma (6)
 
 template <int NN, int NG>
 struct RecoverCfg {
@@ -83,7 +83,7 @@ element_recover_kernel(int64_t n_elem, const int32_t* __restrict__ conn, const d
   double* A = s_a[warp];
   double* GP = s_gp[warp];
   const int64_t step = (int64_t)gridDim.x * WARPS * EPW;
-  const double onu = 1.0 + nu;
+  const double lam1 = nu / ((1.0 + nu) * (1.0 - 2.0 * nu)), mu1 = 0.5 / (1.0 + nu);  // of E = 1
   for (int64_t e0 = ((int64_t)blockIdx.x * WARPS + warp) * EPW; e0 < n_elem; e0 += step) {
     for (int t = lane; t < EPW * ND; t += 32) {
       const int k = t / ND, c = t % ND;
@@ -137,8 +137,7 @@ element_recover_kernel(int64_t n_elem, const int32_t* __restrict__ conn, const d
         }
         const double E = e_elem[e];
         if (!(E > 0.0)) record_error(st, e, AXIA_ERR_MATERIAL);
-        const double lam = E * nu / (onu * (1.0 - 2.0 * nu));
-        const double mu = E / (2.0 * onu);
+        const double lam = E * lam1, mu = E * mu1;
         const double inv = 1.0 / det;
         // du_q/dx_i = sum_p b[p][i] Gu[p][q] / det
         double H[3][3];
@@ -152,17 +151,18 @@ element_recover_kernel(int64_t n_elem, const int32_t* __restrict__ conn, const d
         const double gxy = H[0][1] + H[1][0], gyz = H[1][2] + H[2][1], gzx = H[2][0] + H[0][2];
         double* P = GP + (le * NG + g) * kGp;
         const double wg = s_w[g];
-#pragma unroll
-        for (int p = 0; p < 3; ++p)
-#pragma unroll
-          for (int i = 0; i < 3; ++i) P[3 * p + i] = wg * b[p][i];
         const double l2m = lam + 2.0 * mu;
-        P[9] = l2m * exx + lam * eyy + lam * ezz;
-        P[10] = lam * exx + l2m * eyy + lam * ezz;
-        P[11] = lam * exx + lam * eyy + l2m * ezz;
-        P[12] = mu * gxy;
-        P[13] = mu * gyz;
-        P[14] = mu * gzx;
+        const double sg[6] = {l2m * exx + lam * eyy + lam * ezz, lam * exx + l2m * eyy + lam * ezz,
+                              lam * exx + lam * eyy + l2m * ezz, mu * gxy, mu * gyz, mu * gzx};
+        // w sum_i b[p][i] sigma_ij: a node's force is its dN_a/dxi_p times these
+#pragma unroll
+        for (int p = 0; p < 3; ++p) {
+          P[3 * p] = wg * (b[p][0] * sg[0] + b[p][1] * sg[3] + b[p][2] * sg[5]);
+          P[3 * p + 1] = wg * (b[p][0] * sg[3] + b[p][1] * sg[1] + b[p][2] * sg[4]);
+          P[3 * p + 2] = wg * (b[p][0] * sg[5] + b[p][1] * sg[4] + b[p][2] * sg[2]);
+        }
+#pragma unroll
+        for (int c = 0; c < 6; ++c) P[9 + c] = sg[c];
       }
     }
     __syncwarp();
@@ -178,13 +178,12 @@ element_recover_kernel(int64_t n_elem, const int32_t* __restrict__ conn, const d
         const int gg = s_perm[m];
         const double* P = GP + (k * NG + gg) * kGp;
         const double* dn = s_dn + (gg * NN + a) * 3;
-        // w det dN_a/dx_i = w sum_p b[p][i] dN_a/dxi_p
-        const double gx = P[0] * dn[0] + P[3] * dn[1] + P[6] * dn[2];
-        const double gy = P[1] * dn[0] + P[4] * dn[1] + P[7] * dn[2];
-        const double gz = P[2] * dn[0] + P[5] * dn[1] + P[8] * dn[2];
-        f0 += gx * P[9] + gy * P[12] + gz * P[14];
-        f1 += gy * P[10] + gx * P[12] + gz * P[13];
-        f2 += gz * P[11] + gy * P[13] + gx * P[14];
+#pragma unroll
+        for (int p = 0; p < 3; ++p) {
+          f0 = fma(dn[p], P[3 * p], f0);
+          f1 = fma(dn[p], P[3 * p + 1], f1);
+          f2 = fma(dn[p], P[3 * p + 2], f2);
+        }
         const double xw = xrow[m];
 #pragma unroll
         for (int c = 0; c < 6; ++c) s[c] += xw * P[9 + c];
@@ -214,10 +213,199 @@ element_recover_kernel(int64_t n_elem, const int32_t* __restrict__ conn, const d
   }
 }
 
+// C3D8 with 2 x 2 x 2 points: the same numbers from the element's trilinear
+// structure, x = sum c_ijk xi^i eta^j zeta^k.  FP64 instructions bound this
+// kernel (one per SM about every 16 cycles): contracting eight nodes per point
+// took 498 FP64 instructions per warp of four elements, this form about 270
+// (with the nodal averages 6.8 -> 3.9 ms at 10^6 elements).
+//   * lane (element, field): the seven coefficients of a coordinate or
+//     displacement by a Hadamard transform (relative to node 0, which also
+//     keeps the element's distance from the origin out of the rounding), and
+//     its derivatives: along a direction they are the same at both points, so
+//     three times four values serve the eight points;
+//   * lane (element, point): Jacobian, stress, cofactor rows times stress;
+//   * a node's force needs cofactor rows times sigma only summed over the two
+//     points along each direction;
+//   * the element mean of the extrapolated stresses is the mean over the points.
+__global__ void __launch_bounds__(256)
+element_recover_hex8_kernel(int64_t n_elem, const int32_t* __restrict__ conn, const double* __restrict__ coords,
+                            const double* __restrict__ u, const double* __restrict__ e_elem, double nu,
+                            const double* __restrict__ dn_tab, const double* __restrict__ x_tab,
+                            const int* __restrict__ perm, double* __restrict__ rec, double* __restrict__ emean,
+                            DevStatus* st) {
+  constexpr int EPW = 4, WARPS = 8;
+  __shared__ double s_dn[8 * 8 * 3];
+  __shared__ double s_x[8 * 8];
+  __shared__ int s_perm[8];
+  // per warp: nodal values (4 x 48), then the point-pair sums (4 x 36); derivatives
+  // (4 x 6 x 12), then the points' results
+  __shared__ double s_a[WARPS][EPW * 48];
+  __shared__ double s_gp[WARPS][EPW * 8 * kGp];
+  for (int t = threadIdx.x; t < 8 * 8 * 3; t += blockDim.x) s_dn[t] = dn_tab[t];
+  if (threadIdx.x < 64) s_x[threadIdx.x] = x_tab[threadIdx.x];
+  if (threadIdx.x < 8) s_perm[threadIdx.x] = perm[threadIdx.x];
+  __syncthreads();
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int le = lane >> 3, g = lane & 7;
+  double* A = s_a[warp];
+  double* GP = s_gp[warp];
+  const double lam1 = nu / ((1.0 + nu) * (1.0 - 2.0 * nu)), mu1 = 0.5 / (1.0 + nu);  // of E = 1
+  // point g = 4 [xi > 0] + 2 [eta > 0] + [zeta > 0]: its derivatives along xi, eta, zeta
+  const int gx = g & 3, gy = 4 + (g >> 2) * 2 + (g & 1), gz = 8 + (g >> 1);
+  const int64_t step = (int64_t)gridDim.x * WARPS * EPW;
+  for (int64_t e0 = ((int64_t)blockIdx.x * WARPS + warp) * EPW; e0 < n_elem; e0 += step) {
+    // [element][field][node], fields x y z ux uy uz
+    for (int t = lane; t < EPW * 24; t += 32) {
+      const int k = t / 24, c = t % 24;
+      const int64_t e = e0 + k;
+      double xv = 0.0, uv = 0.0;
+      if (e < n_elem) {
+        const int64_t node = conn[e * 8 + c / 3];
+        xv = coords[3 * node + c % 3];
+        uv = u[3 * node + c % 3];
+      }
+      A[k * 48 + (c % 3) * 8 + c / 3] = xv;
+      A[k * 48 + (3 + c % 3) * 8 + c / 3] = uv;
+    }
+    __syncwarp();
+    if (g < 6) {
+      const double* v = A + le * 48 + g * 8;
+      const double v0 = v[0];
+      const double a1 = v[1] - v0, a2 = v[2] - v0, a3 = v[3] - v0, a4 = v[4] - v0, a5 = v[5] - v0, a6 = v[6] - v0,
+                   a7 = v[7] - v0;
+      // along xi: sums and differences of the edges (eta, zeta) = --, +-, -+, ++
+      const double p0 = a1, p1 = a2 + a3, p2 = a5 + a4, p3 = a6 + a7;
+      const double d0 = a1, d1 = a2 - a3, d2 = a5 - a4, d3 = a6 - a7;
+      const double pe0 = p1 - p0, pe1 = p3 - p2, ps0 = p1 + p0, ps1 = p3 + p2;  // along eta
+      const double de0 = d1 - d0, de1 = d3 - d2, ds0 = d1 + d0, ds1 = d3 + d2;
+      constexpr double G = 0.57735026918962576451;  // 1 / sqrt(3)
+      const double kx = 0.125 * (ds1 + ds0), ky = 0.125 * (pe1 + pe0), kz = 0.125 * (ps1 - ps0);
+      // xi eta, xi zeta, eta zeta at |.| = G, xi eta zeta at G^2
+      const double kxy = 0.125 * G * (de1 + de0), kxz = 0.125 * G * (ds1 - ds0), kyz = 0.125 * G * (pe1 - pe0),
+                   kxyz = (1.0 / 24.0) * (de1 - de0);
+      // d/dxi = kx + s2 kxy + s3 (kxz + s2 kxyz) and so on; signs (-, -) (-, +) (+, -) (+, +)
+      double* D = GP + (le * 6 + g) * 12;
+      const double xm = kx - kxy, xp = kx + kxy, xbm = kxz - kxyz, xbp = kxz + kxyz;
+      const double ym = ky - kxy, yp = ky + kxy, zm = kz - kxz, zp = kz + kxz, bm = kyz - kxyz, bp = kyz + kxyz;
+      D[0] = xm - xbm;
+      D[1] = xm + xbm;
+      D[2] = xp - xbp;
+      D[3] = xp + xbp;
+      D[4] = ym - bm;
+      D[5] = ym + bm;
+      D[6] = yp - bp;
+      D[7] = yp + bp;
+      D[8] = zm - bm;
+      D[9] = zm + bm;
+      D[10] = zp - bp;
+      D[11] = zp + bp;
+    }
+    __syncwarp();
+    const int64_t e = e0 + le;
+    double J[3][3], Gu[3][3];
+#pragma unroll
+    for (int q = 0; q < 3; ++q) {
+      const double *X = GP + (le * 6 + q) * 12, *U = X + 36;
+      J[q][0] = X[gx];
+      J[q][1] = X[gy];
+      J[q][2] = X[gz];
+      Gu[0][q] = U[gx];
+      Gu[1][q] = U[gy];
+      Gu[2][q] = U[gz];
+    }
+    __syncwarp();  // the derivatives are read before the points' results replace them
+    if (e < n_elem) {
+      // cofactors: inverse Jacobian = b / det (invert3 elem.rs:10-29)
+      double b[3][3];
+#pragma unroll
+      for (int i = 0; i < 3; ++i)
+#pragma unroll
+        for (int j = 0; j < 3; ++j) {
+          const int j1 = (j + 1) % 3, j2 = (j + 2) % 3, i1 = (i + 1) % 3, i2 = (i + 2) % 3;
+          b[i][j] = J[j1][i1] * J[j2][i2] - J[j1][i2] * J[j2][i1];
+        }
+      double det = J[0][0] * b[0][0] + J[0][1] * b[1][0] + J[0][2] * b[2][0];
+      if (!(fabs(det) >= 1e-18)) {
+        record_error(st, e, isfinite(det) ? AXIA_ERR_SINGULAR_JACOBIAN : AXIA_ERR_NONFINITE);
+        det = 1.0;
+      } else if (det <= 0.0) {
+        record_error(st, e, AXIA_ERR_NEG_JACOBIAN);
+      }
+      const double E = e_elem[e];
+      if (!(E > 0.0)) record_error(st, e, AXIA_ERR_MATERIAL);
+      const double s = E / det;
+      const double lam = s * lam1, mu = s * mu1;
+      // det du_q/dx_i = sum_p b[p][i] Gu[p][q]
+      double H[3][3];
+#pragma unroll
+      for (int q = 0; q < 3; ++q)
+#pragma unroll
+        for (int i = 0; i < 3; ++i) H[q][i] = fma(b[0][i], Gu[0][q], fma(b[1][i], Gu[1][q], b[2][i] * Gu[2][q]));
+      // Voigt xx yy zz xy yz zx, engineering shears (fill_b3 elem.rs:114-132)
+      const double lt = lam * (H[0][0] + H[1][1] + H[2][2]), mu2 = 2.0 * mu;
+      const double sg[6] = {fma(mu2, H[0][0], lt),      fma(mu2, H[1][1], lt),      fma(mu2, H[2][2], lt),
+                            mu * (H[0][1] + H[1][0]), mu * (H[1][2] + H[2][1]), mu * (H[2][0] + H[0][2])};
+      double* P = GP + (le * 8 + g) * kGp;
+#pragma unroll
+      for (int p = 0; p < 3; ++p) {
+        P[3 * p] = fma(b[p][0], sg[0], fma(b[p][1], sg[3], b[p][2] * sg[5]));
+        P[3 * p + 1] = fma(b[p][0], sg[3], fma(b[p][1], sg[1], b[p][2] * sg[4]));
+        P[3 * p + 2] = fma(b[p][0], sg[5], fma(b[p][1], sg[4], b[p][2] * sg[2]));
+      }
+#pragma unroll
+      for (int c = 0; c < 6; ++c) P[9 + c] = sg[c];
+    }
+    __syncwarp();
+    // sums over the two points along direction p, q = the signs of the other two
+    for (int t = lane; t < EPW * 36; t += 32) {
+      const int k = t / 36, r = t % 36, p = r / 12, j = r % 12 / 4, q = r & 3;
+      const int hi = p == 0 ? 2 : 4, lo = p == 2 ? 2 : 1, along = 4 >> p;
+      const int ga = hi * (q >> 1) + lo * (q & 1);
+      A[t] = GP[(k * 8 + ga) * kGp + 3 * p + j] + GP[(k * 8 + ga + along) * kGp + 3 * p + j];
+    }
+    __syncwarp();
+    if (e < n_elem) {
+      const int a = g;  // lanes are now (element, node)
+      double f[3] = {0.0, 0.0, 0.0}, s[6] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
+#pragma unroll
+      for (int p = 0; p < 3; ++p)
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+          const int hi = p == 0 ? 2 : 4, lo = p == 2 ? 2 : 1;
+          const double dn = s_dn[((hi * (q >> 1) + lo * (q & 1)) * 8 + a) * 3 + p];
+#pragma unroll
+          for (int j = 0; j < 3; ++j) f[j] = fma(dn, A[le * 36 + 12 * p + 4 * j + q], f[j]);
+        }
+#pragma unroll
+      for (int m = 0; m < 8; ++m) {
+        const double* P = GP + (le * 8 + s_perm[m]) * kGp + 9;
+        const double xw = s_x[a * 8 + m];
+#pragma unroll
+        for (int c = 0; c < 6; ++c) s[c] = fma(xw, P[c], s[c]);
+      }
+      double* out = rec + (e * 8 + a) * kRec;
+#pragma unroll
+      for (int c = 0; c < 6; ++c) out[c] = s[c];
+#pragma unroll
+      for (int j = 0; j < 3; ++j) out[6 + j] = f[j];
+    }
+    if (emean) {
+      if (lane < EPW * 6 && e0 + lane / 6 < n_elem) {
+        const double* P = GP + (lane / 6) * 8 * kGp + 9 + lane % 6;
+        double m = 0.0;
+#pragma unroll
+        for (int q = 0; q < 8; ++q) m += P[q * kGp];
+        emean[(e0 + lane / 6) * 6 + lane % 6] = 0.125 * m;
+      }
+    }
+    __syncwarp();
+  }
+}
+
 // One thread per node: average over the incident elements in ascending order.
 __global__ void k_recover_nodes(int64_t n_nodes, int nn, const int64_t* __restrict__ ne_ptr,
                                 const int32_t* __restrict__ ne, const double* __restrict__ rec,
-                                const double* __restrict__ f, double nu, double e_strain, double* __restrict__ stress,
+                                const double* __restrict__ f, double nu, double inv_e, double* __restrict__ stress,
                                 double* __restrict__ strain, double* __restrict__ vm, double* __restrict__ rf) {
   for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n_nodes;
        i += (int64_t)gridDim.x * blockDim.x) {
@@ -235,8 +423,9 @@ __global__ void k_recover_nodes(int64_t n_nodes, int nn, const int64_t* __restri
       cnt += 1.0;
     }
     double s[6];
+    const double inv_cnt = cnt > 0.0 ? 1.0 / cnt : 0.0;
 #pragma unroll
-    for (int c = 0; c < 6; ++c) s[c] = cnt > 0.0 ? acc[c] / cnt : 0.0;
+    for (int c = 0; c < 6; ++c) s[c] = acc[c] * inv_cnt;
     if (stress) {
 #pragma unroll
       for (int c = 0; c < 6; ++c) stress[6 * i + c] = s[c];
@@ -247,11 +436,11 @@ __global__ void k_recover_nodes(int64_t n_nodes, int nn, const int64_t* __restri
     }
     if (strain) {
       const double tr = s[0] + s[1] + s[2];
-      const double g2 = e_strain / (1.0 + nu);
+      const double inv_g2 = (1.0 + nu) * inv_e;
 #pragma unroll
-      for (int c = 0; c < 3; ++c) strain[6 * i + c] = ((1.0 + nu) * s[c] - nu * tr) / e_strain;
+      for (int c = 0; c < 3; ++c) strain[6 * i + c] = ((1.0 + nu) * s[c] - nu * tr) * inv_e;
 #pragma unroll
-      for (int c = 3; c < 6; ++c) strain[6 * i + c] = s[c] / g2;
+      for (int c = 3; c < 6; ++c) strain[6 * i + c] = s[c] * inv_g2;
     }
     if (rf) {
 #pragma unroll
@@ -435,6 +624,14 @@ void launch_element_recover(axia_ctx* ctx, const double* d_u, const double* dn, 
       ctx->d_status);
 }
 
+void launch_recover_hex8(axia_ctx* ctx, const double* d_u, const RecTables& t, double* d_emean) {
+  const unsigned grid = (unsigned)std::max<int64_t>(
+      1, std::min<int64_t>((ctx->n_elem + 31) / 32, (int64_t)ctx->sm_count * 16));
+  element_recover_hex8_kernel<<<grid, 256, 0, ctx->stream>>>(ctx->n_elem, ctx->d_conn, ctx->d_coords, d_u, ctx->d_e,
+                                                             ctx->nu, t.dn, t.x, t.perm, ctx->d_rec, d_emean,
+                                                             ctx->d_status);
+}
+
 }  // namespace
 
 // Device pointers, ordered on the context's stream.  Any output may be null.
@@ -452,7 +649,7 @@ int recover_device(axia_ctx* ctx, const double* d_u, const double* d_f, double e
   if (ctx->nn == 8 && ctx->ngp == 1)
     launch_element_recover<8, 1>(ctx, d_u, t.dn, t.w, t.x, t.perm, d_emean);
   else if (ctx->nn == 8)
-    launch_element_recover<8, 8>(ctx, d_u, t.dn, t.w, t.x, t.perm, d_emean);
+    launch_recover_hex8(ctx, d_u, t, d_emean);
   else if (ctx->nn == 4)
     launch_element_recover<4, 1>(ctx, d_u, t.dn, t.w, t.x, t.perm, d_emean);
   else if (ctx->nn == 10)
@@ -478,7 +675,7 @@ int recover_device(axia_ctx* ctx, const double* d_u, const double* d_f, double e
   const unsigned grid = (unsigned)std::max<int64_t>(
       1, std::min<int64_t>((ctx->n_nodes + 255) / 256, (int64_t)ctx->sm_count * 16));
   k_recover_nodes<<<grid, 256, 0, ctx->stream>>>(ctx->n_nodes, ctx->nn, ctx->d_ne_ptr, ctx->d_ne, ctx->d_rec, d_f,
-                                                 ctx->nu, e_strain, d_stress, d_strain, d_vm, d_rf);
+                                                 ctx->nu, 1.0 / e_strain, d_stress, d_strain, d_vm, d_rf);
   ctx->launches++;
   AXIA_CUDA(ctx, cudaGetLastError());
   DevStatus hs;
