@@ -1669,9 +1669,7 @@ int ensure_batch_buffers(axia_ctx* ctx) {
 int batch_grid(axia_ctx* ctx, const void* kern, int* grid) {
   // static + staging shared memory is above the 48 KB a block gets without opting in
   AXIA_CUDA(ctx, cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)DYN_BYTES));
-  // a thread per float4 chunk of a vector, a warp per block row: more blocks
-  // than the single system's DOF count asks for
-  AXIA_TRY(coop_grid(ctx, kern, (int)std::min<int64_t>(ctx->ndof * 8, INT32_MAX), grid, DYN_BYTES));
+  AXIA_TRY(coop_grid(ctx, kern, ctx->n_nodes * 32, grid, DYN_BYTES));  // a warp per block row
   if ((size_t)*grid * 2 * NR > ctx->partial_slots) *grid = (int)(ctx->partial_slots / (2 * NR));
   return AXIA_OK;
 }

@@ -244,7 +244,7 @@ __global__ void __launch_bounds__(PCG_THREADS) pcg_bsr_kernel(BsrPcgArgs<V> P) {
   __shared__ CgScalars<A> S;
   block_partials<A>(bb_p, rz_p, 2, P.partials, S_RR, S_RZ);
   if (!group_reduce_apply(P.bar, P.st, P.limit_ns, P.partials, P.totals, S_RR, 2, gridDim.x,
-                          [&](const double* t) { cg_begin(S, t); }))
+                          [&](const double* t) { cg_begin(S, t, P.tol); }))
     return;
   long long iters = 0;
   for (long long it = 0; !S.stop && it < P.max_iter; ++it) {
@@ -280,14 +280,14 @@ __global__ void __launch_bounds__(PCG_THREADS) pcg_bsr_kernel(BsrPcgArgs<V> P) {
     }
     block_partials<A>(rr_p, rzn_p, 2, P.partials, S_RR, S_RZ);
     if (!group_reduce_apply(P.bar, P.st, P.limit_ns, P.partials, P.totals, S_RR, 2, gridDim.x,
-                            [&](const double* t) { cg_beta(S, t, P.tol); }))
+                            [&](const double* t) { cg_beta(S, t); }))
       return;
     if (S.status != AXIA_OK || S.stop) break;
     const A beta = S.beta;
     for (int i = tid; i < nd; i += nth) P.p[i] = fma(beta, P.p[i], P.r[i] * P.dinv[i]);
     if (!grid_sync(P.bar, P.st, P.limit_ns)) return;
   }
-  if (blockIdx.x == 0 && threadIdx.x == 0) cg_out(S, P.out, P.tol, iters, 0);
+  if (blockIdx.x == 0 && threadIdx.x == 0) cg_out(S, sqrt(S.rr), P.out, P.tol, iters, 0);
 }
 
 // FP32 CG on the FP32 node-block matrix with FP64 reliable updates (the
@@ -355,7 +355,7 @@ __device__ __forceinline__ void reliable_body(const BsrReliableArgs& P, const Co
   __shared__ CgScalars<float> S;
   block_partials<double>(bb_p, (double)rz_p, 2, partials, S_RR, S_RZ, R.nblk, R.rank);
   if (!group_reduce_apply(R.bar, P.st, P.limit_ns, partials, totals, S_RR, 2, R.nblk,
-                          [&](const double* t) { mixed_begin(S, t); }))
+                          [&](const double* t) { mixed_begin(S, t, P.tol, P.delta); }))
     return;
   long long iters = 0;
   int updates = 0;
@@ -416,7 +416,7 @@ __device__ __forceinline__ void reliable_body(const BsrReliableArgs& P, const Co
     }
     block_partials<float>(rr_p, rzn_p, 2, partials, S_RR, S_RZ, R.nblk, R.rank);
     if (!group_reduce_apply(R.bar, P.st, P.limit_ns, partials, totals, S_RR, 2, R.nblk, [&](const double* t) {
-          mixed_check(S, t[0], P.tol, P.delta);
+          mixed_check(S, t[0]);
           mixed_rz<COARSE>(S, (float)t[1], !S.update);
         }))
       return;
@@ -451,7 +451,7 @@ __device__ __forceinline__ void reliable_body(const BsrReliableArgs& P, const Co
       }
       block_partials<double>(rr64_p, (double)rz_new_p, 2, partials, S_RR, S_RZ, R.nblk, R.rank);
       if (!group_reduce_apply(R.bar, P.st, P.limit_ns, partials, totals, S_RR, 2, R.nblk, [&](const double* t) {
-            mixed_replaced(S, t[0], P.tol);
+            mixed_replaced(S, t[0], P.tol, P.delta);
             mixed_rz<COARSE>(S, (float)t[1], true);
           }))
         return;
@@ -472,7 +472,7 @@ __device__ __forceinline__ void reliable_body(const BsrReliableArgs& P, const Co
       for (int i = i0 + tid; i < nd; i += nth) P.p32[i] = fmaf(beta, P.p32[i], P.r32[i] * P.dinv32[i]);
     if (!group_sync(R.bar, P.st, P.limit_ns, R.nblk)) return;
   }
-  if (R.rank == 0 && threadIdx.x == 0) cg_out(S, R.out, P.tol, iters, updates);
+  if (R.rank == 0 && threadIdx.x == 0) cg_out(S, S.residual, R.out, P.tol, iters, updates);
 }
 
 // FP64 reliable updates: 4 lanes per block row; 2 blocks per load where the
@@ -654,7 +654,7 @@ template <typename V, int L>
 static int launch_bsr_pcg_t(axia_ctx* ctx, BsrPcgArgs<V>& P) {
   auto kern = pcg_bsr_kernel<V, L>;
   int grid = 0;
-  AXIA_TRY(coop_grid(ctx, (const void*)kern, P.nd, &grid));
+  AXIA_TRY(coop_grid(ctx, (const void*)kern, (int64_t)P.M.n_nodes * L, &grid));
   void* params[] = {&P};
   AXIA_CUDA(ctx, cudaLaunchCooperativeKernel((const void*)kern, dim3(grid), dim3(PCG_THREADS), params, 0, ctx->stream));
   ctx->launches++;
@@ -675,7 +675,7 @@ template <int L32, int V32, bool COARSE, bool SYM = false>
 static int launch_bsr_rel_t(axia_ctx* ctx, BsrReliableArgs& P) {
   auto kern = pcg_bsr_reliable_kernel<L32, V32, COARSE, SYM>;
   int grid = 0;
-  AXIA_TRY(coop_grid(ctx, (const void*)kern, P.nd, &grid));
+  AXIA_TRY(coop_grid(ctx, (const void*)kern, (int64_t)P.M64.n_nodes * L32, &grid));
   void* params[] = {&P};
   AXIA_CUDA(ctx, cudaLaunchCooperativeKernel((const void*)kern, dim3(grid), dim3(PCG_THREADS), params, 0, ctx->stream));
   ctx->launches++;

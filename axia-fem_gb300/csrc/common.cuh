@@ -162,7 +162,7 @@ __device__ __forceinline__ bool grid_sync(GridBarrier* bar, DevStatus* st, unsig
 }
 
 // Grid-wide barrier that also reduces.  Every block has stored its partials of
-// nv <= 4 values at partials[(slot0 + k) * nblk + rank]; the last block to
+// nv <= 2 values at partials[(slot0 + k) * nblk + rank]; the last block to
 // arrive sums them (one L2 round trip; thread t takes blocks t, t +
 // blockDim.x, ..., then warps and the warp sums in order: a fixed order, so
 // every run gives the same bits) and publishes totals[slot0 + k] before it
@@ -175,7 +175,7 @@ __device__ __forceinline__ bool grid_sync(GridBarrier* bar, DevStatus* st, unsig
 // a division of about 20 instructions each, executed by all 16 to 64 warps of
 // an SM, took 6 to 30 us per iteration; on one thread they take 0.6 us.
 // Likewise only the warps that hold partials join the sums.
-constexpr int REDUCE_MAX_NV = 4;
+constexpr int REDUCE_MAX_NV = 2;
 
 // The last block's part of group_reduce_sync (every thread of the block calls
 // it).  Not inlined: its registers stay out of the allocation of the CG loops
@@ -184,24 +184,26 @@ static __device__ __noinline__ void reduce_partials_last_block(const double* par
                                                         int slot0, int nv, unsigned nblk) {
   __shared__ double s_sum[REDUCE_MAX_NV][32];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nw = blockDim.x >> 5;
-  const int used = min(nw, (int)((nblk + 31) >> 5));  // the other warps hold no partials
+  // one warp reads up to 5 partials per lane (a second level of FP64 sums costs
+  // more than four dependent additions); beyond that, the warps that hold any
+  const int used = nblk <= 160 ? 1 : min(nw, (int)((nblk + 31) >> 5));
   if (warp < used) {
-    double a[REDUCE_MAX_NV];
-#pragma unroll
-    for (int k = 0; k < REDUCE_MAX_NV; ++k) a[k] = 0.0;
-    for (int j = threadIdx.x; j < (int)nblk; j += blockDim.x) {
-      double v[REDUCE_MAX_NV];
-#pragma unroll
-      for (int k = 0; k < REDUCE_MAX_NV; ++k) v[k] = k < nv ? __ldcg(partials + (size_t)(slot0 + k) * nblk + j) : 0.0;
-#pragma unroll
-      for (int k = 0; k < REDUCE_MAX_NV; ++k) a[k] += v[k];
-    }
 #pragma unroll
     for (int k = 0; k < REDUCE_MAX_NV; ++k) {
-      if (k < nv) {
-        a[k] = warp_sum(a[k]);
-        if (lane == 0) s_sum[k][warp] = a[k];
+      if (k >= nv) break;
+      const double* p = partials + (size_t)(slot0 + k) * nblk;
+      double a = 0.0;
+      for (int j = threadIdx.x; j < (int)nblk; j += 5 * 32 * used) {
+        double v[5];
+#pragma unroll
+        for (int q = 0; q < 5; ++q) v[q] = j + q * 32 * used < (int)nblk ? __ldcg(p + j + q * 32 * used) : 0.0;
+        a += v[0];
+#pragma unroll
+        for (int q = 1; q < 5; ++q)
+          if (q * 32 * used < (int)nblk) a += v[q];
       }
+      a = warp_sum(a);
+      if (lane == 0) s_sum[k][warp] = a;
     }
   }
   __syncthreads();
@@ -210,7 +212,7 @@ static __device__ __noinline__ void reduce_partials_last_block(const double* par
     for (int k = 0; k < REDUCE_MAX_NV; ++k) {
       if (k < nv) {
         double t = lane < used ? s_sum[k][lane] : 0.0;
-        t = warp_sum(t);
+        if (used > 1) t = warp_sum(t);
         if (lane == 0) {
           totals[slot0 + k] = t;
           s_tot[k] = t;
@@ -238,8 +240,7 @@ __device__ __forceinline__ bool group_reduce_apply(GridBarrier* bar, DevStatus* 
   if (threadIdx.x == 0) {
     int ok = 1;
     if (s_last) {
-      __threadfence();
-      barrier_release(bar, s_gen);
+      barrier_release(bar, s_gen);  // a release store: after thread 0's own totals
     } else {
       ok = barrier_wait(bar, st, limit_ns, s_gen);
       if (ok)
@@ -250,24 +251,6 @@ __device__ __forceinline__ bool group_reduce_apply(GridBarrier* bar, DevStatus* 
   }
   __syncthreads();
   return s_ok2 != 0;
-}
-
-// The same, every thread getting the totals themselves in res[0 .. nv).
-__device__ __forceinline__ bool group_reduce_sync(GridBarrier* bar, DevStatus* st, unsigned long long limit_ns,
-                                                  const double* partials, double* totals, int slot0, int nv,
-                                                  unsigned nblk, double* res) {
-  __shared__ double s_res[REDUCE_MAX_NV];
-  const bool ok = group_reduce_apply(bar, st, limit_ns, partials, totals, slot0, nv, nblk, [&](const double* t) {
-    for (int k = 0; k < nv; ++k) s_res[k] = t[k];
-  });
-  for (int k = 0; k < nv; ++k) res[k] = s_res[k];
-  return ok;
-}
-
-__device__ __forceinline__ bool grid_reduce_sync(GridBarrier* bar, DevStatus* st, unsigned long long limit_ns,
-                                                 const double* partials, double* totals, int slot0, int nv,
-                                                 double* res) {
-  return group_reduce_sync(bar, st, limit_ns, partials, totals, slot0, nv, gridDim.x, res);
 }
 
 // Streaming (evict-first) loads for matrix data that is read once per sweep,

@@ -64,7 +64,7 @@ __global__ void __launch_bounds__(PCG_THREADS) pcg_kernel(PcgArgs<V> P) {
   __shared__ CgScalars<A> S;
   block_partials<A>(bb_p, rz_p, 2, P.partials, S_RR, S_RZ);
   if (!group_reduce_apply(P.bar, P.st, P.limit_ns, P.partials, P.totals, S_RR, 2, gridDim.x,
-                          [&](const double* t) { cg_begin(S, t); }))
+                          [&](const double* t) { cg_begin(S, t, P.tol); }))
     return;
   long long iters = 0;
   for (long long it = 0; !S.stop && it < P.max_iter; ++it) {
@@ -97,14 +97,14 @@ __global__ void __launch_bounds__(PCG_THREADS) pcg_kernel(PcgArgs<V> P) {
     }
     block_partials<A>(rr_p, rzn_p, 2, P.partials, S_RR, S_RZ);
     if (!group_reduce_apply(P.bar, P.st, P.limit_ns, P.partials, P.totals, S_RR, 2, gridDim.x,
-                            [&](const double* t) { cg_beta(S, t, P.tol); }))
+                            [&](const double* t) { cg_beta(S, t); }))
       return;
     if (S.status != AXIA_OK || S.stop) break;
     const A beta = S.beta;
     for (int i = tid; i < n; i += nth) P.p[i] = fma(beta, P.p[i], P.r[i] * P.dinv[i]);
     if (!grid_sync(P.bar, P.st, P.limit_ns)) return;
   }
-  if (blockIdx.x == 0 && threadIdx.x == 0) cg_out(S, P.out, P.tol, iters, 0);
+  if (blockIdx.x == 0 && threadIdx.x == 0) cg_out(S, sqrt(S.rr), P.out, P.tol, iters, 0);
 }
 
 // ---------------------------------------------------------------------------
@@ -161,7 +161,7 @@ __global__ void __launch_bounds__(PCG_THREADS, 4) pcg_reliable_kernel(ReliableAr
   __shared__ CgScalars<float> S;
   block_partials<double>(bb_p, (double)rz_p, 2, P.partials, S_RR, S_RZ);
   if (!group_reduce_apply(P.bar, P.st, P.limit_ns, P.partials, P.totals, S_RR, 2, gridDim.x,
-                          [&](const double* t) { mixed_begin(S, t); }))
+                          [&](const double* t) { mixed_begin(S, t, P.tol, P.delta); }))
     return;
   long long iters = 0;
   int updates = 0;
@@ -198,7 +198,7 @@ __global__ void __launch_bounds__(PCG_THREADS, 4) pcg_reliable_kernel(ReliableAr
     block_partials<float>(rr_p, rzn_p, 2, P.partials, S_RR, S_RZ);
     if (!group_reduce_apply(P.bar, P.st, P.limit_ns, P.partials, P.totals, S_RR, 2, gridDim.x,
                             [&](const double* t) {
-                              mixed_check(S, t[0], P.tol, P.delta);
+                              mixed_check(S, t[0]);
                               mixed_rz<false>(S, (float)t[1], !S.update);
                             }))
       return;
@@ -231,7 +231,7 @@ __global__ void __launch_bounds__(PCG_THREADS, 4) pcg_reliable_kernel(ReliableAr
       block_partials<double>(rr64_p, (double)rz_new_p, 2, P.partials, S_RR, S_RZ);
       if (!group_reduce_apply(P.bar, P.st, P.limit_ns, P.partials, P.totals, S_RR, 2, gridDim.x,
                               [&](const double* t) {
-                                mixed_replaced(S, t[0], P.tol);
+                                mixed_replaced(S, t[0], P.tol, P.delta);
                                 mixed_rz<false>(S, (float)t[1], true);
                               }))
         return;
@@ -242,7 +242,7 @@ __global__ void __launch_bounds__(PCG_THREADS, 4) pcg_reliable_kernel(ReliableAr
     for (int i = tid; i < n; i += nth) P.p32[i] = fmaf(beta, P.p32[i], P.r32[i] * P.dinv32[i]);
     if (!grid_sync(P.bar, P.st, P.limit_ns)) return;
   }
-  if (blockIdx.x == 0 && threadIdx.x == 0) cg_out(S, P.out, P.tol, iters, updates);
+  if (blockIdx.x == 0 && threadIdx.x == 0) cg_out(S, S.residual, P.out, P.tol, iters, updates);
 }
 
 // ---------------------------------------------------------------------------
@@ -340,17 +340,20 @@ __global__ void k_reconstruct(int64_t ndof, const int32_t* ind_of, const double*
 // ---------------------------------------------------------------------------
 // Host launchers
 // ---------------------------------------------------------------------------
-// Lanes per CSR row.  FP64 work is scarce on GB300 (about 1/58 of the FP32
+// Lanes per CSR row.  FP64 work is scarce on GB300 (about 1/75 of the FP32
 // rate), so the FP64 SpMV uses few lanes per row (fewer shuffle-add steps per
 // row); the FP32 SpMV can afford wider groups for better coalescing.
-static int pick_lanes(double avg_row, bool fp32) {
+// Measured, FP64 CG of C3D8 blocks, us per iteration with 4 / 8 lanes: 6 k rows
+// 19.0 / 17.8, 17 k 19.9 / 21.1, 71 k 32.8 / 35.1, 104 k 41.1 / 45.0, 670 k
+// 154 / 176, 2.2 M 570 / 532 (there the wider loads stream better).
+static int pick_lanes(double avg_row, bool fp32, int64_t rows) {
   if (fp32) {
     if (avg_row <= 12) return 4;
     if (avg_row <= 128) return 8;
     return 16;
   }
   if (avg_row <= 24) return 4;
-  if (avg_row <= 160) return 8;
+  if (avg_row <= 160) return rows >= 8000 && rows < 1500000 ? 4 : 8;
   return 16;
 }
 
@@ -358,14 +361,14 @@ int pcg_lanes_for(const axia_ctx* ctx, bool fp32, int requested) {
   if (requested == 1 || requested == 2 || requested == 4 || requested == 8 || requested == 16 || requested == 32)
     return requested;
   double avg = ctx->n_free ? (double)ctx->nnz / (double)ctx->n_free : 1.0;
-  return pick_lanes(avg, fp32);
+  return pick_lanes(avg, fp32, ctx->n_free);
 }
 
 template <typename V, int L>
 static int launch_pcg_t(axia_ctx* ctx, PcgArgs<V>& P) {
   auto kern = pcg_kernel<V, L>;
   int grid = 0;
-  AXIA_TRY(coop_grid(ctx, (const void*)kern, P.n, &grid));
+  AXIA_TRY(coop_grid(ctx, (const void*)kern, (int64_t)P.n * L, &grid));
   void* params[] = {&P};
   AXIA_CUDA(ctx, cudaLaunchCooperativeKernel((const void*)kern, dim3(grid), dim3(PCG_THREADS), params, 0, ctx->stream));
   ctx->launches++;
@@ -388,7 +391,7 @@ template <int L32, int L64>
 static int launch_reliable_t(axia_ctx* ctx, ReliableArgs& P) {
   auto kern = pcg_reliable_kernel<L32, L64>;
   int grid = 0;
-  AXIA_TRY(coop_grid(ctx, (const void*)kern, P.n, &grid));
+  AXIA_TRY(coop_grid(ctx, (const void*)kern, (int64_t)P.n * L32, &grid));
   void* params[] = {&P};
   AXIA_CUDA(ctx, cudaLaunchCooperativeKernel((const void*)kern, dim3(grid), dim3(PCG_THREADS), params, 0, ctx->stream));
   ctx->launches++;
