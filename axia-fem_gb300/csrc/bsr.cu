@@ -242,9 +242,8 @@ __global__ void __launch_bounds__(PCG_THREADS) pcg_bsr_kernel(BsrPcgArgs<V> P) {
     bb_p = fma(bi, bi, bb_p);
   }
   __shared__ CgScalars<A> S;
-  block_partials<A>(bb_p, rz_p, 2, P.partials, S_RR, S_RZ);
-  if (!group_reduce_apply(P.bar, P.st, P.limit_ns, P.partials, P.totals, S_RR, 2, gridDim.x,
-                          [&](const double* t) { cg_begin(S, t, P.tol); }))
+  BlockSync<false> Y{P.bar, P.st, P.limit_ns, P.partials, P.totals, gridDim.x, blockIdx.x, 0};
+  if (!Y.template reduce<2>(bb_p, rz_p, S_RR, [&](const double* t) { cg_begin(S, t, P.tol); }))
     return;
   long long iters = 0;
   for (long long it = 0; !S.stop && it < P.max_iter; ++it) {
@@ -263,9 +262,7 @@ __global__ void __launch_bounds__(PCG_THREADS) pcg_bsr_kernel(BsrPcgArgs<V> P) {
         pq_p = fma((A)P.p[3 * a + 2], y2, pq_p);
       }
     }
-    block_partials<A>(pq_p, A(0), 1, P.partials, S_PQ, S_PQ);
-    if (!group_reduce_apply(P.bar, P.st, P.limit_ns, P.partials, P.totals, S_PQ, 1, gridDim.x,
-                            [&](const double* t) { cg_alpha(S, t); }))
+    if (!Y.template reduce<1>(pq_p, A(0), S_PQ, [&](const double* t) { cg_alpha(S, t); }))
       return;
     if (S.status != AXIA_OK) break;
     const A alpha = S.alpha;
@@ -278,14 +275,12 @@ __global__ void __launch_bounds__(PCG_THREADS) pcg_bsr_kernel(BsrPcgArgs<V> P) {
       rr_p = fma(ri, ri, rr_p);
       rzn_p = fma(ri, ri * di, rzn_p);
     }
-    block_partials<A>(rr_p, rzn_p, 2, P.partials, S_RR, S_RZ);
-    if (!group_reduce_apply(P.bar, P.st, P.limit_ns, P.partials, P.totals, S_RR, 2, gridDim.x,
-                            [&](const double* t) { cg_beta(S, t); }))
+    if (!Y.template reduce<2>(rr_p, rzn_p, S_RR, [&](const double* t) { cg_beta(S, t); }))
       return;
     if (S.status != AXIA_OK || S.stop) break;
     const A beta = S.beta;
     for (int i = tid; i < nd; i += nth) P.p[i] = fma(beta, P.p[i], P.r[i] * P.dinv[i]);
-    if (!grid_sync(P.bar, P.st, P.limit_ns)) return;
+    if (!Y.sync()) return;
   }
   if (blockIdx.x == 0 && threadIdx.x == 0) cg_out(S, sqrt(S.rr), P.out, P.tol, iters, 0);
 }
@@ -309,12 +304,12 @@ struct SolveRange {
 // The coarse solve of the two-level preconditioner, r_c complete:
 // y = M r_c, and r_c . y reduced over the group; the direction's beta (or, for
 // the first direction, the coarse part of r.z) follows on thread 0.
-__device__ __forceinline__ bool coarse_step(const BsrReliableArgs& P, const CoarseArgs& C, const SolveRange& R,
-                                            int gwarp, int nwarps, int lane, CgScalars<float>& S, bool first) {
+template <bool CLUSTER>
+__device__ __forceinline__ bool coarse_step(const CoarseArgs& C, BlockSync<CLUSTER>& Y, int gwarp, int nwarps, int lane,
+                                            CgScalars<float>& S, bool first) {
   __shared__ __align__(16) float s_rc[COARSE_MAX];
   const float acc = coarse_solve(C, s_rc, gwarp, nwarps, lane);
-  block_partials<float>(acc, 0.f, 1, R.partials, S_RC, S_RC, R.nblk, R.rank);
-  return group_reduce_apply(R.bar, P.st, P.limit_ns, R.partials, R.totals, S_RC, 1, R.nblk, [&](const double* t) {
+  return Y.template reduce<1>(acc, 0.f, S_PQ, [&](const double* t) {
     if (first)
       S.rz += (float)t[0];
     else
@@ -322,7 +317,7 @@ __device__ __forceinline__ bool coarse_step(const BsrReliableArgs& P, const Coar
   });
 }
 
-template <int L32, int V32, int L64, int V64, bool COARSE = false, bool SYM = false>
+template <int L32, int V32, int L64, int V64, bool COARSE = false, bool SYM = false, bool CLUSTER = false>
 __device__ __forceinline__ void reliable_body(const BsrReliableArgs& P, const CoarseArgs& C, const SolveRange& R) {
   const int n0 = R.node0, n1 = R.node1;
   const int i0 = 3 * n0;
@@ -337,8 +332,6 @@ __device__ __forceinline__ void reliable_body(const BsrReliableArgs& P, const Co
   const int cwarp = (threadIdx.x >> 5) * R.nblk + R.rank;
   const int lane = threadIdx.x & 31;
   const int nd = 3 * n1;  // vector loops run over [i0, 3 n1)
-  double* const partials = R.partials;
-  double* const totals = R.totals;
   float rz_p = 0.f;
   double bb_p = 0.0;
   for (int i = i0 + tid; i < nd; i += nth) {
@@ -353,19 +346,19 @@ __device__ __forceinline__ void reliable_body(const BsrReliableArgs& P, const Co
     bb_p = fma(bi, bi, bb_p);
   }
   __shared__ CgScalars<float> S;
-  block_partials<double>(bb_p, (double)rz_p, 2, partials, S_RR, S_RZ, R.nblk, R.rank);
-  if (!group_reduce_apply(R.bar, P.st, P.limit_ns, partials, totals, S_RR, 2, R.nblk,
-                          [&](const double* t) { mixed_begin(S, t, P.tol, P.delta); }))
+  BlockSync<CLUSTER> Y{R.bar, P.st, P.limit_ns, R.partials, R.totals, R.nblk, R.rank, 0};
+  Y.fence_lifetime();
+  if (!Y.template reduce<2>(bb_p, (double)rz_p, S_RR, [&](const double* t) { mixed_begin(S, t, P.tol, P.delta); }))
     return;
   long long iters = 0;
   int updates = 0;
   if constexpr (COARSE) {
     if (!S.stop) {  // p = D^-1 b + Z M Z^T b
       coarse_restrict(C, P.r32, cwarp, nwarps, lane);
-      if (!group_sync(R.bar, P.st, P.limit_ns, R.nblk)) return;
-      if (!coarse_step(P, C, R, gwarp, nwarps, lane, S, true)) return;
+      if (!Y.sync()) return;
+      if (!coarse_step(C, Y, gwarp, nwarps, lane, S, true)) return;
       coarse_update_p(C, n0, n1, tid, nth, 0.f, P.r32, P.dinv32, P.p32, true);
-      if (!group_sync(R.bar, P.st, P.limit_ns, R.nblk)) return;
+      if (!Y.sync()) return;
     }
   }
   for (long long it = 0; !S.stop && it < P.max_iter; ++it) {
@@ -395,9 +388,7 @@ __device__ __forceinline__ void reliable_body(const BsrReliableArgs& P, const Co
         }
       }
     }
-    block_partials<float>(pq_p, 0.f, 1, partials, S_PQ, S_PQ, R.nblk, R.rank);
-    if (!group_reduce_apply(R.bar, P.st, P.limit_ns, partials, totals, S_PQ, 1, R.nblk,
-                            [&](const double* t) { mixed_alpha(S, t); }))
+    if (!Y.template reduce<1>(pq_p, 0.f, S_PQ, [&](const double* t) { mixed_alpha(S, t); }))
       return;
     if (S.status != AXIA_OK) break;
     const float alpha = S.alpha;
@@ -414,8 +405,7 @@ __device__ __forceinline__ void reliable_body(const BsrReliableArgs& P, const Co
         rzn_p = fmaf(ri, ri * di, rzn_p);
       }
     }
-    block_partials<float>(rr_p, rzn_p, 2, partials, S_RR, S_RZ, R.nblk, R.rank);
-    if (!group_reduce_apply(R.bar, P.st, P.limit_ns, partials, totals, S_RR, 2, R.nblk, [&](const double* t) {
+    if (!Y.template reduce<2>(rr_p, rzn_p, S_RR, [&](const double* t) {
           mixed_check(S, t[0]);
           mixed_rz<COARSE>(S, (float)t[1], !S.update);
         }))
@@ -426,7 +416,7 @@ __device__ __forceinline__ void reliable_body(const BsrReliableArgs& P, const Co
         P.x[i] += (double)P.x32[i];
         P.x32[i] = 0.f;
       }
-      if (!group_sync(R.bar, P.st, P.limit_ns, R.nblk)) return;
+      if (!Y.sync()) return;
       double rr64_p = 0.0;
       float rz_new_p = 0.f;
       {
@@ -449,8 +439,7 @@ __device__ __forceinline__ void reliable_body(const BsrReliableArgs& P, const Co
           }
         }
       }
-      block_partials<double>(rr64_p, (double)rz_new_p, 2, partials, S_RR, S_RZ, R.nblk, R.rank);
-      if (!group_reduce_apply(R.bar, P.st, P.limit_ns, partials, totals, S_RR, 2, R.nblk, [&](const double* t) {
+      if (!Y.template reduce<2>(rr64_p, (double)rz_new_p, S_RR, [&](const double* t) {
             mixed_replaced(S, t[0], P.tol, P.delta);
             mixed_rz<COARSE>(S, (float)t[1], true);
           }))
@@ -459,19 +448,20 @@ __device__ __forceinline__ void reliable_body(const BsrReliableArgs& P, const Co
       if (S.status != AXIA_OK || S.stop) break;
       if constexpr (COARSE) {  // r was replaced: restrict it again
         coarse_restrict(C, P.r32, cwarp, nwarps, lane);
-        if (!group_sync(R.bar, P.st, P.limit_ns, R.nblk)) return;
+        if (!Y.sync()) return;
       }
     }
     if constexpr (COARSE) {
-      if (!coarse_step(P, C, R, gwarp, nwarps, lane, S, false)) return;
+      if (!coarse_step(C, Y, gwarp, nwarps, lane, S, false)) return;
     }
     const float beta = S.beta;
     if constexpr (COARSE)
       coarse_update_p(C, n0, n1, tid, nth, beta, P.r32, P.dinv32, P.p32, false);
     else
       for (int i = i0 + tid; i < nd; i += nth) P.p32[i] = fmaf(beta, P.p32[i], P.r32[i] * P.dinv32[i]);
-    if (!group_sync(R.bar, P.st, P.limit_ns, R.nblk)) return;
+    if (!Y.sync()) return;
   }
+  Y.fence_lifetime();
   if (R.rank == 0 && threadIdx.x == 0) cg_out(S, S.residual, R.out, P.tol, iters, updates);
 }
 
@@ -485,10 +475,10 @@ __host__ __device__ constexpr int rel_v64() { return V32 >= 4 ? 2 : 1; }
 template <int V32>
 __host__ __device__ constexpr int rel_min_blocks() { return V32 >= 4 ? 2 : 3; }
 
-template <int L32, int V32, bool COARSE = false, bool SYM = false>
+template <int L32, int V32, bool COARSE = false, bool SYM = false, bool CLUSTER = false>
 __global__ void __launch_bounds__(PCG_THREADS, rel_min_blocks<V32>()) pcg_bsr_reliable_kernel(BsrReliableArgs P) {
   const SolveRange R{0, P.M64.n_nodes, blockIdx.x, gridDim.x, P.partials, P.totals, P.bar, P.out};
-  reliable_body<L32, V32, kL64, rel_v64<V32>(), COARSE, SYM>(P, P.C, R);
+  reliable_body<L32, V32, kL64, rel_v64<V32>(), COARSE, SYM, CLUSTER>(P, P.C, R);
 }
 
 // Independent systems on disjoint node ranges of one node-block matrix (the
@@ -548,7 +538,7 @@ __global__ void __launch_bounds__(PCG_THREADS) bsr_residual_kernel(BsrMat<double
       rr = fma(r0, r0, fma(r1, r1, fma(r2, r2, rr)));
     }
   }
-  block_partials<double>(rr, 0.0, 1, partials, 0, 0);
+  block_partial(rr, partials);
 }
 
 // ---------------------------------------------------------------------------
@@ -675,6 +665,12 @@ template <int L32, int V32, bool COARSE, bool SYM = false>
 static int launch_bsr_rel_t(axia_ctx* ctx, BsrReliableArgs& P) {
   auto kern = pcg_bsr_reliable_kernel<L32, V32, COARSE, SYM>;
   int grid = 0;
+  if constexpr (V32 == 4 && !SYM) {
+    const void* one = (const void*)pcg_bsr_reliable_kernel<L32, V32, COARSE, false, true>;
+    void* params1[] = {&P};
+    const int blocks = ctx->nbq <= CLUSTER_MAX_BLOCKS ? cluster_blocks(one, (int64_t)P.M64.n_nodes * L32) : 0;
+    if (blocks) return launch_cluster(ctx, one, blocks, params1);
+  }
   AXIA_TRY(coop_grid(ctx, (const void*)kern, (int64_t)P.M64.n_nodes * L32, &grid));
   void* params[] = {&P};
   AXIA_CUDA(ctx, cudaLaunchCooperativeKernel((const void*)kern, dim3(grid), dim3(PCG_THREADS), params, 0, ctx->stream));

@@ -40,7 +40,7 @@ __device__ __forceinline__ A csr_row_dot(int row, int n, int sl, const int* __re
   return group_sum<L>(s);
 }
 
-template <typename V, int L>
+template <typename V, int L, bool CLUSTER = false>
 __global__ void __launch_bounds__(PCG_THREADS) pcg_kernel(PcgArgs<V> P) {
   using A = V;  // accumulation in the storage precision (FP64 or FP32)
   const int n = P.n;
@@ -62,9 +62,9 @@ __global__ void __launch_bounds__(PCG_THREADS) pcg_kernel(PcgArgs<V> P) {
     bb_p = fma(bi, bi, bb_p);
   }
   __shared__ CgScalars<A> S;
-  block_partials<A>(bb_p, rz_p, 2, P.partials, S_RR, S_RZ);
-  if (!group_reduce_apply(P.bar, P.st, P.limit_ns, P.partials, P.totals, S_RR, 2, gridDim.x,
-                          [&](const double* t) { cg_begin(S, t, P.tol); }))
+  BlockSync<CLUSTER> Y{P.bar, P.st, P.limit_ns, P.partials, P.totals, gridDim.x, blockIdx.x, 0};
+  Y.fence_lifetime();
+  if (!Y.template reduce<2>(bb_p, rz_p, S_RR, [&](const double* t) { cg_begin(S, t, P.tol); }))
     return;
   long long iters = 0;
   for (long long it = 0; !S.stop && it < P.max_iter; ++it) {
@@ -79,9 +79,7 @@ __global__ void __launch_bounds__(PCG_THREADS) pcg_kernel(PcgArgs<V> P) {
         pq_p = fma((A)P.p[row], s, pq_p);
       }
     }
-    block_partials<A>(pq_p, A(0), 1, P.partials, S_PQ, S_PQ);
-    if (!group_reduce_apply(P.bar, P.st, P.limit_ns, P.partials, P.totals, S_PQ, 1, gridDim.x,
-                            [&](const double* t) { cg_alpha(S, t); }))
+    if (!Y.template reduce<1>(pq_p, A(0), S_PQ, [&](const double* t) { cg_alpha(S, t); }))
       return;
     if (S.status != AXIA_OK) break;
     const A alpha = S.alpha;
@@ -95,15 +93,14 @@ __global__ void __launch_bounds__(PCG_THREADS) pcg_kernel(PcgArgs<V> P) {
       rr_p = fma(ri, ri, rr_p);
       rzn_p = fma(ri, ri * di, rzn_p);
     }
-    block_partials<A>(rr_p, rzn_p, 2, P.partials, S_RR, S_RZ);
-    if (!group_reduce_apply(P.bar, P.st, P.limit_ns, P.partials, P.totals, S_RR, 2, gridDim.x,
-                            [&](const double* t) { cg_beta(S, t); }))
+    if (!Y.template reduce<2>(rr_p, rzn_p, S_RR, [&](const double* t) { cg_beta(S, t); }))
       return;
     if (S.status != AXIA_OK || S.stop) break;
     const A beta = S.beta;
     for (int i = tid; i < n; i += nth) P.p[i] = fma(beta, P.p[i], P.r[i] * P.dinv[i]);
-    if (!grid_sync(P.bar, P.st, P.limit_ns)) return;
+    if (!Y.sync()) return;
   }
+  Y.fence_lifetime();
   if (blockIdx.x == 0 && threadIdx.x == 0) cg_out(S, sqrt(S.rr), P.out, P.tol, iters, 0);
 }
 
@@ -159,9 +156,8 @@ __global__ void __launch_bounds__(PCG_THREADS, 4) pcg_reliable_kernel(ReliableAr
     bb_p = fma(bi, bi, bb_p);
   }
   __shared__ CgScalars<float> S;
-  block_partials<double>(bb_p, (double)rz_p, 2, P.partials, S_RR, S_RZ);
-  if (!group_reduce_apply(P.bar, P.st, P.limit_ns, P.partials, P.totals, S_RR, 2, gridDim.x,
-                          [&](const double* t) { mixed_begin(S, t, P.tol, P.delta); }))
+  BlockSync<false> Y{P.bar, P.st, P.limit_ns, P.partials, P.totals, gridDim.x, blockIdx.x, 0};
+  if (!Y.template reduce<2>(bb_p, (double)rz_p, S_RR, [&](const double* t) { mixed_begin(S, t, P.tol, P.delta); }))
     return;
   long long iters = 0;
   int updates = 0;
@@ -180,9 +176,7 @@ __global__ void __launch_bounds__(PCG_THREADS, 4) pcg_reliable_kernel(ReliableAr
         }
       }
     }
-    block_partials<float>(pq_p, 0.f, 1, P.partials, S_PQ, S_PQ);
-    if (!group_reduce_apply(P.bar, P.st, P.limit_ns, P.partials, P.totals, S_PQ, 1, gridDim.x,
-                            [&](const double* t) { mixed_alpha(S, t); }))
+    if (!Y.template reduce<1>(pq_p, 0.f, S_PQ, [&](const double* t) { mixed_alpha(S, t); }))
       return;
     if (S.status != AXIA_OK) break;
     const float alpha = S.alpha;
@@ -195,9 +189,7 @@ __global__ void __launch_bounds__(PCG_THREADS, 4) pcg_reliable_kernel(ReliableAr
       rr_p = fmaf(ri, ri, rr_p);
       rzn_p = fmaf(ri, ri * di, rzn_p);
     }
-    block_partials<float>(rr_p, rzn_p, 2, P.partials, S_RR, S_RZ);
-    if (!group_reduce_apply(P.bar, P.st, P.limit_ns, P.partials, P.totals, S_RR, 2, gridDim.x,
-                            [&](const double* t) {
+    if (!Y.template reduce<2>(rr_p, rzn_p, S_RR, [&](const double* t) {
                               mixed_check(S, t[0]);
                               mixed_rz<false>(S, (float)t[1], !S.update);
                             }))
@@ -209,7 +201,7 @@ __global__ void __launch_bounds__(PCG_THREADS, 4) pcg_reliable_kernel(ReliableAr
         P.x[i] += (double)P.x32[i];
         P.x32[i] = 0.f;
       }
-      if (!grid_sync(P.bar, P.st, P.limit_ns)) return;
+      if (!Y.sync()) return;
       double rr64_p = 0.0;
       float rz_new_p = 0.f;
       {
@@ -228,9 +220,7 @@ __global__ void __launch_bounds__(PCG_THREADS, 4) pcg_reliable_kernel(ReliableAr
           }
         }
       }
-      block_partials<double>(rr64_p, (double)rz_new_p, 2, P.partials, S_RR, S_RZ);
-      if (!group_reduce_apply(P.bar, P.st, P.limit_ns, P.partials, P.totals, S_RR, 2, gridDim.x,
-                              [&](const double* t) {
+      if (!Y.template reduce<2>(rr64_p, (double)rz_new_p, S_RR, [&](const double* t) {
                                 mixed_replaced(S, t[0], P.tol, P.delta);
                                 mixed_rz<false>(S, (float)t[1], true);
                               }))
@@ -240,7 +230,7 @@ __global__ void __launch_bounds__(PCG_THREADS, 4) pcg_reliable_kernel(ReliableAr
     }
     const float beta = S.beta;
     for (int i = tid; i < n; i += nth) P.p32[i] = fmaf(beta, P.p32[i], P.r32[i] * P.dinv32[i]);
-    if (!grid_sync(P.bar, P.st, P.limit_ns)) return;
+    if (!Y.sync()) return;
   }
   if (blockIdx.x == 0 && threadIdx.x == 0) cg_out(S, S.residual, P.out, P.tol, iters, updates);
 }
@@ -267,7 +257,7 @@ residual_kernel(int n, const int* rowptr, const int* col, const double* val, con
       rr = fma(ri, ri, rr);
     }
   }
-  block_partials<double>(rr, 0.0, 1, partials, 0, 0);
+  block_partial(rr, partials);
 }
 
 // y = K x, standalone (the matrix product of Csr::matvec, linalg.rs:41-50)
@@ -343,9 +333,10 @@ __global__ void k_reconstruct(int64_t ndof, const int32_t* ind_of, const double*
 // Lanes per CSR row.  FP64 work is scarce on GB300 (about 1/75 of the FP32
 // rate), so the FP64 SpMV uses few lanes per row (fewer shuffle-add steps per
 // row); the FP32 SpMV can afford wider groups for better coalescing.
-// Measured, FP64 CG of C3D8 blocks, us per iteration with 4 / 8 lanes: 6 k rows
-// 19.0 / 17.8, 17 k 19.9 / 21.1, 71 k 32.8 / 35.1, 104 k 41.1 / 45.0, 670 k
-// 154 / 176, 2.2 M 570 / 532 (there the wider loads stream better).
+// Measured, FP64 CG of C3D8 blocks, us per iteration with 4 / 8 lanes: 300 rows
+// 9.5 / 8.4, 1.5 k 10.3 / 11.1, 3.6 k 14.2 / 15.8, 17 k 19.9 / 21.1, 71 k 32.8 /
+// 35.1, 104 k 41.1 / 45.0, 670 k 154 / 176, 2.2 M 570 / 532 (there the wider
+// loads stream better).
 static int pick_lanes(double avg_row, bool fp32, int64_t rows) {
   if (fp32) {
     if (avg_row <= 12) return 4;
@@ -353,7 +344,7 @@ static int pick_lanes(double avg_row, bool fp32, int64_t rows) {
     return 16;
   }
   if (avg_row <= 24) return 4;
-  if (avg_row <= 160) return rows >= 8000 && rows < 1500000 ? 4 : 8;
+  if (avg_row <= 160) return rows >= 1000 && rows < 1500000 ? 4 : 8;
   return 16;
 }
 
@@ -368,8 +359,13 @@ template <typename V, int L>
 static int launch_pcg_t(axia_ctx* ctx, PcgArgs<V>& P) {
   auto kern = pcg_kernel<V, L>;
   int grid = 0;
-  AXIA_TRY(coop_grid(ctx, (const void*)kern, (int64_t)P.n * L, &grid));
   void* params[] = {&P};
+  if constexpr (sizeof(V) == sizeof(double) && (L == 4 || L == 8)) {
+    const void* one = (const void*)pcg_kernel<V, L, true>;
+    const int blocks = ctx->nnz <= CLUSTER_MAX_NNZ ? cluster_blocks(one, (int64_t)P.n * L) : 0;
+    if (blocks) return launch_cluster(ctx, one, blocks, params);
+  }
+  AXIA_TRY(coop_grid(ctx, (const void*)kern, (int64_t)P.n * L, &grid));
   AXIA_CUDA(ctx, cudaLaunchCooperativeKernel((const void*)kern, dim3(grid), dim3(PCG_THREADS), params, 0, ctx->stream));
   ctx->launches++;
   return AXIA_OK;

@@ -7,7 +7,7 @@
 
 constexpr int PCG_THREADS = 512;
 int pcg_lanes_for(const axia_ctx* ctx, bool fp32, int requested);
-constexpr int S_PQ = 0, S_RR = 1, S_RZ = 2, N_SLOTS = 3;
+constexpr int S_PQ = 0, S_RR = 1, N_SLOTS = 3;  // partial-sum slots: p.q; r.r, r.z
 
 // result of one persistent solve, written by block 0
 struct PcgOut {
@@ -47,43 +47,43 @@ __device__ __forceinline__ T group_sum(T v) {
   return v;
 }
 
-// block-reduce up to two values and store them as this block's partials
-// (block `rank` of a group of nblk blocks; the whole grid by default).
+// Block-reduce up to two values; the sums are valid on warp 0.
 // FP64 values go through shared memory: a warp sum costs every warp five
 // dependent FP64 additions per value, and GB300 issues one FP64 warp
 // instruction per SM about every 18 cycles, so 16 warps and two values take
 // 1.5 us per block; four warps per value adding up a quarter of the warps'
 // lanes each, then one warp, need 8 + 3 + 5 instead of 160 of them.
-template <typename A>
-__device__ __forceinline__ void block_partials(A v0, A v1, int nv, double* partials, int slot0, int slot1,
-                                               unsigned nblk = 0, unsigned rank = 0) {
+template <int NV, typename A>
+__device__ __forceinline__ void block_sums(A v0, A v1, double (&out)[2]) {
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nw = blockDim.x >> 5;
-  if (nblk == 0) {
-    nblk = gridDim.x;
-    rank = blockIdx.x;
-  }
+  out[0] = out[1] = 0.0;
   if constexpr (sizeof(A) == sizeof(double)) {
     constexpr int Q = 4;
-    __shared__ A s_all[2][PCG_THREADS];
-    __shared__ A s_part[2][Q][32];
+    __shared__ A s_all[NV][PCG_THREADS];
+    __shared__ A s_part[NV][Q][32];
     s_all[0][threadIdx.x] = v0;
-    if (nv > 1) s_all[1][threadIdx.x] = v1;
+    if (NV > 1) s_all[NV - 1][threadIdx.x] = v1;
     __syncthreads();
-    for (int t = warp; t < Q * nv; t += nw) {
+    for (int t = warp; t < Q * NV; t += nw) {
       const int k = t / Q, g = t % Q;
       A a = A(0);
       for (int w = g; w < nw; w += Q) a += s_all[k][32 * w + lane];
       s_part[k][g][lane] = a;
     }
     __syncthreads();
-    for (int k = warp; k < nv; k += nw) {
-      const A a = warp_sum((s_part[k][0][lane] + s_part[k][1][lane]) + (s_part[k][2][lane] + s_part[k][3][lane]));
-      if (lane == 0) partials[(k == 0 ? slot0 : slot1) * nblk + rank] = a;
+    if (warp == 0) {
+#pragma unroll
+      for (int k = 0; k < NV; ++k)
+        out[k] = (s_part[k][0][lane] + s_part[k][1][lane]) + (s_part[k][2][lane] + s_part[k][3][lane]);
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1)
+#pragma unroll
+        for (int k = 0; k < NV; ++k) out[k] += __shfl_xor_sync(0xffffffffu, out[k], o);
     }
   } else {
     __shared__ A s_red[2][32];
     v0 = warp_sum(v0);
-    if (nv > 1) v1 = warp_sum(v1);
+    if (NV > 1) v1 = warp_sum(v1);
     if (lane == 0) {
       s_red[0][warp] = v0;
       s_red[1][warp] = v1;
@@ -93,14 +93,105 @@ __device__ __forceinline__ void block_partials(A v0, A v1, int nv, double* parti
       A a0 = lane < nw ? s_red[0][lane] : A(0);
       A a1 = lane < nw ? s_red[1][lane] : A(0);
       a0 = warp_sum(a0);
-      if (nv > 1) a1 = warp_sum(a1);
-      if (lane == 0) {
-        partials[slot0 * nblk + rank] = (double)a0;
-        if (nv > 1) partials[slot1 * nblk + rank] = (double)a1;
-      }
+      if (NV > 1) a1 = warp_sum(a1);
+      out[0] = (double)a0;
+      out[1] = (double)a1;
     }
   }
 }
+
+// a value's block sum as this block's partial
+__device__ __forceinline__ void block_partial(double v, double* partials) {
+  double t[2];
+  block_sums<1>(v, 0.0, t);
+  if (threadIdx.x == 0) partials[blockIdx.x] = t[0];
+}
+
+// Barriers and reductions over the co-resident blocks of one system: block
+// `rank` of nblk.  reduce() adds up one or two values over all threads and runs
+// fn(totals) on thread 0 of every block (the scalars of the iteration, left in
+// shared memory).  Every block sees the same totals.
+//
+// CLUSTER: the blocks are one thread-block cluster (at most CLUSTER_MAX): the
+// block sums go to every block's shared memory and the cluster's hardware
+// barrier replaces the counter in L2.  A small system is all barriers: at 1,500
+// rows in FP64 the three of an iteration took 12 of its 17.5 us.
+constexpr int CLUSTER_MAX = 16;
+// Systems up to these sizes run as one cluster: 16 SMs against all of them,
+// cheap barriers against work.  Measured, us per iteration, cluster / whole
+// grid: FP64 CSR 88 k entries 10.3 / 18.1, 240 k 14.2 / 18.0, 430 k 17.6 / 18.1,
+// 690 k 25.2 / 19.3; FP32 node blocks with the two-level preconditioner 14 k
+// blocks 12.5 / 25.0, 52 k 14.9 / 24.3, 120 k 20.4 / 24.9, 230 k 31.0 / 24.7.
+constexpr int64_t CLUSTER_MAX_NNZ = 400000;
+constexpr int64_t CLUSTER_MAX_BLOCKS = 130000;
+
+template <bool CLUSTER>
+struct BlockSync {
+  GridBarrier* bar;
+  DevStatus* st;
+  unsigned long long limit_ns;
+  double* partials;  // [3][nblk]
+  double* totals;    // [3]
+  unsigned nblk, rank;
+  int parity;
+
+  template <int NV, typename A, typename F>
+  __device__ __forceinline__ bool reduce(A v0, A v1, int slot0, F&& fn) {
+    double t[2];
+    block_sums<NV>(v0, v1, t);
+    if constexpr (CLUSTER) {
+      // two sets in turn: a block writes set k again only after a barrier that
+      // every block reached after reading it
+      double (*slots)[2][CLUSTER_MAX] = cluster_slots();
+      parity ^= 1;
+      if (threadIdx.x < nblk) {
+#pragma unroll
+        for (int k = 0; k < NV; ++k) {
+          const unsigned mine = (unsigned)__cvta_generic_to_shared(&slots[parity][k][rank]);
+          unsigned theirs;
+          asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(theirs) : "r"(mine), "r"(threadIdx.x));
+          asm volatile("st.shared::cluster.f64 [%0], %1;" ::"r"(theirs), "d"(t[k]) : "memory");
+        }
+      }
+      sync();
+      if (threadIdx.x < 32) {
+        double a[2];
+#pragma unroll
+        for (int k = 0; k < NV; ++k) a[k] = threadIdx.x < nblk ? slots[parity][k][threadIdx.x] : 0.0;
+#pragma unroll
+        for (int o = CLUSTER_MAX / 2; o > 0; o >>= 1)
+#pragma unroll
+          for (int k = 0; k < NV; ++k) a[k] += __shfl_xor_sync(0xffffffffu, a[k], o);
+        if (threadIdx.x == 0) fn(a);
+      }
+      __syncthreads();
+      return true;
+    } else {
+      if (threadIdx.x == 0) {
+#pragma unroll
+        for (int k = 0; k < NV; ++k) partials[(slot0 + k) * nblk + rank] = t[k];
+      }
+      return group_reduce_apply(bar, st, limit_ns, partials, totals, slot0, NV, nblk, fn);
+    }
+  }
+  __device__ __forceinline__ bool sync() {
+    if constexpr (CLUSTER) {
+      asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+      return true;
+    } else {
+      return group_sync(bar, st, limit_ns, nblk);
+    }
+  }
+  // before the first reduce() / after the last: no block writes to another's
+  // shared memory before it runs or after it has left
+  __device__ __forceinline__ void fence_lifetime() {
+    if constexpr (CLUSTER) sync();
+  }
+  static __device__ __forceinline__ double (*cluster_slots())[2][CLUSTER_MAX] {
+    __shared__ double s_slots[2][2][CLUSTER_MAX];
+    return s_slots;
+  }
+};
 
 // What one iteration of a persistent CG needs from its reductions, computed
 // by thread 0 of each block and read by the block from shared memory.
@@ -230,11 +321,10 @@ struct MeshGroup {
   int col0, ldm;      // its block of the coarse inverse: first unknown, padded size
   long long moff;     // element offset of that block
 };
-constexpr int GROUP_SLOTS = 4;  // partial-sum slots per group: S_PQ, S_RR, S_RZ, S_RC
+constexpr int GROUP_SLOTS = N_SLOTS;  // partial-sum slots per group
 
 constexpr int COARSE_MAX = 4096;    // coarse unknowns (6 per subdomain, padded to 64)
 constexpr int COARSE_CHUNK = 256;   // nodes per restriction chunk at most
-constexpr int S_RC = 3;             // partial-sum slot of r_c . y
 
 struct CoarseArgs {
   int n_sub;             // subdomains (0: no coarse space)
@@ -354,6 +444,47 @@ inline int coop_grid(axia_ctx* ctx, const void* kern, int64_t work, int* grid_ou
   return AXIA_OK;
 }
 
+
+// Blocks of the one-cluster form of a CG launch for `work` threads of one
+// matrix product (0: use the cooperative launch, e.g. where the device cannot
+// hold such a cluster).  kern is the CLUSTER instantiation.
+inline int cluster_blocks(const void* kern, int64_t work) {
+  const int64_t need = std::max<int64_t>(1, (work + PCG_THREADS - 1) / PCG_THREADS);
+  int blocks = 1;
+  while (blocks < need && blocks < CLUSTER_MAX) blocks *= 2;
+  if (blocks > 8 && cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess)
+    blocks = 8;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(blocks);
+  cfg.blockDim = dim3(PCG_THREADS);
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = blocks;
+  attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  int fit = 0;
+  if (cudaOccupancyMaxActiveClusters(&fit, kern, &cfg) != cudaSuccess || fit < 1) {
+    (void)cudaGetLastError();
+    return 0;
+  }
+  return blocks;
+}
+inline int launch_cluster(axia_ctx* ctx, const void* kern, int blocks, void** params) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(blocks);
+  cfg.blockDim = dim3(PCG_THREADS);
+  cfg.stream = ctx->stream;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = blocks;
+  attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  AXIA_CUDA(ctx, cudaLaunchKernelExC(&cfg, kern, params));
+  ctx->launches++;
+  return AXIA_OK;
+}
 
 // one persistent launch bracketed by CUDA events on the launching stream
 template <typename F>
