@@ -224,7 +224,7 @@ struct BsrPcgArgs {
 
 // Jacobi PCG on the node-block form (same recurrence as pcg_kernel).
 template <typename V, int L>
-__global__ void __launch_bounds__(PCG_THREADS) pcg_bsr_kernel(BsrPcgArgs<V> P) {
+__global__ void __launch_bounds__(PCG_THREADS, 2) pcg_bsr_kernel(BsrPcgArgs<V> P) {
   using A = V;
   const int nd = P.nd, n_nodes = P.M.n_nodes;
   const int tid = blockIdx.x * blockDim.x + threadIdx.x, nth = gridDim.x * blockDim.x;
@@ -304,8 +304,8 @@ struct SolveRange {
 // The coarse solve of the two-level preconditioner, r_c complete:
 // y = M r_c, and r_c . y reduced over the group; the direction's beta (or, for
 // the first direction, the coarse part of r.z) follows on thread 0.
-template <bool CLUSTER>
-__device__ __forceinline__ bool coarse_step(const CoarseArgs& C, BlockSync<CLUSTER>& Y, int gwarp, int nwarps, int lane,
+template <typename SYNC>
+__device__ __forceinline__ bool coarse_step(const CoarseArgs& C, SYNC& Y, int gwarp, int nwarps, int lane,
                                             CgScalars<float>& S, bool first) {
   __shared__ __align__(16) float s_rc[COARSE_MAX];
   const float acc = coarse_solve(C, s_rc, gwarp, nwarps, lane);
@@ -346,9 +346,9 @@ __device__ __forceinline__ void reliable_body(const BsrReliableArgs& P, const Co
     bb_p = fma(bi, bi, bb_p);
   }
   __shared__ CgScalars<float> S;
-  BlockSync<CLUSTER> Y{R.bar, P.st, P.limit_ns, R.partials, R.totals, R.nblk, R.rank, 0};
+  BlockSync<CLUSTER, !COARSE && !CLUSTER> Y{R.bar, P.st, P.limit_ns, R.partials, R.totals, R.nblk, R.rank, 0};
   Y.fence_lifetime();
-  if (!Y.template reduce<2>(bb_p, (double)rz_p, S_RR, [&](const double* t) { mixed_begin(S, t, P.tol, P.delta); }))
+  if (!Y.template reduce<2, true>(bb_p, (double)rz_p, S_RR, [&](const double* t) { mixed_begin(S, t, P.tol, P.delta); }))
     return;
   long long iters = 0;
   int updates = 0;
@@ -439,7 +439,7 @@ __device__ __forceinline__ void reliable_body(const BsrReliableArgs& P, const Co
           }
         }
       }
-      if (!Y.template reduce<2>(rr64_p, (double)rz_new_p, S_RR, [&](const double* t) {
+      if (!Y.template reduce<2, true>(rr64_p, (double)rz_new_p, S_RR, [&](const double* t) {
             mixed_replaced(S, t[0], P.tol, P.delta);
             mixed_rz<COARSE>(S, (float)t[1], true);
           }))

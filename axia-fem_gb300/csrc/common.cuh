@@ -177,10 +177,8 @@ __device__ __forceinline__ bool grid_sync(GridBarrier* bar, DevStatus* st, unsig
 // Likewise only the warps that hold partials join the sums.
 constexpr int REDUCE_MAX_NV = 2;
 
-// The last block's part of group_reduce_sync (every thread of the block calls
-// it).  Not inlined: its registers stay out of the allocation of the CG loops
-// that call the barrier.
-static __device__ __noinline__ void reduce_partials_last_block(const double* partials, double* totals, double* s_tot,
+// The last block's part of group_reduce_apply (every thread of the block calls it).
+__device__ __forceinline__ void reduce_partials_last_block(const double* partials, double* totals, double* s_tot,
                                                         int slot0, int nv, unsigned nblk) {
   __shared__ double s_sum[REDUCE_MAX_NV][32];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nw = blockDim.x >> 5;
@@ -222,7 +220,14 @@ static __device__ __noinline__ void reduce_partials_last_block(const double* par
   }
 }
 
-template <typename F>
+// The same out of line.  Which of the two gives a CG loop the better register
+// allocation is measured per kernel (BlockSync).
+static __device__ __noinline__ void reduce_partials_outlined(const double* partials, double* totals, double* s_tot,
+                                                            int slot0, int nv, unsigned nblk) {
+  reduce_partials_last_block(partials, totals, s_tot, slot0, nv, nblk);
+}
+
+template <bool OUTLINED = false, typename F>
 __device__ __forceinline__ bool group_reduce_apply(GridBarrier* bar, DevStatus* st, unsigned long long limit_ns,
                                                    const double* partials, double* totals, int slot0, int nv,
                                                    unsigned nblk, F&& fn) {
@@ -236,7 +241,12 @@ __device__ __forceinline__ bool group_reduce_apply(GridBarrier* bar, DevStatus* 
     s_last = last;
   }
   __syncthreads();
-  if (s_last) reduce_partials_last_block(partials, totals, s_tot, slot0, nv, nblk);
+  if (s_last) {
+    if constexpr (OUTLINED)
+      reduce_partials_outlined(partials, totals, s_tot, slot0, nv, nblk);
+    else
+      reduce_partials_last_block(partials, totals, s_tot, slot0, nv, nblk);
+  }
   if (threadIdx.x == 0) {
     int ok = 1;
     if (s_last) {

@@ -41,7 +41,7 @@ __device__ __forceinline__ A csr_row_dot(int row, int n, int sl, const int* __re
 }
 
 template <typename V, int L, bool CLUSTER = false>
-__global__ void __launch_bounds__(PCG_THREADS) pcg_kernel(PcgArgs<V> P) {
+__global__ void __launch_bounds__(PCG_THREADS, CLUSTER ? 1 : 3) pcg_kernel(PcgArgs<V> P) {
   using A = V;  // accumulation in the storage precision (FP64 or FP32)
   const int n = P.n;
   const int tid = blockIdx.x * blockDim.x + threadIdx.x;
@@ -157,7 +157,7 @@ __global__ void __launch_bounds__(PCG_THREADS, 4) pcg_reliable_kernel(ReliableAr
   }
   __shared__ CgScalars<float> S;
   BlockSync<false> Y{P.bar, P.st, P.limit_ns, P.partials, P.totals, gridDim.x, blockIdx.x, 0};
-  if (!Y.template reduce<2>(bb_p, (double)rz_p, S_RR, [&](const double* t) { mixed_begin(S, t, P.tol, P.delta); }))
+  if (!Y.template reduce<2, true>(bb_p, (double)rz_p, S_RR, [&](const double* t) { mixed_begin(S, t, P.tol, P.delta); }))
     return;
   long long iters = 0;
   int updates = 0;
@@ -220,7 +220,7 @@ __global__ void __launch_bounds__(PCG_THREADS, 4) pcg_reliable_kernel(ReliableAr
           }
         }
       }
-      if (!Y.template reduce<2>(rr64_p, (double)rz_new_p, S_RR, [&](const double* t) {
+      if (!Y.template reduce<2, true>(rr64_p, (double)rz_new_p, S_RR, [&](const double* t) {
                                 mixed_replaced(S, t[0], P.tol, P.delta);
                                 mixed_rz<false>(S, (float)t[1], true);
                               }))

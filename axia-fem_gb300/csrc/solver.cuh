@@ -47,22 +47,32 @@ __device__ __forceinline__ T group_sum(T v) {
   return v;
 }
 
-// Block-reduce up to two values; the sums are valid on warp 0.
+// Block-reduce up to two values: emit(k, sum) runs on one warp per value (all
+// its lanes hold the sum).
 // FP64 values go through shared memory: a warp sum costs every warp five
 // dependent FP64 additions per value, and GB300 issues one FP64 warp
 // instruction per SM about every 18 cycles, so 16 warps and two values take
 // 1.5 us per block; four warps per value adding up a quarter of the warps'
-// lanes each, then one warp, need 8 + 3 + 5 instead of 160 of them.
-template <int NV, typename A>
-__device__ __forceinline__ void block_sums(A v0, A v1, double (&out)[2]) {
+// lanes each, then one warp, need 8 + 3 + 5 instead of 160 of them.  RARE: warp
+// sums all the same, for the FP64 sums of a mixed solve (a few in all), where
+// 10 KB of shared memory would cost the matrix product L1.
+struct SumsScratch {
+  double all[2][PCG_THREADS];
+  double part[2][4][32];
+};
+__device__ __forceinline__ SumsScratch& sums_scratch() {  // one for every instantiation
+  __shared__ SumsScratch s;
+  return s;
+}
+template <int NV, bool RARE, typename A, typename E>
+__device__ __forceinline__ void block_sums(A v0, A v1, E&& emit) {
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nw = blockDim.x >> 5;
-  out[0] = out[1] = 0.0;
-  if constexpr (sizeof(A) == sizeof(double)) {
+  if constexpr (sizeof(A) == sizeof(double) && !RARE) {
     constexpr int Q = 4;
-    __shared__ A s_all[NV][PCG_THREADS];
-    __shared__ A s_part[NV][Q][32];
+    auto& s_all = sums_scratch().all;
+    auto& s_part = sums_scratch().part;
     s_all[0][threadIdx.x] = v0;
-    if (NV > 1) s_all[NV - 1][threadIdx.x] = v1;
+    if (NV > 1) s_all[1][threadIdx.x] = v1;
     __syncthreads();
     for (int t = warp; t < Q * NV; t += nw) {
       const int k = t / Q, g = t % Q;
@@ -71,15 +81,9 @@ __device__ __forceinline__ void block_sums(A v0, A v1, double (&out)[2]) {
       s_part[k][g][lane] = a;
     }
     __syncthreads();
-    if (warp == 0) {
-#pragma unroll
-      for (int k = 0; k < NV; ++k)
-        out[k] = (s_part[k][0][lane] + s_part[k][1][lane]) + (s_part[k][2][lane] + s_part[k][3][lane]);
-#pragma unroll
-      for (int o = 16; o > 0; o >>= 1)
-#pragma unroll
-        for (int k = 0; k < NV; ++k) out[k] += __shfl_xor_sync(0xffffffffu, out[k], o);
-    }
+    if (warp < NV)
+      emit(warp, warp_sum((s_part[warp][0][lane] + s_part[warp][1][lane]) +
+                          (s_part[warp][2][lane] + s_part[warp][3][lane])));
   } else {
     __shared__ A s_red[2][32];
     v0 = warp_sum(v0);
@@ -92,19 +96,17 @@ __device__ __forceinline__ void block_sums(A v0, A v1, double (&out)[2]) {
     if (warp == 0) {
       A a0 = lane < nw ? s_red[0][lane] : A(0);
       A a1 = lane < nw ? s_red[1][lane] : A(0);
-      a0 = warp_sum(a0);
-      if (NV > 1) a1 = warp_sum(a1);
-      out[0] = (double)a0;
-      out[1] = (double)a1;
+      emit(0, (double)warp_sum(a0));
+      if (NV > 1) emit(1, (double)warp_sum(a1));
     }
   }
 }
 
 // a value's block sum as this block's partial
 __device__ __forceinline__ void block_partial(double v, double* partials) {
-  double t[2];
-  block_sums<1>(v, 0.0, t);
-  if (threadIdx.x == 0) partials[blockIdx.x] = t[0];
+  block_sums<1, true>(v, 0.0, [&](int, double t) {
+    if (threadIdx.x == 0) partials[blockIdx.x] = t;
+  });
 }
 
 // Barriers and reductions over the co-resident blocks of one system: block
@@ -125,7 +127,10 @@ constexpr int CLUSTER_MAX = 16;
 constexpr int64_t CLUSTER_MAX_NNZ = 400000;
 constexpr int64_t CLUSTER_MAX_BLOCKS = 130000;
 
-template <bool CLUSTER>
+// OUTLINED: the last block's sums in a function of their own.  Measured at C3D8
+// 90^3 / 100^3: mixed node blocks with the diagonal 167 us per iteration inline,
+// 152 outlined; two-level 53.8 ms against 54.2, 64 cubes 68.4 against 71.4.
+template <bool CLUSTER, bool OUTLINED = false>
 struct BlockSync {
   GridBarrier* bar;
   DevStatus* st;
@@ -135,24 +140,22 @@ struct BlockSync {
   unsigned nblk, rank;
   int parity;
 
-  template <int NV, typename A, typename F>
+  template <int NV, bool RARE = false, typename A, typename F>
   __device__ __forceinline__ bool reduce(A v0, A v1, int slot0, F&& fn) {
-    double t[2];
-    block_sums<NV>(v0, v1, t);
     if constexpr (CLUSTER) {
       // two sets in turn: a block writes set k again only after a barrier that
       // every block reached after reading it
       double (*slots)[2][CLUSTER_MAX] = cluster_slots();
       parity ^= 1;
-      if (threadIdx.x < nblk) {
-#pragma unroll
-        for (int k = 0; k < NV; ++k) {
+      block_sums<NV, RARE>(v0, v1, [&](int k, double t) {
+        const unsigned lane = threadIdx.x & 31;
+        if (lane < nblk) {
           const unsigned mine = (unsigned)__cvta_generic_to_shared(&slots[parity][k][rank]);
           unsigned theirs;
-          asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(theirs) : "r"(mine), "r"(threadIdx.x));
-          asm volatile("st.shared::cluster.f64 [%0], %1;" ::"r"(theirs), "d"(t[k]) : "memory");
+          asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(theirs) : "r"(mine), "r"(lane));
+          asm volatile("st.shared::cluster.f64 [%0], %1;" ::"r"(theirs), "d"(t) : "memory");
         }
-      }
+      });
       sync();
       if (threadIdx.x < 32) {
         double a[2];
@@ -167,11 +170,10 @@ struct BlockSync {
       __syncthreads();
       return true;
     } else {
-      if (threadIdx.x == 0) {
-#pragma unroll
-        for (int k = 0; k < NV; ++k) partials[(slot0 + k) * nblk + rank] = t[k];
-      }
-      return group_reduce_apply(bar, st, limit_ns, partials, totals, slot0, NV, nblk, fn);
+      block_sums<NV, RARE>(v0, v1, [&](int k, double t) {
+        if ((threadIdx.x & 31) == 0) partials[(slot0 + k) * nblk + rank] = t;
+      });
+      return group_reduce_apply<OUTLINED>(bar, st, limit_ns, partials, totals, slot0, NV, nblk, fn);
     }
   }
   __device__ __forceinline__ bool sync() {
@@ -427,7 +429,8 @@ int reconstruct_system(axia_ctx* ctx, const ReducedSystem& S, const double* d_x,
 // Blocks of a cooperative CG launch for `work` threads of one matrix product
 // (rows x lanes per row): one block per PCG_THREADS up to one per SM, then a
 // multiple of the SM count (a part-filled last round left SMs with twice the
-// work of others), another per SM for about 1.5 PCG_THREADS of work each.
+// work of others): a second block per SM from 2.25 blocks of work per SM, as
+// many as fit from 12.
 // Measured, us per iteration of the FP64 CSR form with 4 lanes: 17 k rows 152
 // blocks 19.9, 304 23.4; 71 k 37.6, 304 32.8, 456 38.2; 104 k 51.7, 41.8, 41.1;
 // 670 k 247, 164, 154.
@@ -437,7 +440,7 @@ inline int coop_grid(axia_ctx* ctx, const void* kern, int64_t work, int* grid_ou
   if (per_sm < 1) return set_error(ctx, AXIA_ERR_CUDA, "PCG kernel does not fit on an SM");
   const int64_t need = std::max<int64_t>(1, (work + PCG_THREADS - 1) / PCG_THREADS);
   const int sms = ctx->sm_count;
-  const int rounds = (int)std::min<int64_t>(per_sm, std::max<int64_t>(1, (2 * need + 3 * sms / 2) / (3 * sms)));
+  const int rounds = need >= 12 * sms ? per_sm : std::min(per_sm, need >= 9 * sms / 4 ? 2 : 1);
   const int grid = (int)std::min<int64_t>(need, (int64_t)rounds * sms);
   if ((size_t)grid * N_SLOTS > ctx->partial_slots) return set_error(ctx, AXIA_ERR_STATE, "partials buffer too small");
   *grid_out = grid;
