@@ -546,6 +546,9 @@ __global__ void __launch_bounds__(PCG_THREADS) bsr_residual_kernel(BsrMat<double
 // ---------------------------------------------------------------------------
 // Lanes per block row and blocks per lane load.  FP32: 4 blocks per load;
 // lanes so that a row of the mesh's mean length takes one or two steps.
+// Measured, two-level CG kernel with 8 / 16 lanes: C3D20 50^3 (56 blocks per row)
+// 85.1 / 71.0 ms, 30^3 15.6 / 14.5; C3D10 28^3 (27) 14.3 / 15.1; C3D8 100^3 (28)
+// 42.3 / 52.1.
 // FP64: 2 blocks per load.  Requests outside the instantiated set fall back
 // to the automatic choice.
 struct RowLayout {
@@ -559,8 +562,7 @@ static RowLayout bsr_layout(const axia_ctx* ctx, bool fp32, int lanes_req, int v
   const double steps = avg / r.vec;  // vector steps per row
   const int auto_l = steps <= 3 ? 2 : (steps <= 6 ? 4 : (steps <= 12 ? 8 : 16));
   r.lanes = (lanes_req == 2 || lanes_req == 4 || lanes_req == 8 || lanes_req == 16) ? lanes_req : auto_l;
-  // instantiated: vec 4 with 2/4/8 lanes, vec 2 with 4/8, vec 1 with 4/8/16
-  if (r.vec == 4 && r.lanes == 16) r.lanes = 8;
+  // instantiated: vec 4 with 2/4/8/16 lanes, vec 2 with 4/8, vec 1 with 4/8/16
   if (r.vec == 2 && (r.lanes == 2 || r.lanes == 16)) r.lanes = r.lanes == 2 ? 4 : 8;
   if (r.vec == 1 && r.lanes == 2) r.lanes = 4;
   return r;
@@ -573,6 +575,7 @@ static int with_layout(RowLayout r, F&& f) {
   if (r.vec == 4) {
     if (r.lanes == 2) return f(integral_constant<int, 2>{}, integral_constant<int, 4>{});
     if (r.lanes == 4) return f(integral_constant<int, 4>{}, integral_constant<int, 4>{});
+    if (r.lanes == 16) return f(integral_constant<int, 16>{}, integral_constant<int, 4>{});
     return f(integral_constant<int, 8>{}, integral_constant<int, 4>{});
   }
   if (r.vec == 2) {
@@ -943,7 +946,7 @@ int bsr_autotune(axia_ctx* ctx, const char* cache_path, int* lanes_out, int* vec
   AXIA_TRY(dev_alloc(ctx, &d_ones, (size_t)ctx->ndof));
   k_fill_ones<<<ctx->sm_count * 4, 256, 0, ctx->stream>>>(ctx->ndof, d_ones);
   int st = launch_full_rhs(ctx, d_ones);
-  const RowLayout cands[] = {{8, 4}, {4, 4}, {2, 4}, {8, 2}, {4, 2}, {16, 1}, {8, 1}, {4, 1}};
+  const RowLayout cands[] = {{8, 4}, {16, 4}, {4, 4}, {2, 4}, {8, 2}, {4, 2}, {16, 1}, {8, 1}, {4, 1}};
   const long long iters = 40;
   double best = 1e300;
   RowLayout pick{0, 0};
