@@ -280,6 +280,9 @@ int ensure_tables(axia_ctx* ctx, int nn, int ng, ElemTables* out) {
   return AXIA_OK;
 }
 
+// Batches of at most this many C3D20(R) elements per SM take a team of warps each.
+constexpr int64_t PAIR_TEAM_MAX = 4;
+
 // DW: the double-word Gauss loop (element_dw.cuh) instead of the FP64 one
 template <int NN, int NG, int WARPS, bool DW = false>
 int launch_element_ke(axia_ctx* ctx, const ElemArgs& args) {
@@ -287,9 +290,18 @@ int launch_element_ke(axia_ctx* ctx, const ElemArgs& args) {
   AXIA_TRY(ensure_tables(ctx, NN, NG, &tab));
   size_t smem;
   void (*kern)(ElemArgs, ElemTables);
+  int64_t per_block = WARPS;  // elements per block and step
+  int threads = WARPS * 32;
   if constexpr (DW && NN == 20) {
     smem = element_dw_pair_smem_bytes<NN, NG>(WARPS);
     kern = element_ke_dw_pair_kernel<NN, NG, WARPS>;
+    if (args.n_elem <= PAIR_TEAM_MAX * ctx->sm_count) {
+      constexpr int TEAM = ElemDwPairTraits<NN, NG>::NR;
+      smem = element_dw_pair_smem_bytes<NN, NG>(1);
+      kern = element_ke_dw_pair_kernel<NN, NG, TEAM, TEAM>;
+      per_block = 1;
+      threads = TEAM * 32;
+    }
   } else if constexpr (DW) {
     smem = element_dw_smem_bytes<NN, NG>(WARPS);
     kern = element_ke_dw_kernel<NN, NG, WARPS>;
@@ -299,12 +311,12 @@ int launch_element_ke(axia_ctx* ctx, const ElemArgs& args) {
   }
   AXIA_CUDA(ctx, cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
   int per_sm = 0;
-  AXIA_CUDA(ctx, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, WARPS * 32, smem));
+  AXIA_CUDA(ctx, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, threads, smem));
   if (per_sm < 1) return set_error(ctx, AXIA_ERR_CUDA, "element kernel does not fit on an SM");
-  int64_t need = (args.n_elem + WARPS - 1) / WARPS;
+  int64_t need = (args.n_elem + per_block - 1) / per_block;
   int64_t grid = std::min<int64_t>(need, (int64_t)per_sm * ctx->sm_count);
   if (grid < 1) grid = 1;
-  kern<<<(unsigned)grid, WARPS * 32, smem, ctx->stream>>>(args, tab);
+  kern<<<(unsigned)grid, threads, smem, ctx->stream>>>(args, tab);
   ctx->launches++;
   AXIA_CUDA(ctx, cudaGetLastError());
   return AXIA_OK;

@@ -306,7 +306,11 @@ constexpr size_t element_dw_pair_smem_bytes(int warps) {
   return (size_t)(D::TAB + warps * D::WARP_UNITS) * sizeof(double);
 }
 
-template <int NN, int NG, int WARPS>
+// TEAM: warps that share one element (a block then has one team, WARPS ==
+// TEAM).  A few elements leave most SMs idle with a warp each, 102 us for 37
+// of them; the whole call from host arrays 178 us, 91 with the rounds of node
+// pairs over 7 warps (152 elements 264 and 173, 608 597 and 495).
+template <int NN, int NG, int WARPS, int TEAM = 1>
 __global__ void __launch_bounds__(WARPS * 32)
 element_ke_dw_pair_kernel(ElemArgs args, ElemTables tab) {
   using T = ElemTraits<NN, NG>;
@@ -316,7 +320,16 @@ element_ke_dw_pair_kernel(ElemArgs args, ElemTables tab) {
   dw* s_w = s_dnw + NG * NN * 3;            // [NG]
   dw* s_cm = s_w + NG;                      // [2]: c_lam, c_mu
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  double* W = smem + D::TAB + warp * D::WARP_UNITS;
+  static_assert(TEAM == 1 || TEAM == WARPS, "a block holds one team");
+  const int tw = TEAM > 1 ? warp : 0;  // warp of the team
+  const int tid = 32 * tw + lane;      // thread of the team
+  auto team_sync = [] {
+    if constexpr (TEAM > 1)
+      __syncthreads();
+    else
+      __syncwarp();
+  };
+  double* W = smem + D::TAB + (TEAM > 1 ? 0 : warp) * D::WARP_UNITS;
   dw* Xw = reinterpret_cast<dw*>(W + D::OFF_X);
   dw* G = reinterpret_cast<dw*>(W + D::OFF_G);
   dw* S = reinterpret_cast<dw*>(W + D::OFF_S);
@@ -330,9 +343,11 @@ element_ke_dw_pair_kernel(ElemArgs args, ElemTables tab) {
   }
   __syncthreads();
 
-  const int64_t warps_total = (int64_t)gridDim.x * WARPS;
-  for (int64_t e = (int64_t)blockIdx.x * WARPS + warp; e < args.n_elem; e += warps_total) {
-    // 1. coordinates relative to node 0; 2^k above the largest difference
+  const int64_t teams = (int64_t)gridDim.x * (WARPS / TEAM);
+  for (int64_t e = (int64_t)blockIdx.x * (WARPS / TEAM) + (TEAM > 1 ? 0 : warp); e < args.n_elem; e += teams) {
+    // 1. coordinates relative to node 0; 2^k above the largest difference (every
+    // warp of a team finds k, the first stores the coordinates)
+    if constexpr (TEAM > 1) __syncthreads();  // the previous element's c is read
     constexpr int PER = (T::NDOF + 31) / 32;
     double dif[PER];
     int emax = 0;
@@ -363,11 +378,11 @@ element_ke_dw_pair_kernel(ElemArgs args, ElemTables tab) {
 #pragma unroll
     for (int s = 0; s < PER; ++s) {
       const int t = lane + 32 * s;
-      if (t < T::NDOF) Xw[t] = dw_split_scaled(dif[s], k);
+      if (t < T::NDOF && tw == 0) Xw[t] = dw_split_scaled(dif[s], k);
     }
-    __syncwarp();  // also: the previous element's c / h (J's space) are read
+    team_sync();  // also: the previous element's c / h (J's space) are read
     // 2. J[g][q][p] = sum_a dN_a/dxi_p x_a,q (quadratic.rs:122-146 via elem.rs:175-181)
-    for (int t = lane; t < NG * 9; t += 32) {
+    for (int t = tid; t < NG * 9; t += 32 * TEAM) {
       const int g = t / 9, q = (t % 9) / 3, p = t % 3;
       const dw* dn = s_dnw + g * NN * 3;
       dw_acc s;
@@ -375,9 +390,9 @@ element_ke_dw_pair_kernel(ElemArgs args, ElemTables tab) {
       for (int a = 0; a < NN; ++a) dw_fma(s, dn[3 * a + p], Xw[3 * a + q]);
       J[t] = dw_value(s);
     }
-    __syncwarp();
+    team_sync();
     // 3. cofactor matrix b[i][j] (invert3 before the 1/det scaling, elem.rs:18-26)
-    for (int t = lane; t < NG * 9; t += 32) {
+    for (int t = tid; t < NG * 9; t += 32 * TEAM) {
       const int g = t / 9, i = (t % 9) / 3, j = t % 3;
       const dw* a = J + 9 * g;
       const int j1 = (j + 1) % 3, j2 = (j + 2) % 3, i1 = (i + 1) % 3, i2 = (i + 2) % 3;
@@ -386,9 +401,9 @@ element_ke_dw_pair_kernel(ElemArgs args, ElemTables tab) {
       dw_fma(s, dw_neg(a[3 * j1 + i2]), a[3 * j2 + i1]);
       G[t] = dw_value(s);
     }
-    __syncwarp();
+    team_sync();
     double vol_part = 0.0;
-    for (int g = lane; g < NG; g += 32) {
+    for (int g = tid; g < NG; g += 32 * TEAM) {
       const dw* a = J + 9 * g;
       const dw* b = G + 9 * g;
       dw_acc s;
@@ -413,15 +428,16 @@ element_ke_dw_pair_kernel(ElemArgs args, ElemTables tab) {
       vol_part += tab.w[g] * det;
     }
     if (!(__double_as_longlong(E) > 0 && __double_as_longlong(E) <= 0x7ff0000000000000ll)) {  // !(E > 0)
-      if (lane == 0) record_error(args.status, e, AXIA_ERR_MATERIAL);
+      if (tid == 0) record_error(args.status, e, AXIA_ERR_MATERIAL);
     }
-    if (args.vol_out) {
+    static_assert(NG <= 32, "the volume is one warp's sum");
+    if (args.vol_out && tw == 0) {
       vol_part = warp_sum(vol_part);
       if (lane == 0) args.vol_out[e] = vol_part;
     }
-    __syncwarp();  // J is read; c overwrites it
+    team_sync();  // J is read; c overwrites it
     // 4. c_a[i] = sum_p b[p][i] dN_a/dxi_p at every Gauss point
-    for (int t = lane; t < NG * T::NDOF; t += 32) {
+    for (int t = tid; t < NG * T::NDOF; t += 32 * TEAM) {
       const int g = t / T::NDOF, r = t % T::NDOF, a = r / 3, i = r % 3;
       const dw* b = G + 9 * g;
       const dw* dn = s_dnw + (g * NN + a) * 3;
@@ -441,12 +457,12 @@ element_ke_dw_pair_kernel(ElemArgs args, ElemTables tab) {
       lam = dw_from_double(E * args.c_lam * pow2(k));
       mu = dw_from_double(E * args.c_mu * pow2(k));
     }
-    __syncwarp();
+    team_sync();
     // 5. node pairs p = lane + 32 r, a <= b in row order of the upper triangle:
     // A_ab = sum_g h_a c_b^T
     double* const ke = args.ke_out + e * T::KE;
 #pragma unroll 1
-    for (int r = 0; r < D::NR; ++r) {
+    for (int r = tw; r < D::NR; r += TEAM) {
       const int p = lane + 32 * r;
       int a = 0, rem = p < T::NB ? p : 0;
       while (rem >= NN - a) {
