@@ -31,6 +31,7 @@
 #include <cmath>
 #include <vector>
 
+#include "hex8.cuh"
 #include "solver.cuh"
 
 int element_tables_for(axia_ctx* ctx, int nn, int ng, const double** dn, const double** w);
@@ -214,15 +215,12 @@ element_recover_kernel(int64_t n_elem, const int32_t* __restrict__ conn, const d
 }
 
 // C3D8 with 2 x 2 x 2 points: the same numbers from the element's trilinear
-// structure, x = sum c_ijk xi^i eta^j zeta^k.  FP64 instructions bound this
+// structure.  FP64 instructions bound this
 // kernel (one per SM about every 16 cycles): contracting eight nodes per point
 // took 498 FP64 instructions per warp of four elements, this form about 270
 // (with the nodal averages 6.8 -> 3.9 ms at 10^6 elements).
-//   * lane (element, field): the seven coefficients of a coordinate or
-//     displacement by a Hadamard transform (relative to node 0, which also
-//     keeps the element's distance from the origin out of the rounding), and
-//     its derivatives: along a direction they are the same at both points, so
-//     three times four values serve the eight points;
+//   * lane (element, field): the derivatives of a coordinate or displacement
+//     at the points (hex8.cuh);
 //   * lane (element, point): Jacobian, stress, cofactor rows times stress;
 //   * a node's force needs cofactor rows times sigma only summed over the two
 //     points along each direction;
@@ -250,8 +248,7 @@ element_recover_hex8_kernel(int64_t n_elem, const int32_t* __restrict__ conn, co
   double* A = s_a[warp];
   double* GP = s_gp[warp];
   const double lam1 = nu / ((1.0 + nu) * (1.0 - 2.0 * nu)), mu1 = 0.5 / (1.0 + nu);  // of E = 1
-  // point g = 4 [xi > 0] + 2 [eta > 0] + [zeta > 0]: its derivatives along xi, eta, zeta
-  const int gx = g & 3, gy = 4 + (g >> 2) * 2 + (g & 1), gz = 8 + (g >> 1);
+  const int gx = hex8_dxi(g), gy = hex8_deta(g), gz = hex8_dzeta(g);
   const int64_t step = (int64_t)gridDim.x * WARPS * EPW;
   for (int64_t e0 = ((int64_t)blockIdx.x * WARPS + warp) * EPW; e0 < n_elem; e0 += step) {
     // [element][field][node], fields x y z ux uy uz
@@ -268,38 +265,7 @@ element_recover_hex8_kernel(int64_t n_elem, const int32_t* __restrict__ conn, co
       A[k * 48 + (3 + c % 3) * 8 + c / 3] = uv;
     }
     __syncwarp();
-    if (g < 6) {
-      const double* v = A + le * 48 + g * 8;
-      const double v0 = v[0];
-      const double a1 = v[1] - v0, a2 = v[2] - v0, a3 = v[3] - v0, a4 = v[4] - v0, a5 = v[5] - v0, a6 = v[6] - v0,
-                   a7 = v[7] - v0;
-      // along xi: sums and differences of the edges (eta, zeta) = --, +-, -+, ++
-      const double p0 = a1, p1 = a2 + a3, p2 = a5 + a4, p3 = a6 + a7;
-      const double d0 = a1, d1 = a2 - a3, d2 = a5 - a4, d3 = a6 - a7;
-      const double pe0 = p1 - p0, pe1 = p3 - p2, ps0 = p1 + p0, ps1 = p3 + p2;  // along eta
-      const double de0 = d1 - d0, de1 = d3 - d2, ds0 = d1 + d0, ds1 = d3 + d2;
-      constexpr double G = 0.57735026918962576451;  // 1 / sqrt(3)
-      const double kx = 0.125 * (ds1 + ds0), ky = 0.125 * (pe1 + pe0), kz = 0.125 * (ps1 - ps0);
-      // xi eta, xi zeta, eta zeta at |.| = G, xi eta zeta at G^2
-      const double kxy = 0.125 * G * (de1 + de0), kxz = 0.125 * G * (ds1 - ds0), kyz = 0.125 * G * (pe1 - pe0),
-                   kxyz = (1.0 / 24.0) * (de1 - de0);
-      // d/dxi = kx + s2 kxy + s3 (kxz + s2 kxyz) and so on; signs (-, -) (-, +) (+, -) (+, +)
-      double* D = GP + (le * 6 + g) * 12;
-      const double xm = kx - kxy, xp = kx + kxy, xbm = kxz - kxyz, xbp = kxz + kxyz;
-      const double ym = ky - kxy, yp = ky + kxy, zm = kz - kxz, zp = kz + kxz, bm = kyz - kxyz, bp = kyz + kxyz;
-      D[0] = xm - xbm;
-      D[1] = xm + xbm;
-      D[2] = xp - xbp;
-      D[3] = xp + xbp;
-      D[4] = ym - bm;
-      D[5] = ym + bm;
-      D[6] = yp - bp;
-      D[7] = yp + bp;
-      D[8] = zm - bm;
-      D[9] = zm + bm;
-      D[10] = zp - bp;
-      D[11] = zp + bp;
-    }
+    if (g < 6) hex8_point_derivatives(A + le * 48 + g * 8, GP + (le * 6 + g) * 12);
     __syncwarp();
     const int64_t e = e0 + le;
     double J[3][3], Gu[3][3];
