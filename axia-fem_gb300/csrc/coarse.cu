@@ -21,9 +21,9 @@
 //   * a stable radix sort by key, then every run summed in item order gives
 //     S_IJ = Z_I^T K Z_J; A_IJ = T_I^T S_IJ T_J goes into a dense FP64 matrix;
 //   * A scaled to unit diagonal, rounded to FP32 and inverted in place by a
-//     symmetric blocked Gauss-Jordan elimination (64 x 64 tiles, one
-//     cooperative launch, three bounded grid barriers per tile step, the next
-//     pivot tile inverted during the current trailing update);
+//     symmetric blocked Gauss-Jordan elimination (64 x 64 tiles on and below
+//     the diagonal, one cooperative launch, two bounded grid barriers per tile
+//     step, the next pivot tile inverted during the current trailing update);
 //   * M = T diag(s) A^-1 diag(s) T^T per subdomain pair, in FP32.
 // Every sum has a fixed order: the same inputs give the same bits.
 #include <algorithm>
@@ -513,19 +513,30 @@ __global__ void k_scale_to_f32(const CoarseBlk* blk, const double* A, const doub
 
 // ---------------------------------------------------------------------------
 // Blocked Gauss-Jordan inverse of an SPD matrix (FP32, in place, no pivoting).
-// Step k with P = A_kk^-1 and the new row panel R_j = P A_kj (j != k):
-//   A_ij <- A_ij - A_ik R_j  (i, j != k),  A_kj <- R_j,  A_ik <- -R_i^T,  A_kk <- P.
+// Step k with P = A_kk^-1, the old row panel C_j = A_kj and the new one
+// R_j = P C_j (j != k):
+//   A_ij <- A_ij - A_ik R_j  (i, j != k),  A_kj <- R_j,  A_ik <- -A_ik P,  A_kk <- P.
 // With S_i = -1 for the block indices eliminated so far and +1 for the rest,
 // every intermediate satisfies A_ij = S_i S_j A_ji^T (the final inverse,
-// S = -1 throughout, is symmetric).  So the trailing update runs over the
-// tiles with j <= i and mirrors them with that sign, and the new column panel
-// is A_ik = -S_i R_i^T.
+// S = -1 throughout, is symmetric).  So only the tiles j <= i are kept:
+// C_j = A_jk^T for j > k, A_ik = S_i C_i^T and the new A_ik = -R_i^T (i > k).
+// C and R go to a panel buffer W; both operands of the trailing update are
+// then read along their rows, and nothing else is transposed or mirrored.
+// Two barriers per step: panels, then trailing tiles with the stores of R and P.
+// What bounds it: per step the trailing tiles' traffic (two operand tiles, the
+// tile in and out, 64 KB from and to L2 for 2 x 64^3 flops) and the latencies of
+// the panel, the look-ahead and the barriers.  3072 unknowns: 2.98 ms with
+// mirrored tiles, transposed operand loads, three barriers and the 64 pivots of
+// a tile unrolled in one warpgroup; 1.76 in this form, 1.52 with the next
+// tile's operands requested before the product.
 // ---------------------------------------------------------------------------
 constexpr int GJ_LD = GJ_T + 4;   // shared-memory row stride (16-byte aligned rows)
+constexpr int GJ_S = 16;          // pivots per step inside a tile
 
 struct GjArgs {
   float* A;
   int n;             // multiple of GJ_T
+  float* W;          // [2][GJ_T][n]: C, then R
   float* piv;        // [2][GJ_T][GJ_T] P of step k in buffer k & 1
   GridBarrier* bar;
   DevStatus* st;
@@ -533,10 +544,7 @@ struct GjArgs {
   int rank, nb;      // this block's rank in its group of nb blocks (at least 2)
 };
 
-// operand tiles: sa[q][r] = X[r][q] (transposed), sb[q][c] = Y[q][c]
-__device__ __forceinline__ void gj_load_t(float (*sa)[GJ_LD], const float* g, int ld) {
-  for (int t = threadIdx.x; t < GJ_T * GJ_T; t += blockDim.x) sa[t % GJ_T][t / GJ_T] = g[(size_t)(t / GJ_T) * ld + t % GJ_T];
-}
+// a tile's rows into shared memory
 __device__ __forceinline__ void gj_load(float (*sb)[GJ_LD], const float* g, int ld) {
   for (int t = threadIdx.x; t < GJ_T * GJ_T / 4; t += blockDim.x) {
     const int r = t / (GJ_T / 4), c = 4 * (t % (GJ_T / 4));
@@ -544,7 +552,7 @@ __device__ __forceinline__ void gj_load(float (*sb)[GJ_LD], const float* g, int 
   }
 }
 
-// out[4][4] = rows 4ty.. / cols 4tx.. of X Y
+// out[4][4] = rows 4ty.. / cols 4tx.. of sa^T sb
 __device__ __forceinline__ void gj_mul(float (*sa)[GJ_LD], float (*sb)[GJ_LD], float out[4][4]) {
   const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
 #pragma unroll
@@ -563,7 +571,7 @@ __device__ __forceinline__ void gj_mul(float (*sa)[GJ_LD], float (*sb)[GJ_LD], f
   }
 }
 
-// thread (ty, tx)'s 4 x 4 part of a tile into registers
+// thread (ty, tx)'s 4 x 4 part of a tile
 __device__ __forceinline__ void gj_load_regs(float (&a)[4][4], const float* g, int ld) {
   const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
 #pragma unroll
@@ -575,95 +583,6 @@ __device__ __forceinline__ void gj_load_regs(float (&a)[4][4], const float* g, i
     a[r][3] = v.w;
   }
 }
-
-// a dense 64 x 64 buffer into a tile of the matrix
-__device__ __forceinline__ void gj_store_global(const float* src, float* g, int ld) {
-  for (int t = threadIdx.x; t < GJ_T * GJ_T / 4; t += blockDim.x) {
-    const int r = t / (GJ_T / 4), c = 4 * (t % (GJ_T / 4));
-    *reinterpret_cast<float4*>(g + (size_t)r * ld + c) = *reinterpret_cast<const float4*>(src + (size_t)r * GJ_T + c);
-  }
-}
-
-// column panel of step k: tile (i, k) = -S_i tile (k, i)^T (i != k; S_i = -1 for i < k)
-__device__ __forceinline__ void gj_column_panel(const GjArgs& P, int k, int first, int stride) {
-  const int nt = P.n / GJ_T, ld = P.n;
-  for (int i = first; i < nt; i += stride) {
-    if (i == k) continue;
-    const float sg = i < k ? 1.f : -1.f;
-    const float* src = P.A + (size_t)k * GJ_T * ld + (size_t)i * GJ_T;
-    float* dst = P.A + (size_t)i * GJ_T * ld + (size_t)k * GJ_T;
-    for (int t = threadIdx.x; t < GJ_T * GJ_T; t += blockDim.x) {
-      const int r = t / GJ_T, c = t % GJ_T;  // coalesced reads of src row r
-      dst[(size_t)c * ld + r] = sg * src[(size_t)r * ld + c];
-    }
-  }
-}
-
-// Gauss-Jordan inverse of one 64 x 64 SPD tile, the register form: the
-// block's threads place their 4 x 4 parts in T (row stride GJ_LD); the 128
-// threads of warps 0..3 then take half a column each (column j = tid % 64,
-// rows 32 h .. 32 h + 31, h = tid / 64) into registers and run the 64 pivots
-// fully unrolled.  Pivot p needs column p, A_ip = S_i A_pi with S_i = -1 for
-// the pivots already taken (the sign structure of the symmetric elimination),
-// and row p sits in half p / 32: its 64 threads publish S_j A_pj to cpiv
-// (double-buffered) and a 128-thread named barrier per pivot.  Measured per
-// 64 x 64 tile at 3072 unknowns: 26 us, against 47 us for all 256 threads on
-// 4 x 4 parts with a block barrier per pivot and 33 us for the tile kept in
-// shared memory with a rolled pivot loop; the inversion runs beside the
-// trailing update of the step (34 us), so it is no longer the step's critical
-// path.  The inverse is written to the 64 x 64 buffer out (row-major).
-__device__ __forceinline__ void gj_invert_tile(const float (&a)[4][4], float* T, float* cpiv, float* out,
-                                               DevStatus* st, int base) {
-  const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
-#pragma unroll
-  for (int r = 0; r < 4; ++r)
-    *reinterpret_cast<float4*>(T + (4 * ty + r) * GJ_LD + 4 * tx) = make_float4(a[r][0], a[r][1], a[r][2], a[r][3]);
-  __syncthreads();
-  if (threadIdx.x < 2 * GJ_T) {
-    constexpr int HR = GJ_T / 2;  // rows per half
-    const int j = threadIdx.x % GJ_T, h = threadIdx.x / GJ_T;
-    float col[HR];
-#pragma unroll
-    for (int i = 0; i < HR; ++i) col[i] = T[(HR * h + i) * GJ_LD + j];
-#pragma unroll
-    for (int p = 0; p < GJ_T; ++p) {
-      float* cp = cpiv + (p & 1) * GJ_T;
-      const bool mine = (p / HR) == h;  // warp-uniform: row p is in this half
-      if (mine) cp[j] = j < p ? -col[p % HR] : col[p % HR];
-      asm volatile("bar.sync 1, 128;" ::: "memory");
-      const float piv = cp[p];
-      if (threadIdx.x == 0 && (!(piv > 0.f) || !isfinite(piv))) record_error(st, base + p, AXIA_ERR_ZERO_PIVOT);
-      const float d = __frcp_rn(piv);
-      const float rp = (j < p ? -cp[j] : cp[j]) * d;  // A_pj / A_pp
-      const float* ch = cp + HR * h;
-      if (j == p) {  // the pivot column: -A_ip / A_pp, and 1 / A_pp on the pivot
-#pragma unroll
-        for (int i4 = 0; i4 < HR; i4 += 4) {
-          const float4 c4 = *reinterpret_cast<const float4*>(ch + i4);
-          col[i4] = -c4.x * d;
-          col[i4 + 1] = -c4.y * d;
-          col[i4 + 2] = -c4.z * d;
-          col[i4 + 3] = -c4.w * d;
-        }
-        if (mine) col[p % HR] = d;
-      } else {
-#pragma unroll
-        for (int i4 = 0; i4 < HR; i4 += 4) {
-          const float4 c4 = *reinterpret_cast<const float4*>(ch + i4);
-          col[i4] = fmaf(-c4.x, rp, col[i4]);
-          col[i4 + 1] = fmaf(-c4.y, rp, col[i4 + 1]);
-          col[i4 + 2] = fmaf(-c4.z, rp, col[i4 + 2]);
-          col[i4 + 3] = fmaf(-c4.w, rp, col[i4 + 3]);
-        }
-        if (mine) col[p % HR] = rp;
-      }
-    }
-#pragma unroll
-    for (int i = 0; i < HR; ++i) out[(HR * h + i) * GJ_T + j] = col[i];
-  }
-  __syncthreads();
-}
-
 __device__ __forceinline__ void gj_store_regs(const float (&a)[4][4], float* g, int ld) {
   const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
 #pragma unroll
@@ -671,112 +590,217 @@ __device__ __forceinline__ void gj_store_regs(const float (&a)[4][4], float* g, 
     *reinterpret_cast<float4*>(g + (size_t)(4 * ty + r) * ld + 4 * tx) = make_float4(a[r][0], a[r][1], a[r][2], a[r][3]);
 }
 
+// Gauss-Jordan inverse of one 64 x 64 SPD tile held as the threads' 4 x 4
+// parts: four steps of 16 pivots, the same elimination with 16 x 16 tiles.
+// Warp 0 inverts the pivot tile with half a column per lane and shuffles; all
+// threads form the 16 new rows in Rb and update their parts.  A serial chain
+// of 64 pivots bounds it; this rolled form replaced 64 unrolled pivots on 128
+// threads, which took 26 us per tile (figures of the whole inverse above).
+// T: 64 rows and Rb: 16 rows of stride GJ_LD; the inverse goes to out (row-major).
+__device__ __forceinline__ void gj_invert_tile(float (&a)[4][4], float (*T)[GJ_LD], float (*Rb)[GJ_LD], float* out,
+                                               DevStatus* st, int base) {
+  const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4, lane = threadIdx.x & 31;
+#pragma unroll 1
+  for (int s = 0; s < GJ_T / GJ_S; ++s) {
+    const int s0 = GJ_S * s;
+    gj_store_regs(a, &T[0][0], GJ_LD);
+    __syncthreads();
+    if (threadIdx.x < 32) {
+      const int j = lane & 15, h = lane >> 4;  // column j, rows 8 h .. 8 h + 7
+      float col[8];
+#pragma unroll
+      for (int r = 0; r < 8; ++r) col[r] = T[s0 + 8 * h + r][s0 + j];
+#pragma unroll
+      for (int p = 0; p < GJ_S; ++p) {
+        const float piv = __shfl_sync(0xffffffffu, col[p % 8], (p / 8) * 16 + p);
+        const float apj = __shfl_sync(0xffffffffu, col[p % 8], (p / 8) * 16 + j);
+        if (lane == 0 && (!(piv > 0.f) || !isfinite(piv))) record_error(st, base + s0 + p, AXIA_ERR_ZERO_PIVOT);
+        const float d = __frcp_rn(piv);
+        const float rp = apj * d;
+#pragma unroll
+        for (int r = 0; r < 8; ++r) {
+          const float aip = __shfl_sync(0xffffffffu, col[r], h * 16 + p);
+          const float v = j == p ? -aip * d : fmaf(-aip, rp, col[r]);
+          col[r] = r == p % 8 && h == p / 8 ? (j == p ? d : rp) : v;
+        }
+      }
+#pragma unroll
+      for (int r = 0; r < 8; ++r) Rb[8 * h + r][s0 + j] = col[r];
+    }
+    __syncthreads();
+    if (tx / 4 != s) {  // new row ty of the panel, columns 4 tx ..
+      float o[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+      for (int q = 0; q < GJ_S; ++q) {
+        const float x = Rb[ty][s0 + q];
+        const float4 y = *reinterpret_cast<const float4*>(&T[s0 + q][4 * tx]);
+        o[0] = fmaf(x, y.x, o[0]);
+        o[1] = fmaf(x, y.y, o[1]);
+        o[2] = fmaf(x, y.z, o[2]);
+        o[3] = fmaf(x, y.w, o[3]);
+      }
+      *reinterpret_cast<float4*>(&Rb[ty][4 * tx]) = make_float4(o[0], o[1], o[2], o[3]);
+    }
+    __syncthreads();
+    if (ty / 4 == s) {
+#pragma unroll
+      for (int r = 0; r < 4; ++r)
+#pragma unroll
+        for (int c = 0; c < 4; ++c) a[r][c] = Rb[4 * (ty & 3) + r][4 * tx + c];
+    } else {
+      if (tx / 4 == s) {
+#pragma unroll
+        for (int r = 0; r < 4; ++r)
+#pragma unroll
+          for (int c = 0; c < 4; ++c) a[r][c] = 0.f;
+      }
+#pragma unroll
+      for (int q = 0; q < GJ_S; ++q) {
+        const float4 y = *reinterpret_cast<const float4*>(&Rb[q][4 * tx]);
+#pragma unroll
+        for (int r = 0; r < 4; ++r) {
+          const float x = -T[4 * ty + r][s0 + q];
+          a[r][0] = fmaf(x, y.x, a[r][0]);
+          a[r][1] = fmaf(x, y.y, a[r][1]);
+          a[r][2] = fmaf(x, y.z, a[r][2]);
+          a[r][3] = fmaf(x, y.w, a[r][3]);
+        }
+      }
+    }
+    __syncthreads();
+  }
+  gj_store_regs(a, out, GJ_T);
+}
+
 // Step k uses P_k = piv[k & 1].  The next pivot tile (k+1, k+1) is a trailing
 // tile of step k: block 0 updates it alone and inverts it at once (lookahead)
 // while the other blocks update the remaining tiles, so no step waits for a
 // serial pivot inversion except the first.
-// Inverts the n x n block at P.A in place; false when a barrier gave up.
+// Inverts the n x n block at P.A, of which only the tiles j <= i are read and
+// written; false when a barrier gave up.
 __device__ __forceinline__ bool gj_invert_block(GjArgs P) {
   __shared__ __align__(16) float sa[GJ_T][GJ_LD];
   __shared__ __align__(16) float sb[GJ_T][GJ_LD];
   const int nt = P.n / GJ_T, ld = P.n;
-  const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
   auto tile = [&](int i, int j) { return P.A + (size_t)i * GJ_T * ld + (size_t)j * GJ_T; };
   auto piv = [&](int k) { return P.piv + (size_t)(k & 1) * GJ_T * GJ_T; };
+  float* const C = P.W;
+  float* const R = P.W + (size_t)GJ_T * ld;
+  float a[4][4], o[4][4];
+  if (P.rank == 0) {
+    gj_load_regs(a, tile(0, 0), ld);
+    gj_invert_tile(a, sa, sb, piv(0), P.st, 0);
+  }
   for (int k = 0; k < nt; ++k) {
-    // 1. block 0 stores P_(k-1) into its tile (and inverts tile (0, 0) at
-    //    k = 0); the other blocks write step k-1's column panel
-    if (P.rank == 0) {
-      if (k > 0) gj_store_global(piv(k - 1), tile(k - 1, k - 1), ld);
-      if (k == 0) {
-        float a[4][4];
-        gj_load_regs(a, tile(0, 0), ld);
-        gj_invert_tile(a, &sa[0][0], &sb[0][0], piv(0), P.st, 0);
-      }
-    } else if (k > 0) {
-      gj_column_panel(P, k - 1, P.rank - 1, P.nb - 1);
-    }
     if (!group_sync(P.bar, P.st, P.limit_ns, P.nb)) return false;
-    // 2. row panel: A_kj <- P_k A_kj
+    // 1. panels: C_j and R_j = P_k C_j (P_k is symmetric)
     for (int j = P.rank; j < nt; j += P.nb) {
       if (j == k) continue;
       __syncthreads();
-      gj_load_t(sa, piv(k), GJ_T);
-      gj_load(sb, tile(k, j), ld);
+      gj_load(sa, piv(k), GJ_T);
+      if (j < k) {
+        gj_load(sb, tile(k, j), ld);
+      } else {  // A_jk^T
+        const float* g = tile(j, k);
+        for (int t = threadIdx.x; t < GJ_T * GJ_T; t += blockDim.x)
+          sb[t % GJ_T][t / GJ_T] = g[(size_t)(t / GJ_T) * ld + t % GJ_T];
+      }
       __syncthreads();
-      float o[4][4];
+      gj_load_regs(a, &sb[0][0], GJ_LD);
+      gj_store_regs(a, C + (size_t)j * GJ_T, ld);
       gj_mul(sa, sb, o);
-      gj_store_regs(o, tile(k, j), ld);
+      gj_store_regs(o, R + (size_t)j * GJ_T, ld);
     }
     if (!group_sync(P.bar, P.st, P.limit_ns, P.nb)) return false;
-    // 3. trailing tiles j <= i (i, j != k): A_ij -= A_ik R_j, mirrored into
-    //    A_ji; block 0 takes tile (k+1, k+1) alone and inverts it
+    // 2. trailing tiles j <= i (i, j != k): A_ij -= S_i C_i^T R_j; block 0
+    //    takes tile (k+1, k+1) alone and inverts it
     const int m = nt - 1, ntiles = m * (m + 1) / 2;
-    const bool ahead = k + 1 < nt && P.nb > 1;
+    const bool ahead = k + 1 < nt;
     const int tdiag = ahead ? k * (k + 1) / 2 + k : -1;  // (k+1, k+1) in the compressed numbering
     if (ahead && P.rank == 0) {
       __syncthreads();
-      gj_load_t(sa, tile(k + 1, k), ld);
-      gj_load(sb, tile(k, k + 1), ld);
+      gj_load(sa, C + (size_t)(k + 1) * GJ_T, ld);
+      gj_load(sb, R + (size_t)(k + 1) * GJ_T, ld);
+      gj_load_regs(a, tile(k + 1, k + 1), ld);
       __syncthreads();
-      float o[4][4], a[4][4];
       gj_mul(sa, sb, o);
-      const float* g = tile(k + 1, k + 1);
 #pragma unroll
-      for (int r = 0; r < 4; ++r) {
-        const float4 c = *reinterpret_cast<const float4*>(g + (size_t)(4 * ty + r) * ld + 4 * tx);
-        a[r][0] = c.x - o[r][0];
-        a[r][1] = c.y - o[r][1];
-        a[r][2] = c.z - o[r][2];
-        a[r][3] = c.w - o[r][3];
-      }
-      __syncthreads();  // sa / sb are reused as the tile and pivot-column buffers
-      gj_invert_tile(a, &sa[0][0], &sb[0][0], piv(k + 1), P.st, (k + 1) * GJ_T);
+      for (int r = 0; r < 4; ++r)
+#pragma unroll
+        for (int c = 0; c < 4; ++c) a[r][c] -= o[r][c];
+      __syncthreads();  // sa / sb are reused
+      gj_invert_tile(a, sa, sb, piv(k + 1), P.st, (k + 1) * GJ_T);
     }
     const int first = ahead ? P.rank - 1 : P.rank;
     const int stride = ahead ? P.nb - 1 : P.nb;
-    for (int t = first; first >= 0 && t < ntiles; t += stride) {
-      if (t == tdiag) continue;
-      int i = (int)((sqrtf(8.f * t + 1.f) - 1.f) * 0.5f);
-      while (i * (i + 1) / 2 > t) --i;
-      while ((i + 1) * (i + 2) / 2 <= t) ++i;
-      int j = t - i * (i + 1) / 2;
-      if (i >= k) ++i;
-      if (j >= k) ++j;
-      __syncthreads();
-      gj_load_t(sa, tile(i, k), ld);
-      gj_load(sb, tile(k, j), ld);
-      __syncthreads();
-      float o[4][4];
-      gj_mul(sa, sb, o);
-      float* g = tile(i, j);
-      float v[4][4];
-#pragma unroll
-      for (int r = 0; r < 4; ++r) {
-        const float4 c = *reinterpret_cast<const float4*>(g + (size_t)(4 * ty + r) * ld + 4 * tx);
-        v[r][0] = c.x - o[r][0];
-        v[r][1] = c.y - o[r][1];
-        v[r][2] = c.z - o[r][2];
-        v[r][3] = c.w - o[r][3];
-        *reinterpret_cast<float4*>(g + (size_t)(4 * ty + r) * ld + 4 * tx) = make_float4(v[r][0], v[r][1], v[r][2], v[r][3]);
-      }
-      if (i != j) {  // A_ji = S_i S_j A_ij^T
-        const float sg = (i < k) == (j < k) ? 1.f : -1.f;
-        float* h = tile(j, i);
-#pragma unroll
-        for (int c = 0; c < 4; ++c)
-          *reinterpret_cast<float4*>(h + (size_t)(4 * tx + c) * ld + 4 * ty) =
-              make_float4(sg * v[0][c], sg * v[1][c], sg * v[2][c], sg * v[3][c]);
+    if (first < 0) continue;
+    // the new row and column k, from the last block on (the first have the most tiles)
+    for (int j = stride - 1 - first; j < nt; j += stride) {
+      if (j == k) {
+        gj_load_regs(a, piv(k), GJ_T);
+        gj_store_regs(a, tile(k, k), ld);
+      } else if (j < k) {
+        gj_load_regs(a, R + (size_t)j * GJ_T, ld);
+        gj_store_regs(a, tile(k, j), ld);
+      } else {  // -R_j^T through shared memory
+        __syncthreads();
+        gj_load(sa, R + (size_t)j * GJ_T, ld);
+        __syncthreads();
+        float* g = tile(j, k);
+        for (int q = threadIdx.x; q < GJ_T * GJ_T; q += blockDim.x)
+          g[(size_t)(q / GJ_T) * ld + q % GJ_T] = -sa[q % GJ_T][q / GJ_T];
       }
     }
-    if (!group_sync(P.bar, P.st, P.limit_ns, P.nb)) return false;
-  }
-  // the last step's P and column panel
-  const int k = nt - 1;
-  if (P.rank == 0) {
-    gj_store_global(piv(k), tile(k, k), ld);
-  } else {
-    gj_column_panel(P, k, P.rank - 1, P.nb - 1);
+    // trailing tiles; the next tile's operands are requested before this one's product
+    auto locate = [&](int t, int& i, int& j) {
+      i = (int)((sqrtf(8.f * t + 1.f) - 1.f) * 0.5f);
+      while (i * (i + 1) / 2 > t) --i;
+      while ((i + 1) * (i + 2) / 2 <= t) ++i;
+      j = t - i * (i + 1) / 2;
+      if (i >= k) ++i;
+      if (j >= k) ++j;
+    };
+    float4 pc[4], pr[4];
+    auto request = [&](int i, int j) {
+#pragma unroll
+      for (int u = 0; u < 4; ++u) {
+        const int r = (threadIdx.x >> 4) + 16 * u, c = 4 * (threadIdx.x & 15);
+        pc[u] = *reinterpret_cast<const float4*>(C + (size_t)r * ld + (size_t)i * GJ_T + c);
+        pr[u] = *reinterpret_cast<const float4*>(R + (size_t)r * ld + (size_t)j * GJ_T + c);
+      }
+      gj_load_regs(a, tile(i, j), ld);
+    };
+    int t = first == tdiag ? first + stride : first, i = 0, j = 0;
+    if (t < ntiles) {
+      locate(t, i, j);
+      request(i, j);
+    }
+    while (t < ntiles) {
+      __syncthreads();
+      float v[4][4];
+#pragma unroll
+      for (int u = 0; u < 4; ++u) {
+        const int r = (threadIdx.x >> 4) + 16 * u, c = 4 * (threadIdx.x & 15);
+        *reinterpret_cast<float4*>(&sa[r][c]) = pc[u];
+        *reinterpret_cast<float4*>(&sb[r][c]) = pr[u];
+#pragma unroll
+        for (int w = 0; w < 4; ++w) v[u][w] = a[u][w];
+      }
+      __syncthreads();
+      const int ci = i, cj = j;
+      t += t + stride == tdiag ? 2 * stride : stride;
+      if (t < ntiles) {
+        locate(t, i, j);
+        request(i, j);
+      }
+      gj_mul(sa, sb, o);
+      const float sg = ci < k ? 1.f : -1.f;
+#pragma unroll
+      for (int r = 0; r < 4; ++r)
+#pragma unroll
+        for (int c = 0; c < 4; ++c) v[r][c] = fmaf(sg, o[r][c], v[r][c]);
+      gj_store_regs(v, tile(ci, cj), ld);
+    }
   }
   return true;
 }
@@ -796,6 +820,7 @@ __global__ void __launch_bounds__(GJ_THREADS, 2) k_gj_inverse(GjArgs P, const Co
   for (int b = g; b < nblk; b += ngroups) {
     if (b != g && !group_sync(Q.bar, Q.st, Q.limit_ns, Q.nb)) return;
     Q.A = P.A + blk[b].off;
+    Q.W = P.W + blk[b].off;
     Q.n = blk[b].p;
     if (!gj_invert_block(Q)) return;
   }
@@ -814,8 +839,10 @@ __global__ void k_minv(const CoarseBlk* blk, const float* __restrict__ B, const 
     double Bs[6][6];
     for (int i = 0; i < 6; ++i)
       for (int j = 0; j < 6; ++j)
-        Bs[i][j] = (double)B[K.off + (size_t)(6 * I + i - K.u0) * ncp + 6 * J + j - K.u0] * scale[6 * I + i] *
-                   scale[6 * J + j];
+        {
+          const int r = 6 * I + i - K.u0, c = 6 * J + j - K.u0;  // the tiles on and below the diagonal hold B
+          Bs[i][j] = (double)B[K.off + (size_t)max(r, c) * ncp + min(r, c)] * scale[6 * I + i] * scale[6 * J + j];
+        }
     // U[i][l] = sum_j Bs[i][j] T_J[l][j]
     double U[6][6];
     for (int i = 0; i < 6; ++i)
@@ -1283,7 +1310,8 @@ int build_operator(axia_ctx* ctx, CoarseState* S) {
       ngroups = std::max(1, std::min(std::min(nblk, GJ_GROUPS), grid / 16));
     }
     AXIA_CUDA(ctx, cudaMemsetAsync(S->gj_bar, 0, sizeof(GridBarrier) * GJ_GROUPS, ctx->stream));
-    GjArgs P{S->a32, S->max_p, S->piv, S->gj_bar, ctx->d_status, 2000000000ull, 0, grid};
+    // the panels of a block (2 x 64 x p) use its place in minv, which is written next
+    GjArgs P{S->a32, S->max_p, S->minv, S->piv, S->gj_bar, ctx->d_status, 2000000000ull, 0, grid};
     const CoarseBlk* dblk = S->d_blk;
     void* params[] = {&P, &dblk, (void*)&nblk, &ngroups};
     AXIA_CUDA(ctx, cudaLaunchCooperativeKernel((const void*)k_gj_inverse, dim3(grid), dim3(GJ_THREADS), params, 0,
