@@ -1,14 +1,15 @@
 // batch.cu -- many load cases on one mesh in one persistent launch.
 //
-// 32 right-hand sides share every sweep over the node-block matrix: the
-// vectors are stored [nd][32] (the 32 load cases of a DOF contiguous), a warp
-// owns one block row, its four 8-lane groups walk the row's blocks, and each
-// lane applies the 3x3 block to 4 load cases with 16-byte vector loads, so a
-// block's 9 values are read once for 32 products.  Every column runs its own
-// Jacobi-PCG recurrence (solver/src/linalg.rs:199-259: its own alpha, beta,
-// convergence test) on the FP32 node-block matrix, with FP64 reliable updates
-// (x += x32, r = b - K x in FP64 for all columns) when every active column's
-// FP32 residual has dropped by delta, or one has reached the tolerance.
+// Up to NC = 8, 16 or 32 right-hand sides share every sweep over the node-block
+// matrix: the vectors are stored [nd][NC] (the load cases of a DOF contiguous),
+// a warp owns one block row, its groups of NC / TC lanes walk the row's blocks,
+// and each lane applies the 3x3 block to TC load cases, so a block's 9 values
+// are read once for NC products.  Every column runs its own Jacobi-PCG or
+// two-level recurrence (solver/src/linalg.rs:199-259: its own alpha, beta,
+// convergence test) on the FP32 node-block matrix, with reliable updates of all
+// columns (x += x32, r = b - K x: in FP64, or in double words with an FP64
+// confirmation where the FP32 low parts are assembled) when every active
+// column's FP32 residual has dropped by delta, or one has reached the tolerance.
 // A converged column is frozen (alpha = beta = 0).
 #include <algorithm>
 #include <cmath>
@@ -1531,6 +1532,10 @@ const void* batch_kernel(BatchTile t) {
 // of the products.
 int batch_width(int nc) { return nc <= 8 ? 8 : nc <= 16 ? 16 : NR; }
 
+// Their tiles: 7 cases at 60^3 with 8 columns (2,1) 33.1, (2,2) 30.8, (2,4) 31.1,
+// (1,4) 32.4, (4,2) 32.4 ms; 16 columns (4,1) 40.7, (2,2) 40.8, (2,4) 41.4, (4,2)
+// 42.3, (1,4) 45.7 ms.  32 cases at 80^3: (4,1) 140, (2,2) 147, (2,4) 149, (1,4)
+// 178, (1,8) 181 ms, hence kBatchDefault.
 template <bool COARSE>
 const void* narrow_kernel(int width) {
   return width == 8 ? (const void*)pcg_bsr_multi_kernel<COARSE, 8, 2, 2>
