@@ -505,7 +505,10 @@ pcg_group_reliable_kernel(BsrReliableArgs P, const MeshGroup* groups, const int*
     C.ldm = G.ldm;
     C.minv += G.moff;
   }
-  reliable_body<L32, V32, kL64, 2, COARSE>(P, C, R);
+  // one block per FP64 load without the coarse space: with two, the kernel kept
+  // its group's range in too few registers and spilled in the FP32 product's
+  // loop, 64 cubes of 10 to 40 edges 352 ms against 284
+  reliable_body<L32, V32, kL64, COARSE ? 2 : 1, COARSE>(P, C, R);
 }
 
 // b[d] = f[d] - K_fp u0 for free d, 0 for prescribed d
