@@ -815,6 +815,10 @@ int bsr_solve(axia_ctx* ctx, const double* d_f, double* d_u, const axia_solve_op
                       delta, max_iter, limit_ns};
     if (opts->preconditioner == AXIA_PRECOND_COARSE) {
       AXIA_TRY(coarse_prepare(ctx, opts->coarse_nodes, &P.C));
+      if (P.C.ldm > COARSE_MAX)  // coarse_step keeps r_c in shared memory (the batched solve does not)
+        return set_error(ctx, AXIA_ERR_TOO_LARGE,
+                         "coarse space: " + std::to_string(P.C.n_sub) + " subdomains in one system, " +
+                             std::to_string(COARSE_MAX / 6) + " at most");
       AXIA_TRY(reset_dev_status(ctx));
       AXIA_CUDA(ctx, cudaMemsetAsync(ctx->d_bar, 0, sizeof(GridBarrier), ctx->stream));
     }

@@ -929,8 +929,17 @@ int build_space(axia_ctx* ctx, CoarseState* S) {
     tsum += target[k];
   }
   if (!S->per_mesh) {
-    if (tsum > max_boxes)
-      for (int k = 0; k < nm; ++k) target[k] = std::max<int64_t>(1, target[k] * max_boxes / tsum);
+    if (tsum > max_boxes) {
+      int64_t sum = 0;
+      for (int k = 0; k < nm; ++k) sum += target[k] = std::max<int64_t>(1, target[k] * max_boxes / tsum);
+      // meshes rounded up to one subdomain take it from the largest ones
+      while (sum > max_boxes) {
+        const auto big = std::max_element(target.begin(), target.end());
+        if (*big <= 1) break;  // more meshes than subdomains: the CG kernel's launcher rejects them
+        --*big;
+        --sum;
+      }
+    }
   } else {
     // a block per mesh: at most max_boxes subdomains each, and the blocked
     // inversion (work ~ sum of block sizes cubed) at most twice that of one
@@ -993,8 +1002,6 @@ int build_space(axia_ctx* ctx, CoarseState* S) {
   }
   dev_release(ctx, d_bb);
   const int ncell = cell_base[nm];
-  if (!S->per_mesh && ncell > max_boxes + nm)
-    return set_error(ctx, AXIA_ERR_TOO_LARGE, "coarse space: more than " + std::to_string(max_boxes) + " subdomains");
   int *d_cell = nullptr, *d_count = nullptr, *d_sub = nullptr, *d_iota = nullptr, *d_cellsub = nullptr;
   int* d_sub_sorted = nullptr;
   double *d_centre = nullptr, *d_inv_h = nullptr;
