@@ -591,84 +591,113 @@ __device__ __forceinline__ void gj_store_regs(const float (&a)[4][4], float* g, 
 }
 
 // Gauss-Jordan inverse of one 64 x 64 SPD tile held as the threads' 4 x 4
-// parts: four steps of 16 pivots, the same elimination with 16 x 16 tiles.
-// Warp 0 inverts the pivot tile with half a column per lane and shuffles; all
-// threads form the 16 new rows in Rb and update their parts.  A serial chain
-// of 64 pivots bounds it; this rolled form replaced 64 unrolled pivots on 128
-// threads, which took 26 us per tile (figures of the whole inverse above).
-// T: 64 rows and Rb: 16 rows of stride GJ_LD; the inverse goes to out (row-major).
-__device__ __forceinline__ void gj_invert_tile(float (&a)[4][4], float (*T)[GJ_LD], float (*Rb)[GJ_LD], float* out,
+// parts, in four steps of 16 pivots.  The column of a pivot is always taken from
+// its row, A_ip = S_i A_pi, never from the other triangle: kept apart, the two
+// triangles drift by the condition times the rounding, and the lower one alone
+// is then no inverse (folded and slender meshes: eigenvalues of A M of -108 to
+// 100 where they are 0.99 to 1.01).  And the 16 pivots are applied one by one to
+// the 16 rows, whose values at their own pivots (U, and W = U / pivot) give the
+// rank-16 update of the rest: no inverse of a pivot block enters it.
+// A serial chain of 64 pivots bounds it: warp 0 runs the pivot block with half a
+// column per lane and shuffles, then four lanes share a column of the 16 rows.
+// T: 16 rows and B: 48 rows of stride GJ_LD; the inverse goes to out (row-major).
+__device__ __forceinline__ void gj_invert_tile(float (&a)[4][4], float (*T)[GJ_LD], float (*B)[GJ_LD], float* out,
                                                DevStatus* st, int base) {
+  __shared__ float s_d[GJ_S];
+  float (*const R)[GJ_LD] = B;              // the 16 rows after the step
+  float (*const U)[GJ_LD] = B + GJ_S;
+  float (*const W)[GJ_LD] = B + 2 * GJ_S;
   const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4, lane = threadIdx.x & 31;
 #pragma unroll 1
   for (int s = 0; s < GJ_T / GJ_S; ++s) {
     const int s0 = GJ_S * s;
-    gj_store_regs(a, &T[0][0], GJ_LD);
+    if (ty / 4 == s)
+#pragma unroll
+      for (int r = 0; r < 4; ++r)
+        *reinterpret_cast<float4*>(&T[4 * (ty & 3) + r][4 * tx]) = make_float4(a[r][0], a[r][1], a[r][2], a[r][3]);
     __syncthreads();
     if (threadIdx.x < 32) {
       const int j = lane & 15, h = lane >> 4;  // column j, rows 8 h .. 8 h + 7
       float col[8];
 #pragma unroll
-      for (int r = 0; r < 8; ++r) col[r] = T[s0 + 8 * h + r][s0 + j];
+      for (int r = 0; r < 8; ++r) col[r] = T[8 * h + r][s0 + j];
 #pragma unroll
       for (int p = 0; p < GJ_S; ++p) {
-        const float piv = __shfl_sync(0xffffffffu, col[p % 8], (p / 8) * 16 + p);
-        const float apj = __shfl_sync(0xffffffffu, col[p % 8], (p / 8) * 16 + j);
+        const float row = col[p % 8];  // of pivot p in the lanes of half p / 8
+        const float piv = __shfl_sync(0xffffffffu, row, (p / 8) * 16 + p);
+        const float apj = __shfl_sync(0xffffffffu, row, (p / 8) * 16 + j);
         if (lane == 0 && (!(piv > 0.f) || !isfinite(piv))) record_error(st, base + s0 + p, AXIA_ERR_ZERO_PIVOT);
         const float d = __frcp_rn(piv);
         const float rp = apj * d;
+        if (h == 0) U[p][s0 + j] = apj;
+        if (lane == 0) s_d[p] = d;
 #pragma unroll
         for (int r = 0; r < 8; ++r) {
-          const float aip = __shfl_sync(0xffffffffu, col[r], h * 16 + p);
+          const float api = __shfl_sync(0xffffffffu, row, (p / 8) * 16 + 8 * h + r);
+          const float aip = 8 * h + r < p ? -api : api;
           const float v = j == p ? -aip * d : fmaf(-aip, rp, col[r]);
           col[r] = r == p % 8 && h == p / 8 ? (j == p ? d : rp) : v;
         }
       }
 #pragma unroll
-      for (int r = 0; r < 8; ++r) Rb[8 * h + r][s0 + j] = col[r];
+      for (int r = 0; r < 8; ++r) R[8 * h + r][s0 + j] = col[r];
     }
     __syncthreads();
-    if (tx / 4 != s) {  // new row ty of the panel, columns 4 tx ..
-      float o[4] = {0.f, 0.f, 0.f, 0.f};
+    {
+      const int j = threadIdx.x >> 2, g = threadIdx.x & 3;  // column j, rows 4 g .. 4 g + 3
+      if (j / GJ_S != s) {                                  // the same for a whole warp
+        float v[4];
 #pragma unroll
-      for (int q = 0; q < GJ_S; ++q) {
-        const float x = Rb[ty][s0 + q];
-        const float4 y = *reinterpret_cast<const float4*>(&T[s0 + q][4 * tx]);
-        o[0] = fmaf(x, y.x, o[0]);
-        o[1] = fmaf(x, y.y, o[1]);
-        o[2] = fmaf(x, y.z, o[2]);
-        o[3] = fmaf(x, y.w, o[3]);
+        for (int r = 0; r < 4; ++r) v[r] = T[4 * g + r][j];
+#pragma unroll
+        for (int p = 0; p < GJ_S; ++p) {
+          const float u = __shfl_sync(0xffffffffu, v[p & 3], (lane & ~3) + (p >> 2));
+          const float rp = u * s_d[p];
+          if (g == p >> 2) {
+            U[p][j] = u;
+            W[p][j] = rp;
+          }
+          const float4 c4 = *reinterpret_cast<const float4*>(&U[p][s0 + 4 * g]);
+          const float c[4] = {c4.x, c4.y, c4.z, c4.w};
+#pragma unroll
+          for (int r = 0; r < 4; ++r) {
+            const int i = 4 * g + r;
+            v[r] = i == p ? rp : fmaf(i < p ? c[r] : -c[r], rp, v[r]);
+          }
+        }
+#pragma unroll
+        for (int r = 0; r < 4; ++r) R[4 * g + r][j] = v[r];
       }
-      *reinterpret_cast<float4*>(&Rb[ty][4 * tx]) = make_float4(o[0], o[1], o[2], o[3]);
     }
     __syncthreads();
+    const float sg = ty / 4 < s ? 1.f : -1.f;  // -S_i of this thread's rows
     if (ty / 4 == s) {
 #pragma unroll
       for (int r = 0; r < 4; ++r)
 #pragma unroll
-        for (int c = 0; c < 4; ++c) a[r][c] = Rb[4 * (ty & 3) + r][4 * tx + c];
+        for (int c = 0; c < 4; ++c) a[r][c] = R[4 * (ty & 3) + r][4 * tx + c];
+    } else if (tx / 4 == s) {
+#pragma unroll
+      for (int r = 0; r < 4; ++r)
+#pragma unroll
+        for (int c = 0; c < 4; ++c) a[r][c] = sg * R[4 * (tx & 3) + c][4 * ty + r];
     } else {
-      if (tx / 4 == s) {
-#pragma unroll
-        for (int r = 0; r < 4; ++r)
-#pragma unroll
-          for (int c = 0; c < 4; ++c) a[r][c] = 0.f;
-      }
 #pragma unroll
       for (int q = 0; q < GJ_S; ++q) {
-        const float4 y = *reinterpret_cast<const float4*>(&Rb[q][4 * tx]);
+        const float4 x = *reinterpret_cast<const float4*>(&U[q][4 * ty]);
+        const float4 y = *reinterpret_cast<const float4*>(&W[q][4 * tx]);
+        const float xr[4] = {sg * x.x, sg * x.y, sg * x.z, sg * x.w};
 #pragma unroll
         for (int r = 0; r < 4; ++r) {
-          const float x = -T[4 * ty + r][s0 + q];
-          a[r][0] = fmaf(x, y.x, a[r][0]);
-          a[r][1] = fmaf(x, y.y, a[r][1]);
-          a[r][2] = fmaf(x, y.z, a[r][2]);
-          a[r][3] = fmaf(x, y.w, a[r][3]);
+          a[r][0] = fmaf(xr[r], y.x, a[r][0]);
+          a[r][1] = fmaf(xr[r], y.y, a[r][1]);
+          a[r][2] = fmaf(xr[r], y.z, a[r][2]);
+          a[r][3] = fmaf(xr[r], y.w, a[r][3]);
         }
       }
     }
-    __syncthreads();
   }
+  __syncthreads();  // B is read
   gj_store_regs(a, out, GJ_T);
 }
 
