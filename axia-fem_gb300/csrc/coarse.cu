@@ -55,6 +55,8 @@ struct CoarseBlk {
 struct CoarseState {
   int nodes_target = 0;          // nodes per subdomain; 0: default_subdomains
   int fewer = 0;                 // automatic size: how often it was coarsened
+  std::vector<char> few;         // [n_meshes] automatic size: at most few_subdomains
+  std::vector<char> reducible;   // [n_meshes] few_subdomains is less than its subdomains now
   bool row_overflow = false;     // a node row reaches more subdomains than its item list holds
   bool per_mesh = false;         // one block per mesh
   std::vector<CoarseBlk> blk;
@@ -928,14 +930,18 @@ int grid_for(const axia_ctx* ctx, int64_t n, int threads) {
 // 15^3 48 7.3, 150 6.1, 252 6.4; 25^3 125 16.1, 343 14.9, 648 17.0; C3D10
 // 13x11x12 27 6.5, 120 4.6.  64 cubes of 10 to 40 edges, solve: 232 in all
 // 187 ms, 1071 104, 3085 77, 4899 77 (and 5 ms more for the inverse).
-// `fewer` counts fallbacks to larger subdomains: a quarter each time, at
-// the last step of 500 nodes (13,500 blocks) and 1/512 of the mesh at least.
+// `fewer` counts the fallbacks after a row overflow: a quarter each time, and
+// at the last step no more than few_subdomains.
 constexpr int DEFAULT_SUBDOMAIN_STEPS = 3;
-int64_t default_subdomains(double nodes, double blocks_per_row, int fewer) {
+// At least 500 nodes of C3D8 (13,500 node blocks) per subdomain, at most 512 subdomains.
+double few_subdomains(double nodes, double blocks_per_row) {
+  return nodes / std::max(500.0 * 27.0 / std::max(blocks_per_row, 1.0), nodes / 512.0);
+}
+int64_t default_subdomains(double nodes, double blocks_per_row, int fewer, bool few) {
   const double dense = std::max(blocks_per_row, 1.0) / 27.0;
   double v = std::min(0.46 * std::pow(std::max(nodes, 1.0), 0.55) * std::max(dense, 1.0), nodes / 50.0);
   for (int k = 0; k < fewer; ++k) v *= 0.25;
-  if (fewer >= DEFAULT_SUBDOMAIN_STEPS) v = std::min(v, nodes / std::max(500.0 / dense, nodes / 512.0));
+  if (few || fewer >= DEFAULT_SUBDOMAIN_STEPS) v = std::min(v, few_subdomains(nodes, blocks_per_row));
   return std::max<int64_t>(1, (int64_t)std::min(512.0, v));
 }
 
@@ -949,12 +955,15 @@ int build_space(axia_ctx* ctx, CoarseState* S) {
   auto mesh_a0 = [&](int k) { return nm > 1 ? ctx->mesh_node0[k] : (int64_t)0; };
   auto mesh_a1 = [&](int k) { return nm > 1 ? ctx->mesh_node0[k + 1] : n; };
   const int max_boxes = COARSE_MAX / 6;
+  const double blocks_per_row = (double)ctx->n_adj / (double)n;
   std::vector<int64_t> target(nm);
+  S->few.resize(nm, 0);
+  S->reducible.assign(nm, 0);
   int64_t tsum = 0;
   for (int k = 0; k < nm; ++k) {
     const int64_t nk = mesh_a1(k) - mesh_a0(k);
     target[k] = S->nodes_target > 0 ? std::max<int64_t>(1, nk / S->nodes_target)
-                                    : default_subdomains((double)nk, (double)ctx->n_adj / (double)n, S->fewer);
+                                    : default_subdomains((double)nk, blocks_per_row, S->fewer, S->few[k]);
     tsum += target[k];
   }
   if (!S->per_mesh) {
@@ -1021,6 +1030,8 @@ int build_space(axia_ctx* ctx, CoarseState* S) {
       g.nx = g.ny = g.nz = 1;
       h = 2.0 * emax;
     }
+    S->reducible[k] = S->nodes_target == 0 &&
+                      std::max(1.0, std::floor(few_subdomains((double)nk, blocks_per_row))) < (double)target[k];
     g.x0 = lo[0];
     g.y0 = lo[1];
     g.z0 = lo[2];
@@ -1367,6 +1378,81 @@ int build_operator(axia_ctx* ctx, CoarseState* S) {
   return read_status(ctx, "coarse operator is not positive definite");
 }
 
+// What a coarse correction's rounding does to the residual, per subdomain: the
+// mean diagonal entry of K over its free DOFs times its part of the trace of the
+// coarse inverse (orthonormal modes); infinite where a diagonal entry of the
+// inverse is not positive.  Warp per subdomain, fixed order.
+__global__ void k_reach(int n_sub, const int* sub_ptr, const int* sub_node, const float4* geo,
+                        const float* __restrict__ dinv, const CoarseBlk* blk, const int* sub_blk,
+                        const float* __restrict__ B, const double* __restrict__ scale, double* reach) {
+  const int lane = threadIdx.x & 31;
+  const int nw = (gridDim.x * blockDim.x) >> 5;
+  for (int I = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; I < n_sub; I += nw) {
+    float k = 0.f, cnt = 0.f;
+#pragma unroll 4
+    for (int t = sub_ptr[I] + lane; t < sub_ptr[I + 1]; t += 32) {
+      const int a = sub_node[t];
+      const unsigned m = geo_bits(geo[a]);
+      for (int d = 0; d < 3; ++d)
+        if ((m >> d) & 1u) {
+          k += 1.f / dinv[3 * a + d];
+          cnt += 1.f;
+        }
+    }
+    k = warp_sum(k);
+    cnt = warp_sum(cnt);
+    if (lane == 0) {
+      const CoarseBlk K = blk[sub_blk[I]];
+      double s = 0.0;
+      for (int i = 6 * I; i < 6 * I + 6; ++i) {
+        const double b = B[K.off + (size_t)(i - K.u0) * (K.p + 1)];
+        if (scale[i] > 0.0) s += b > 0.0 ? scale[i] * scale[i] * b : 1.0 / 0.0;
+      }
+      reach[I] = cnt > 0.f ? s * (double)(k / cnt) : 0.0;
+    }
+  }
+}
+
+// The limit of a mesh's summed reach.  FP32 rounds what the correction adds to
+// K p at about 6e-8 of |K| |p|, so the noise it leaves in the residual is 6e-8
+// of the reach: 3 % at the limit.  Slender, thin and folded meshes pass it, the
+// more so the more subdomains they have; compact blocks stay below 1e5.
+// Measured on 114 slender, thin, folded and hollow shapes under several loads,
+// 1e-3 to 1e-8, the default count against few_subdomains: below 5e5 (58 shapes)
+// fewer iterations in 606 solves, more in 18, solved only by the one in 16 and
+// only by the other in 11; from 5e5 on 126, 18, 12 and 53.  Axial loads,
+// iterations with few_subdomains / the default: bar 90x10x10 (4.3e5) to 1e-8 107 /
+// 65, 120x12x12 (7.7e5) to 1e-8 136 / NaN, 128x8x8 (1.9e6) to 1e-6 68 / not converged.
+constexpr double FP32_REACH = 5e5;
+
+// Automatic size, after build_operator returned st: marks in `few` the meshes
+// out of FP32's reach (a pivot that was not positive, without such a mesh: all);
+// true when that is any.
+bool mark_few(axia_ctx* ctx, CoarseState* S, int st, std::vector<char>& few) {
+  const size_t nm = S->reducible.size();
+  if ((st != AXIA_OK && st != AXIA_ERR_ZERO_PIVOT) ||
+      std::find(S->reducible.begin(), S->reducible.end(), 1) == S->reducible.end())
+    return false;
+  const int n_sub = S->args.n_sub;
+  double* d_reach = nullptr;
+  std::vector<double> reach(n_sub);
+  if (dev_alloc(ctx, &d_reach, (size_t)n_sub) != AXIA_OK) return false;
+  k_reach<<<grid_for(ctx, (int64_t)n_sub * 32, 128), 128, 0, ctx->stream>>>(
+      n_sub, S->sub_ptr, S->sub_node, S->geo, ctx->d_bdinv32, S->d_blk, S->d_sub_blk, S->a32, S->scale, d_reach);
+  ctx->launches++;
+  const int cst = copy_to_host(ctx, reach.data(), d_reach, (size_t)n_sub);
+  dev_release(ctx, d_reach);
+  if (cst != AXIA_OK) return false;
+  bool any = false;
+  for (int pass = 0; pass < (st == AXIA_OK ? 1 : 2) && !any; ++pass)
+    for (size_t k = 0; k < nm; ++k) {
+      double sum = 0.0;
+      for (int I = S->mesh_sub[k]; I < S->mesh_sub[k + 1]; ++I) sum += reach[I];
+      if (S->reducible[k] && (pass || !(sum <= FP32_REACH))) any = few[k] = 1;
+    }
+  return any;
+}
+
 }  // namespace
 
 void coarse_release(axia_ctx* ctx) {
@@ -1390,12 +1476,16 @@ int coarse_prepare(axia_ctx* ctx, int nodes_target, CoarseArgs* out, bool per_me
     coarse_release(ctx);
     S = nullptr;
   }
-  for (int fewer = 0;; ++fewer) {
+  int fewer = S ? S->fewer : 0;
+  std::vector<char> few;
+  if (S) few = S->few;
+  for (;;) {
     if (!S) {
       S = new CoarseState();
       S->nodes_target = nodes_target;
       S->per_mesh = per_mesh;
       S->fewer = fewer;
+      S->few = few;
       ++ctx->coarse_gen;
       ctx->coarse = S;
       const int st = build_space(ctx, S);
@@ -1403,16 +1493,24 @@ int coarse_prepare(axia_ctx* ctx, int nodes_target, CoarseArgs* out, bool per_me
         coarse_release(ctx);
         return st;
       }
+      few = S->few;
     }
     if (S->op_gen == ctx->assemble_gen) break;
     const int st = build_operator(ctx, S);
-    if (st == AXIA_OK) {
+    // The automatic size falls back to larger subdomains where a node row
+    // reaches more of them than an item list holds (very flat elements, hub
+    // nodes) and where the correction is out of FP32's reach.
+    bool retry = false;
+    if (S->row_overflow) {
+      retry = nodes_target == 0 && fewer < DEFAULT_SUBDOMAIN_STEPS;
+      ++fewer;
+    } else {
+      retry = mark_few(ctx, S, st, few);
+    }
+    if (st == AXIA_OK && !retry) {
       S->op_gen = ctx->assemble_gen;
       break;
     }
-    // very flat elements or hub nodes: a node row reaches more subdomains than
-    // an item list holds; the automatic size then falls back to larger ones
-    const bool retry = S->row_overflow && nodes_target == 0 && fewer < DEFAULT_SUBDOMAIN_STEPS;
     coarse_release(ctx);  // a half-built operator is not reused
     S = nullptr;
     if (!retry) return st;
