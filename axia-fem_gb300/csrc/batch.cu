@@ -2187,6 +2187,11 @@ int batch_solve(axia_ctx* ctx, int nrhs, const double* d_F, double* d_U, const a
                                                            ctx->d_mB);
     ctx->launches++;
     AXIA_CUDA(ctx, cudaMemsetAsync(ctx->d_bar, 0, sizeof(GridBarrier), ctx->stream));
+    // coarse_solve_m reads R_c up to the padded size; past nc a launch of another
+    // width has left rows of its own there, and 0 times a NaN of it is no zero
+    if (coarse && cargs.ncp > cargs.nc)
+      AXIA_CUDA(ctx, cudaMemsetAsync(cargs.rc_m + (size_t)cargs.nc * width, 0,
+                                     (size_t)(cargs.ncp - cargs.nc) * width * sizeof(float), ctx->stream));
     MultiArgs P = multi_args(ctx, opts->rtol, delta, max_iter, cargs);
     if (split) {
       P.state = static_cast<BatchState*>(ctx->d_mstate);
