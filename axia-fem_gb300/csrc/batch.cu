@@ -353,6 +353,9 @@ struct MultiArgs {
   int resume = 0;       // start from state, after an update whose |r|^2 and r.D^-1 r are in totals
 };
 
+// in place of a case's residual norm: its CG met p.Ap = 0, its load is not finite
+constexpr double RES_BROKE = -1.0, RES_NONFINITE = -2.0;
+
 constexpr int SL_A = 0;  // two banks of NC slots: SL_A .. and NC ..
 
 // ---------------------------------------------------------------------------
@@ -743,6 +746,10 @@ __global__ void __launch_bounds__(PCG_THREADS, 2) pcg_bsr_multi_kernel(MultiArgs
     s_restart[c] = 0;
     s_rrec[c] = s_bnorm[c];
     if (!s_active[c]) s_res[c] = 0.0;
+    if (!isfinite(s_bnorm[c])) {  // not a zero load: reported below
+      s_active[c] = 0;
+      s_res[c] = RES_NONFINITE;
+    }
   }
   __syncthreads();
   if constexpr (COARSE) {  // P = D^-1 B + Z M Z^T B
@@ -824,7 +831,7 @@ __global__ void __launch_bounds__(PCG_THREADS, 2) pcg_bsr_multi_kernel(MultiArgs
       if (s_active[c]) {
         if (!(fabs(pq) >= 1e-30) || !isfinite(pq)) {
           s_active[c] = 0;  // breakdown: freeze the column, report below
-          s_res[c] = -1.0;
+          s_res[c] = RES_BROKE;
         } else {
           al = (float)(s_rz[c] / pq);
           s_citers[c] = it + 1;
@@ -949,12 +956,14 @@ __global__ void __launch_bounds__(PCG_THREADS, 2) pcg_bsr_multi_kernel(MultiArgs
     }
     if (!iteration_tail(!s_flag)) return;
   }
-  int any_active = 0, broke = 0;
+  int any_active = 0, broke = 0, bad = 0;
   for (int c = 0; c < NC; ++c) {
     any_active |= s_active[c];
-    broke |= s_res[c] < 0.0;
+    broke |= s_res[c] == RES_BROKE;
+    bad |= s_res[c] == RES_NONFINITE;
   }
-  if (broke) status = AXIA_ERR_ZERO_PIVOT;
+  if (bad) status = AXIA_ERR_NONFINITE;
+  else if (broke) status = AXIA_ERR_ZERO_PIVOT;
   else if (any_active) status = AXIA_ERR_NOT_CONVERGED;
   if (blockIdx.x == 0 && threadIdx.x < NC) {
     const int c = threadIdx.x;
@@ -1946,11 +1955,13 @@ int batch_block_solve(axia_ctx* ctx, int nrhs, const double* d_F, double* d_U, c
     for (int c = 0; c < NR; ++c) {
       bnorm[c] = std::sqrt(h[c]);
       rmax[c] = res[c] = bnorm[c];
+      if (!std::isfinite(bnorm[c])) st = set_error(ctx, AXIA_ERR_NONFINITE, "block CG: a load case is not finite");
       if (!(bnorm[c] >= 1e-30)) {
         frozen |= 1u << c;
         res[c] = 0.0;
       }
     }
+    if (st != AXIA_OK) break;
     long long iters = 0;
     int updates = 0;
     if (frozen != 0xffffffffu) {
@@ -2212,12 +2223,13 @@ int batch_solve(axia_ctx* ctx, int nrhs, const double* d_F, double* d_U, const a
     info->iters = std::max<int64_t>(info->iters, o.iters);
     info->outer_iters += o.updates;
     for (int c = 0; c < nc; ++c) {
-      const double rr = o.bnorm[c] > 0 ? o.residual[c] / o.bnorm[c] : 0.0;
+      const double rr = o.residual[c] == RES_NONFINITE ? std::nan("") : o.bnorm[c] > 0 ? o.residual[c] / o.bnorm[c] : 0.0;
       if (rel_res) rel_res[c0 + c] = rr;
       worst = std::max(worst, rr);
     }
     if (o.status != AXIA_OK) {
       if (o.status == AXIA_ERR_ZERO_PIVOT) return set_error(ctx, o.status, "batched CG: zero pivot in a load case");
+      if (o.status == AXIA_ERR_NONFINITE) return set_error(ctx, o.status, "batched CG: a load case is not finite");
       return set_error(ctx, o.status, "batched CG did not converge in " + std::to_string(o.iters) + " iterations");
     }
     k_batch_out<<<ctx->sm_count * 8, 256, 0, ctx->stream>>>(nd, width, nc, ctx->d_ind_of, ctx->d_u0, ctx->d_mX,

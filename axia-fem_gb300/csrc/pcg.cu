@@ -497,6 +497,7 @@ int pcg_solve(axia_ctx* ctx, const axia_solve_opts* opts, axia_solve_info* info)
   info->iters = 0;
   info->outer_iters = 0;
   double rnorm = bnorm;
+  if (!std::isfinite(bnorm)) return set_error(ctx, AXIA_ERR_NONFINITE, "CG: the load is not finite");
   if (bnorm < 1e-30) {
     info->residual = 0.0;
     return AXIA_OK;

@@ -221,10 +221,11 @@ __device__ __forceinline__ void mixed_begin(CgScalars<float>& S, const double* t
   S.rz = (float)t[1];
   S.bnorm = S.residual = sqrt(t[0]);
   mixed_limit(S, tol, delta);
-  S.status = AXIA_OK;
+  S.status = isfinite(t[0]) ? AXIA_OK : AXIA_ERR_NONFINITE;  // a load that is not finite is no zero load
   S.update = 0;
   S.stop = S.bnorm < 1e-30;
   if (S.stop) S.residual = 0.0;
+  if (S.status != AXIA_OK) S.stop = 1;
 }
 __device__ __forceinline__ void mixed_alpha(CgScalars<float>& S, const double* t) {
   const float pq = (float)t[0];
@@ -261,9 +262,10 @@ __device__ __forceinline__ void cg_begin(CgScalars<A>& S, const double* t, doubl
   S.rr = t[0];
   S.bnorm = sqrt(t[0]);
   S.limit2 = tol * S.bnorm * (tol * S.bnorm);
-  S.status = AXIA_OK;
-  S.stop = !(S.bnorm >= 1e-30);
+  S.status = isfinite(t[0]) ? AXIA_OK : AXIA_ERR_NONFINITE;
+  S.stop = S.bnorm < 1e-30;
   if (S.stop) S.rr = 0.0;
+  if (S.status != AXIA_OK) S.stop = 1;
 }
 template <typename A>
 __device__ __forceinline__ void cg_alpha(CgScalars<A>& S, const double* t) {
