@@ -362,7 +362,7 @@ static int launch_pcg_t(axia_ctx* ctx, PcgArgs<V>& P) {
   void* params[] = {&P};
   if constexpr (sizeof(V) == sizeof(double) && (L == 4 || L == 8)) {
     const void* one = (const void*)pcg_kernel<V, L, true>;
-    const int blocks = ctx->nnz <= CLUSTER_MAX_NNZ ? cluster_blocks(one, (int64_t)P.n * L) : 0;
+    const int blocks = cluster_csr(ctx->nnz, P.n, L) ? cluster_blocks(one, (int64_t)P.n * L) : 0;
     if (blocks) return launch_cluster(ctx, one, blocks, params);
   }
   AXIA_TRY(coop_grid(ctx, (const void*)kern, (int64_t)P.n * L, &grid));

@@ -120,12 +120,20 @@ __device__ __forceinline__ void block_partial(double v, double* partials) {
 // rows in FP64 the three of an iteration took 12 of its 17.5 us.
 constexpr int CLUSTER_MAX = 16;
 // Systems up to these sizes run as one cluster: 16 SMs against all of them,
-// cheap barriers against work.  Measured, us per iteration, cluster / whole
-// grid: FP64 CSR 88 k entries 10.3 / 18.1, 240 k 14.2 / 18.0, 430 k 17.6 / 18.1,
-// 690 k 25.2 / 19.3; FP32 node blocks with the two-level preconditioner 14 k
-// blocks 12.5 / 25.0, 52 k 14.9 / 24.3, 120 k 20.4 / 24.9, 230 k 31.0 / 24.7.
-constexpr int64_t CLUSTER_MAX_NNZ = 400000;
+// cheap barriers against work.  FP32 node blocks, two-level, us per iteration,
+// cluster / whole grid: 14 k blocks 12.5 / 25.0, 52 k 14.9 / 24.3, 120 k 20.4 /
+// 24.9, 230 k 31.0 / 24.7.
+// FP64 CSR: the entries, and 6.25 for every lane of a row, whose sums and vector
+// updates take the FP64 issue slots of 16 SMs (about 8 us + 0.018 per 1,000
+// entries + 0.11 per 1,000 rows and lane).  C3D8, 4 lanes: 88 k entries 10.3 / 18.1,
+// 240 k 14.2 / 18.0, 430 k (6 k rows) 17.6 / 18.1, 690 k 25.2 / 19.3; 5 and 7
+// entries per row: 20 k rows 19.0 / 16.7, 27 k 24.8 / 17.5, 55 k 41.0 / 22.6; 3 per
+// row: 40 k rows 26.6 / 17.9, 130 k 69.9 / 24.5.
 constexpr int64_t CLUSTER_MAX_BLOCKS = 130000;
+constexpr int64_t CLUSTER_MAX_CSR = 550000;
+constexpr bool cluster_csr(int64_t nnz, int64_t rows, int lanes) {
+  return nnz + rows * lanes * 25 / 4 <= CLUSTER_MAX_CSR;
+}
 
 // OUTLINED: the last block's sums in a function of their own.  Measured at C3D8
 // 90^3 / 100^3: mixed node blocks with the diagonal 167 us per iteration inline,
