@@ -650,7 +650,11 @@ template <typename V, int L>
 static int launch_bsr_pcg_t(axia_ctx* ctx, BsrPcgArgs<V>& P) {
   auto kern = pcg_bsr_kernel<V, L>;
   int grid = 0;
-  AXIA_TRY(coop_grid(ctx, (const void*)kern, (int64_t)P.M.n_nodes * L, &grid));
+  // one block per SM: a second one shares the FP64 pipe that bounds the products
+  // and doubles the partials of every barrier.  Solve in ms, one / two: C3D8 22^3
+  // 8.7 / 10.7, 26^3 13.6 / 16.2, 30^3 20.6 / 23.3, 40^3 51.0 / 54.2, 64^3 264 / 267;
+  // C3D20 14^3 28.9 / 33.1, 24^3 151 / 162.
+  AXIA_TRY(coop_grid(ctx, (const void*)kern, (int64_t)P.M.n_nodes * L, &grid, 0, 1));
   void* params[] = {&P};
   AXIA_CUDA(ctx, cudaLaunchCooperativeKernel((const void*)kern, dim3(grid), dim3(PCG_THREADS), params, 0, ctx->stream));
   ctx->launches++;

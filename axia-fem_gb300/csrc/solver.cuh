@@ -444,13 +444,15 @@ int reconstruct_system(axia_ctx* ctx, const ReducedSystem& S, const double* d_x,
 // Measured, us per iteration of the FP64 CSR form with 4 lanes: 17 k rows 152
 // blocks 19.9, 304 23.4; 71 k 37.6, 304 32.8, 456 38.2; 104 k 51.7, 41.8, 41.1;
 // 670 k 247, 164, 154.
-inline int coop_grid(axia_ctx* ctx, const void* kern, int64_t work, int* grid_out, size_t dyn_smem = 0) {
+// most: blocks per SM at most.
+inline int coop_grid(axia_ctx* ctx, const void* kern, int64_t work, int* grid_out, size_t dyn_smem = 0,
+                     int most = 1 << 30) {
   int per_sm = 0;
   AXIA_CUDA(ctx, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, PCG_THREADS, dyn_smem));
   if (per_sm < 1) return set_error(ctx, AXIA_ERR_CUDA, "PCG kernel does not fit on an SM");
   const int64_t need = std::max<int64_t>(1, (work + PCG_THREADS - 1) / PCG_THREADS);
   const int sms = ctx->sm_count;
-  const int rounds = need >= 12 * sms ? per_sm : std::min(per_sm, need >= 9 * sms / 4 ? 2 : 1);
+  const int rounds = std::min(std::min(per_sm, most), need >= 12 * sms ? per_sm : need >= 9 * sms / 4 ? 2 : 1);
   const int grid = (int)std::min<int64_t>(need, (int64_t)rounds * sms);
   if ((size_t)grid * N_SLOTS > ctx->partial_slots) return set_error(ctx, AXIA_ERR_STATE, "partials buffer too small");
   *grid_out = grid;
