@@ -467,8 +467,10 @@ inline int cluster_blocks(const void* kern, int64_t work) {
   const int64_t need = std::max<int64_t>(1, (work + PCG_THREADS - 1) / PCG_THREADS);
   int blocks = 1;
   while (blocks < need && blocks < CLUSTER_MAX) blocks *= 2;
-  if (blocks > 8 && cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess)
+  if (blocks > 8 && cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess) {
+    (void)cudaGetLastError();
     blocks = 8;
+  }
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(blocks);
   cfg.blockDim = dim3(PCG_THREADS);
