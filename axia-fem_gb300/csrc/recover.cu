@@ -371,12 +371,13 @@ element_recover_hex8_kernel(int64_t n_elem, const int32_t* __restrict__ conn, co
 // One thread per node: average over the incident elements in ascending order.
 __global__ void k_recover_nodes(int64_t n_nodes, int nn, const int64_t* __restrict__ ne_ptr,
                                 const int32_t* __restrict__ ne, const double* __restrict__ rec,
-                                const double* __restrict__ f, double nu, double inv_e, double* __restrict__ stress,
+                                const double* __restrict__ f, double nu, double e_strain, double* __restrict__ stress,
                                 double* __restrict__ strain, double* __restrict__ vm, double* __restrict__ rf) {
   for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n_nodes;
        i += (int64_t)gridDim.x * blockDim.x) {
-    double acc[6] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0}, ku[3] = {0.0, 0.0, 0.0}, cnt = 0.0;
-    for (int64_t k = ne_ptr[i]; k < ne_ptr[i + 1]; ++k) {
+    double acc[6] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0}, ku[3] = {0.0, 0.0, 0.0};
+    const int64_t k0 = ne_ptr[i], k1 = ne_ptr[i + 1];
+    for (int64_t k = k0; k < k1; ++k) {
       const int32_t packed = ne[k];
       const int64_t e = packed >> 5;
       const int a = packed & 31;
@@ -386,12 +387,19 @@ __global__ void k_recover_nodes(int64_t n_nodes, int nn, const int64_t* __restri
       ku[0] += r[6];
       ku[1] += r[7];
       ku[2] += r[8];
-      cnt += 1.0;
     }
+    // the mean as a division rounds it; 1, 2, 4 and 8 elements, all of a grid of
+    // hexahedra, have an exact reciprocal
     double s[6];
-    const double inv_cnt = cnt > 0.0 ? 1.0 / cnt : 0.0;
+    const int64_t n = k1 - k0;
+    const double cnt = (double)n, inv_cnt = n > 0 ? 1.0 / cnt : 0.0;
+    if ((n & (n - 1)) == 0) {
 #pragma unroll
-    for (int c = 0; c < 6; ++c) s[c] = acc[c] * inv_cnt;
+      for (int c = 0; c < 6; ++c) s[c] = acc[c] * inv_cnt;
+    } else {
+#pragma unroll
+      for (int c = 0; c < 6; ++c) s[c] = acc[c] / cnt;
+    }
     if (stress) {
 #pragma unroll
       for (int c = 0; c < 6; ++c) stress[6 * i + c] = s[c];
@@ -402,11 +410,11 @@ __global__ void k_recover_nodes(int64_t n_nodes, int nn, const int64_t* __restri
     }
     if (strain) {
       const double tr = s[0] + s[1] + s[2];
-      const double inv_g2 = (1.0 + nu) * inv_e;
+      const double g2 = e_strain / (1.0 + nu);
 #pragma unroll
-      for (int c = 0; c < 3; ++c) strain[6 * i + c] = ((1.0 + nu) * s[c] - nu * tr) * inv_e;
+      for (int c = 0; c < 3; ++c) strain[6 * i + c] = ((1.0 + nu) * s[c] - nu * tr) / e_strain;
 #pragma unroll
-      for (int c = 3; c < 6; ++c) strain[6 * i + c] = s[c] * inv_g2;
+      for (int c = 3; c < 6; ++c) strain[6 * i + c] = s[c] / g2;
     }
     if (rf) {
 #pragma unroll
@@ -641,7 +649,7 @@ int recover_device(axia_ctx* ctx, const double* d_u, const double* d_f, double e
   const unsigned grid = (unsigned)std::max<int64_t>(
       1, std::min<int64_t>((ctx->n_nodes + 255) / 256, (int64_t)ctx->sm_count * 16));
   k_recover_nodes<<<grid, 256, 0, ctx->stream>>>(ctx->n_nodes, ctx->nn, ctx->d_ne_ptr, ctx->d_ne, ctx->d_rec, d_f,
-                                                 ctx->nu, 1.0 / e_strain, d_stress, d_strain, d_vm, d_rf);
+                                                 ctx->nu, e_strain, d_stress, d_strain, d_vm, d_rf);
   ctx->launches++;
   AXIA_CUDA(ctx, cudaGetLastError());
   DevStatus hs;
