@@ -39,3 +39,14 @@ def test_shear_strains_of_hexahedra(gpu_ctx, n):
     want = ((1.0 + NU) * stress[:, :3] - NU * tr) / E
     # the numerator's rounding differs by a fused multiply-add: a few ulp of its terms
     assert np.abs(strain[:, :3] - want).max() <= 4 * 2.0**-53 * np.abs(stress[:, :3]).max() * 3 / E
+
+
+def test_not_finite(gpu_ctx):
+    """Infinities and NaN of the stresses go through as a division passes them."""
+    m = meshgen.block_c3d8_pressure(n=3, e=E, nu=NU, perturb=0.2)
+    gpu_ctx.setup(m)
+    u = np.random.default_rng(3).standard_normal(m.ndof) * 3e302  # strains of 1e303, E times that overflows
+    stress, strain, _, _, _ = gpu_ctx.recover(u, e_strain=E)
+    assert np.isinf(stress[:, 3:]).any()
+    with np.errstate(all="ignore"):
+        assert np.array_equal(strain[:, 3:], stress[:, 3:] / (E / (1.0 + NU)), equal_nan=True)
