@@ -8,7 +8,7 @@
 //   * bounding box -> a uniform grid of at most COARSE_MAX / 6 boxes of about
 //     `nodes_target` nodes each; every non-empty box is a subdomain;
 //   * the nodes sorted by subdomain (stable radix sort: ascending node order
-//     inside each subdomain), cut into chunks of COARSE_CHUNK nodes;
+//     inside each subdomain), cut into chunks of 32 to COARSE_CHUNK nodes;
 //   * centre c_I, and per node (x_a - c_I) / h and its free-DOF mask (geo);
 //   * per subdomain the Gram matrix G = Z_I^T Z_I over the free DOFs and
 //     T = L^-T from its Cholesky factor, modes whose pivot vanishes dropped
@@ -57,6 +57,8 @@ struct CoarseState {
   int fewer = 0;                 // automatic size: how often it was coarsened
   std::vector<char> few;         // [n_meshes] automatic size: at most few_subdomains
   std::vector<char> reducible;   // [n_meshes] few_subdomains is less than its subdomains now
+  double* reach = nullptr;       // [n_sub] k_reach, with a reducible mesh
+  std::vector<double> h_reach;   // of the last operator
   bool row_overflow = false;     // a node row reaches more subdomains than its item list holds
   bool per_mesh = false;         // one block per mesh
   std::vector<CoarseBlk> blk;
@@ -116,6 +118,7 @@ struct CoarseState {
     dev_release(ctx, a64);
     dev_release(ctx, a32);
     dev_release(ctx, scale);
+    dev_release(ctx, reach);
     dev_release(ctx, piv);
     dev_release(ctx, gj_bar);
     dev_release(ctx, part_m);
@@ -1320,6 +1323,41 @@ __global__ void k_diag_scale(int nc, int ncp, const double* A, const CoarseBlk* 
   }
 }
 
+// What a coarse correction's rounding does to the residual, per subdomain: the
+// mean diagonal entry of K over its free DOFs times its part of the trace of the
+// coarse inverse (orthonormal modes); infinite where a diagonal entry of the
+// inverse is not positive.  Warp per subdomain, fixed order.
+__global__ void k_reach(int n_sub, const int* sub_ptr, const int* sub_node, const float4* geo,
+                        const float* __restrict__ dinv, const CoarseBlk* blk, const int* sub_blk,
+                        const float* __restrict__ B, const double* __restrict__ scale, double* reach) {
+  const int lane = threadIdx.x & 31;
+  const int nw = (gridDim.x * blockDim.x) >> 5;
+  for (int I = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; I < n_sub; I += nw) {
+    float k = 0.f, cnt = 0.f;
+#pragma unroll 4
+    for (int t = sub_ptr[I] + lane; t < sub_ptr[I + 1]; t += 32) {
+      const int a = sub_node[t];
+      const unsigned m = geo_bits(geo[a]);
+      for (int d = 0; d < 3; ++d)
+        if ((m >> d) & 1u) {
+          k += 1.f / dinv[3 * a + d];
+          cnt += 1.f;
+        }
+    }
+    k = warp_sum(k);
+    cnt = warp_sum(cnt);
+    if (lane == 0) {
+      const CoarseBlk K = blk[sub_blk[I]];
+      double s = 0.0;
+      for (int i = 6 * I; i < 6 * I + 6; ++i) {
+        const double b = B[K.off + (size_t)(i - K.u0) * (K.p + 1)];
+        if (scale[i] > 0.0) s += b > 0.0 ? scale[i] * scale[i] * b : 1.0 / 0.0;
+      }
+      reach[I] = cnt > 0.f ? s * (double)(k / cnt) : 0.0;
+    }
+  }
+}
+
 // coarse operator and its inverse from the assembled FP64 node-block matrix
 int build_operator(axia_ctx* ctx, CoarseState* S) {
   CoarseArgs& A = S->args;
@@ -1375,42 +1413,16 @@ int build_operator(axia_ctx* ctx, CoarseState* S) {
   }
   ctx->launches++;
   AXIA_CUDA(ctx, cudaGetLastError());
-  return read_status(ctx, "coarse operator is not positive definite");
-}
-
-// What a coarse correction's rounding does to the residual, per subdomain: the
-// mean diagonal entry of K over its free DOFs times its part of the trace of the
-// coarse inverse (orthonormal modes); infinite where a diagonal entry of the
-// inverse is not positive.  Warp per subdomain, fixed order.
-__global__ void k_reach(int n_sub, const int* sub_ptr, const int* sub_node, const float4* geo,
-                        const float* __restrict__ dinv, const CoarseBlk* blk, const int* sub_blk,
-                        const float* __restrict__ B, const double* __restrict__ scale, double* reach) {
-  const int lane = threadIdx.x & 31;
-  const int nw = (gridDim.x * blockDim.x) >> 5;
-  for (int I = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; I < n_sub; I += nw) {
-    float k = 0.f, cnt = 0.f;
-#pragma unroll 4
-    for (int t = sub_ptr[I] + lane; t < sub_ptr[I + 1]; t += 32) {
-      const int a = sub_node[t];
-      const unsigned m = geo_bits(geo[a]);
-      for (int d = 0; d < 3; ++d)
-        if ((m >> d) & 1u) {
-          k += 1.f / dinv[3 * a + d];
-          cnt += 1.f;
-        }
-    }
-    k = warp_sum(k);
-    cnt = warp_sum(cnt);
-    if (lane == 0) {
-      const CoarseBlk K = blk[sub_blk[I]];
-      double s = 0.0;
-      for (int i = 6 * I; i < 6 * I + 6; ++i) {
-        const double b = B[K.off + (size_t)(i - K.u0) * (K.p + 1)];
-        if (scale[i] > 0.0) s += b > 0.0 ? scale[i] * scale[i] * b : 1.0 / 0.0;
-      }
-      reach[I] = cnt > 0.f ? s * (double)(k / cnt) : 0.0;
-    }
+  if (std::find(S->reducible.begin(), S->reducible.end(), 1) != S->reducible.end()) {
+    if (!S->reach) AXIA_TRY(dev_alloc(ctx, &S->reach, (size_t)n_sub));
+    k_reach<<<grid_for(ctx, (int64_t)n_sub * 32, 128), 128, 0, ctx->stream>>>(
+        n_sub, S->sub_ptr, S->sub_node, A.geo, ctx->d_bdinv32, S->d_blk, S->d_sub_blk, S->a32, S->scale, S->reach);
+    ctx->launches++;
+    AXIA_CUDA(ctx, cudaGetLastError());
+    S->h_reach.resize(n_sub);
+    AXIA_TRY(copy_to_host(ctx, S->h_reach.data(), S->reach, (size_t)n_sub));
   }
+  return read_status(ctx, "coarse operator is not positive definite");
 }
 
 // The limit of a mesh's summed reach.  FP32 rounds what the correction adds to
@@ -1428,27 +1440,15 @@ constexpr double FP32_REACH = 5e5;
 // Automatic size, after build_operator returned st: marks in `few` the meshes
 // out of FP32's reach (a pivot that was not positive, without such a mesh: all);
 // true when that is any.
-bool mark_few(axia_ctx* ctx, CoarseState* S, int st, std::vector<char>& few) {
-  const size_t nm = S->reducible.size();
-  if ((st != AXIA_OK && st != AXIA_ERR_ZERO_PIVOT) ||
-      std::find(S->reducible.begin(), S->reducible.end(), 1) == S->reducible.end())
-    return false;
-  const int n_sub = S->args.n_sub;
-  double* d_reach = nullptr;
-  std::vector<double> reach(n_sub);
-  if (dev_alloc(ctx, &d_reach, (size_t)n_sub) != AXIA_OK) return false;
-  k_reach<<<grid_for(ctx, (int64_t)n_sub * 32, 128), 128, 0, ctx->stream>>>(
-      n_sub, S->sub_ptr, S->sub_node, S->geo, ctx->d_bdinv32, S->d_blk, S->d_sub_blk, S->a32, S->scale, d_reach);
-  ctx->launches++;
-  const int cst = copy_to_host(ctx, reach.data(), d_reach, (size_t)n_sub);
-  dev_release(ctx, d_reach);
-  if (cst != AXIA_OK) return false;
+bool mark_few(const CoarseState* S, int st, std::vector<char>& few) {
+  if (st != AXIA_OK && st != AXIA_ERR_ZERO_PIVOT) return false;
   bool any = false;
   for (int pass = 0; pass < (st == AXIA_OK ? 1 : 2) && !any; ++pass)
-    for (size_t k = 0; k < nm; ++k) {
+    for (size_t k = 0; k < S->reducible.size(); ++k) {
+      if (!S->reducible[k]) continue;
       double sum = 0.0;
-      for (int I = S->mesh_sub[k]; I < S->mesh_sub[k + 1]; ++I) sum += reach[I];
-      if (S->reducible[k] && (pass || !(sum <= FP32_REACH))) any = few[k] = 1;
+      for (int I = S->mesh_sub[k]; I < S->mesh_sub[k + 1]; ++I) sum += S->h_reach[I];
+      if (pass || !(sum <= FP32_REACH)) any = few[k] = 1;
     }
   return any;
 }
@@ -1505,7 +1505,7 @@ int coarse_prepare(axia_ctx* ctx, int nodes_target, CoarseArgs* out, bool per_me
       retry = nodes_target == 0 && fewer < DEFAULT_SUBDOMAIN_STEPS;
       ++fewer;
     } else {
-      retry = mark_few(ctx, S, st, few);
+      retry = mark_few(S, st, few);
     }
     if (st == AXIA_OK && !retry) {
       S->op_gen = ctx->assemble_gen;
