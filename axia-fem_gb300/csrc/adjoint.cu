@@ -136,7 +136,7 @@ element_energy_kernel(int64_t n_elem, const int32_t* __restrict__ conn, const do
 
 // C3D8 with 2 x 2 x 2 points: the form from the element's trilinear structure,
 // lane (element, field) for the derivatives, then lane (element, point).  FP64
-// instructions bound it (one per SM about every 16 cycles): summing eight nodes
+// instructions bound it (one per SM about every 18 cycles): summing eight nodes
 // per point took 1.10 ms for 250,000 elements with u = v, this form 0.48
 // (bitwise independent of the element's place in the batch).
 // SAME: u and v are one vector, whose terms are formed once.

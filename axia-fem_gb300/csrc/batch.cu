@@ -327,7 +327,7 @@ struct BatchState {
 };
 
 struct MultiArgs {
-  const int* order;     // [n_nodes] block rows in the order the SpMV takes them (batch_row_order)
+  const int* order;     // [n_nodes] block rows in the order the SpMV takes them (ensure_row_order)
   BsrMatM<float> M32;
   BsrMatM<double> M64;
   int nd;

@@ -163,10 +163,10 @@ __device__ __forceinline__ bool grid_sync(GridBarrier* bar, DevStatus* st, unsig
 
 // Grid-wide barrier that also reduces.  Every block has stored its partials of
 // nv <= 2 values at partials[(slot0 + k) * nblk + rank]; the last block to
-// arrive sums them (one L2 round trip; thread t takes blocks t, t +
-// blockDim.x, ..., then warps and the warp sums in order: a fixed order, so
-// every run gives the same bits) and publishes totals[slot0 + k] before it
-// releases the others.  Same bounded wait as grid_sync.
+// arrive sums them (one L2 round trip; one warp up to 160 blocks, else `used`
+// warps, thread t taking blocks t, t + 32 used, ..., then the warp sums: a fixed
+// order, so every run gives the same bits) and publishes totals[slot0 + k]
+// before it releases the others.  Same bounded wait as grid_sync.
 //
 // What an iteration needs from the totals (step lengths, norms, branch flags)
 // is computed by `fn(totals)` on thread 0 of every block, which leaves it in

@@ -7,7 +7,9 @@
 // with the r.r and r.z partial sums, and the p update.  The two reductions are
 // reduce-and-sync grid barriers (the last block to arrive sums all block
 // partials in a fixed order and publishes the totals), the p update ends with
-// a plain grid barrier; every wait is bounded.  Every block sees the same
+// a plain grid barrier, every wait of them bounded; a small system runs as one
+// thread-block cluster on the hardware's cluster barrier, which all its blocks
+// reach (no block leaves the loop alone).  Every block sees the same
 // totals, takes the same branch, and results are bitwise reproducible.
 //
 // SpMV: L lanes per CSR row (vectorised CSR), matrix values and column

@@ -216,9 +216,6 @@ struct CgScalars {
   int stop;                      // converged
 };
 
-__device__ __forceinline__ double total(const double* totals, int slot) { return __ldcg(totals + slot); }
-
-
 // The scalar steps of the FP32 CG with FP64 reliable updates, on thread 0 of
 // each block.  beta is r.z (new) / r.z (old), with the replaced r after an update.
 __device__ __forceinline__ void mixed_limit(CgScalars<float>& S, double tol, double delta) {
