@@ -532,8 +532,8 @@ __global__ void k_scale_to_f32(const CoarseBlk* blk, const double* A, const doub
 // tile in and out, 64 KB from and to L2 for 2 x 64^3 flops) and the latencies of
 // the panel, the look-ahead and the barriers.  3072 unknowns: 2.98 ms with
 // mirrored tiles, transposed operand loads, three barriers and the 64 pivots of
-// a tile unrolled in one warpgroup; 1.76 in this form, 1.52 with the next
-// tile's operands requested before the product.
+// a tile unrolled in one warpgroup; 1.70 in this form with the next tile's
+// operands requested before the product (0.24 more without).
 // ---------------------------------------------------------------------------
 constexpr int GJ_LD = GJ_T + 4;   // shared-memory row stride (16-byte aligned rows)
 constexpr int GJ_S = 16;          // pivots per step inside a tile
@@ -1427,15 +1427,18 @@ int build_operator(axia_ctx* ctx, CoarseState* S) {
 
 // The limit of a mesh's summed reach.  FP32 rounds what the correction adds to
 // K p at about 6e-8 of |K| |p|, so the noise it leaves in the residual is 6e-8
-// of the reach: 3 % at the limit.  Slender, thin and folded meshes pass it, the
-// more so the more subdomains they have; compact blocks stay below 1e5.
-// Measured on 114 slender, thin, folded and hollow shapes under several loads,
-// 1e-3 to 1e-8, the default count against few_subdomains: below 5e5 (58 shapes)
-// fewer iterations in 606 solves, more in 18, solved only by the one in 16 and
-// only by the other in 11; from 5e5 on 126, 18, 12 and 53.  Axial loads,
-// iterations with few_subdomains / the default: bar 90x10x10 (4.3e5) to 1e-8 107 /
-// 65, 120x12x12 (7.7e5) to 1e-8 136 / NaN, 128x8x8 (1.9e6) to 1e-6 68 / not converged.
-constexpr double FP32_REACH = 5e5;
+// of the reach: 1.2 % at the limit, about the smaller of the usual inner
+// tolerances.  Slender, thin and folded meshes pass it, the more so the more
+// subdomains they have; compact blocks stay below 3e4.
+// Measured on 89 slender, thin and hollow shapes under several loads, 1e-4 to 1e-8,
+// the default count against few_subdomains, inner tolerance 0.1 (and 0.01): below
+// 2e5 fewer iterations in 464 (355) solves, more in 14 (1), solved only by the one
+// in 4 (4) and only by the other in 3 (14); from 2e5 on 242 (158), 21 (15), 16 (9) and
+// 55 (40).  Limits of 5e4 to 1e6 leave 633 to 639 of 1,476 solves unsolved (859 to
+// 883), none 674 (895).  Axial loads, iterations with few_subdomains / the default:
+// bar 70x10x10 (1.7e5) to 1e-8 93 / 66, 120x12x12 (7.7e5) to 1e-8 136 / NaN, 128x8x8
+// (1.9e6) to 1e-6 68 / not converged.
+constexpr double FP32_REACH = 2e5;
 
 // Automatic size, after build_operator returned st: marks in `few` the meshes
 // out of FP32's reach (a pivot that was not positive, without such a mesh: all);

@@ -30,20 +30,24 @@ def _axial(m):
     return f
 
 
-@pytest.mark.parametrize("shape,rtol,few", [
-    ((120, 12, 12), 1e-8, True), ((132, 12, 12), 1e-8, True), ((144, 12, 12), 1e-6, True), ((128, 8, 8), 1e-6, True),
-    ((112, 8, 8), 1e-8, True), ((140, 10, 10), 1e-6, True), ((60, 60, 1), 1e-5, True),
-    ((90, 10, 10), 1e-8, False), ((48, 4, 4), 1e-8, False), ((40, 40, 4), 1e-8, False), ((40, 8, 8), 1e-8, False)])
-def test_bars_and_plates(gpu_ctx, shape, rtol, few):
+# (the longest bars are beyond FP32 with updates only every factor 100, whatever the subdomains)
+@pytest.mark.parametrize("shape,rtol,inner,few", [
+    ((120, 12, 12), 1e-8, 0.1, True), ((132, 12, 12), 1e-8, 0.1, True), ((144, 12, 12), 1e-6, 0.1, True),
+    ((128, 8, 8), 1e-6, 0.1, True), ((112, 8, 8), 1e-8, 0.1, True), ((140, 10, 10), 1e-6, 0.1, True),
+    ((60, 60, 1), 1e-5, 0.1, True), ((90, 10, 10), 1e-8, 0.1, True), ((72, 8, 8), 1e-8, 0.1, True),
+    ((72, 8, 8), 1e-8, 0.01, True), ((80, 8, 8), 1e-8, 0.01, True), ((70, 10, 10), 1e-8, 0.1, False),
+    ((40, 4, 4), 1e-8, 0.1, False), ((40, 40, 4), 1e-8, 0.01, False), ((40, 8, 8), 1e-8, 0.01, False)])
+def test_bars_and_plates(gpu_ctx, shape, rtol, inner, few):
     m = meshgen.cantilever_c3d8(*shape)
     K, f, free = _assemble(gpu_ctx, m), _axial(m), m.free_mask()
-    u, info = gpu_ctx.solve(f, rtol=rtol, **MIXED)
+    kw = dict(MIXED, inner_rtol=inner)
+    u, info = gpu_ctx.solve(f, rtol=rtol, **kw)
     assert np.linalg.norm(K @ u[free] - f[free]) <= 1.01 * rtol * np.linalg.norm(f[free])
     assert (gpu_ctx.coarse_size()[0] <= m.n_nodes / 500 * 1.2) == few
     # the next assembly keeps the size
     n_sub = gpu_ctx.coarse_size()[0]
     gpu_ctx.assemble_ex(_lib.ASM_BSR64 | _lib.ASM_BSR32)
-    again, _ = gpu_ctx.solve(f, rtol=rtol, **MIXED)
+    again, _ = gpu_ctx.solve(f, rtol=rtol, **kw)
     assert gpu_ctx.coarse_size()[0] == n_sub and np.array_equal(u, again)
 
 
