@@ -104,16 +104,16 @@ class ClockSampler:
 
 
 # DRAM bytes per algorithmic byte of pcg_bsr_reliable_kernel<8, 4>, from the ncu
-# capture of the same kernel on the 60^3 block (75.49 GB over 300 iterations
-# against 273.5 MB of algorithmic bytes per iteration; the matrix, padding
+# capture of the same kernel on the 60^3 block (221.84 GB over 885 iterations and
+# 5 FP64 updates against 244.36 GB of algorithmic bytes; the matrix, padding
 # included, is streamed once per iteration and the CG vectors stay in L2);
 # scaled to a launch here by its algorithmic bytes (traffic grows with the
 # iteration count and the matrix size).
-MIXED_TRAFFIC_PER_ALG_BYTE = 0.920
+MIXED_TRAFFIC_PER_ALG_BYTE = 0.908
 # the same for pcg_bsr_reliable_kernel<8, 4, true> (two-level), from its ncu
-# capture on the 60^3 block (52.73 GB over 198 iterations and 5 FP64 updates
-# against 57.48 GB of algorithmic bytes, 64 subdomains)
-COARSE_TRAFFIC_PER_ALG_BYTE = 0.919
+# capture on the 60^3 block (34.94 GB over 119 iterations and 5 FP64 updates
+# against 37.47 GB of algorithmic bytes, 343 subdomains)
+COARSE_TRAFFIC_PER_ALG_BYTE = 0.932
 
 
 def spmv_bytes(nnz, n, vbytes):
@@ -942,7 +942,7 @@ def main():
     ms_rec, _ = Timer(torch, stream)(recover, 3, 10)
     rec_bytes = recover_bytes(model.n_elem, model.nn, nn_)
     recovery = {"ms": ms_rec, "bytes": rec_bytes, "gbs": rec_bytes / (ms_rec * 1e-3) / 1e9,
-                "kernels": "element_recover_kernel<8,8> + k_recover_nodes",
+                "kernels": "element_recover_hex8_kernel + k_recover_nodes",
                 "bound": "fp64 pipe (about 7 kFLOP per C3D8 element)"}
 
     # accuracy: mixed vs FP64 solution, both with true FP64 residual <= 1e-10 ||b||, and both

@@ -131,8 +131,9 @@ typedef struct axia_solve_opts {
   int32_t spmv_vec;        /* node-block form: blocks per lane load (1, 2, 4; 0 = automatic) */
   int32_t preconditioner;  /* axia_preconditioner (0 = Jacobi) */
   int32_t coarse_nodes;    /* AXIA_PRECOND_COARSE: nodes per subdomain (0 = chosen by the mesh: about
-                              0.46 nodes^0.55 subdomains, more for denser rows, 512 at most; at most
-                              682 subdomains per system, in a multi-mesh solve per mesh) */
+                              0.46 nodes^0.55 subdomains, more for denser rows, 512 at most, fewer for
+                              slender and thin meshes; at most 682 subdomains per system, in a
+                              multi-mesh solve per mesh) */
   int32_t krylov;          /* axia_krylov: batched load cases only (0 = one recurrence per case) */
   int32_t reserved;        /* zero */
 } axia_solve_opts;
@@ -239,7 +240,8 @@ AXIA_API int32_t axia_gpu_solve(axia_ctx* ctx, const double* f_full, double* u_f
                        const axia_solve_opts* opts, axia_solve_info* info);
 
 /* Same with f_full and u_full in device memory (for callers that keep the
- * load and displacement vectors resident on the GPU). */
+ * load and displacement vectors resident on the GPU).  A load that is not
+ * finite is AXIA_ERR_NONFINITE here too, found in its norm. */
 AXIA_API int32_t axia_gpu_solve_device(axia_ctx* ctx, const double* f_full_dev, double* u_full_dev,
                               const axia_solve_opts* opts, axia_solve_info* info);
 
