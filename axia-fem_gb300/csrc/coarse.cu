@@ -59,6 +59,8 @@ struct CoarseState {
   std::vector<char> reducible;   // [n_meshes] few_subdomains is less than its subdomains now
   double* reach = nullptr;       // [n_sub] k_reach, with a reducible mesh
   std::vector<double> h_reach;   // of the last operator
+  CoarseState* other = nullptr;  // automatic size: the default space beside the one with few, or the reverse
+  int64_t gen = 0;               // ctx->coarse_gen while this space is the one in use
   bool row_overflow = false;     // a node row reaches more subdomains than its item list holds
   bool per_mesh = false;         // one block per mesh
   std::vector<CoarseBlk> blk;
@@ -1436,7 +1438,7 @@ int build_operator(axia_ctx* ctx, CoarseState* S) {
 // in 4 (4) and only by the other in 3 (14); from 2e5 on 242 (158), 21 (15), 16 (9) and
 // 55 (40).  Limits of 5e4 to 1e6 leave 633 to 639 of 1,476 solves unsolved (859 to
 // 883), none 674 (895).  Axial loads, iterations with few_subdomains / the default:
-// bar 70x10x10 (1.7e5) to 1e-8 93 / 66, 120x12x12 (7.7e5) to 1e-8 136 / NaN, 128x8x8
+// bar 70x10x10 (1.7e5) to 1e-8 101 / 67, 120x12x12 (7.7e5) to 1e-8 136 / NaN, 128x8x8
 // (1.9e6) to 1e-6 68 / not converged.
 constexpr double FP32_REACH = 2e5;
 
@@ -1458,12 +1460,19 @@ bool mark_few(const CoarseState* S, int st, std::vector<char>& few) {
 
 }  // namespace
 
+static void release_state(axia_ctx* ctx, CoarseState*& S) {
+  if (!S) return;
+  S->release(ctx);
+  delete S;
+  S = nullptr;
+}
+
 void coarse_release(axia_ctx* ctx) {
   auto* S = static_cast<CoarseState*>(ctx->coarse);
   if (!S) return;
   if (ctx->stream) cudaStreamSynchronize(ctx->stream);
-  S->release(ctx);
-  delete S;
+  release_state(ctx, S->other);
+  release_state(ctx, S);
   ctx->coarse = nullptr;
 }
 
@@ -1479,45 +1488,61 @@ int coarse_prepare(axia_ctx* ctx, int nodes_target, CoarseArgs* out, bool per_me
     coarse_release(ctx);
     S = nullptr;
   }
-  int fewer = S ? S->fewer : 0;
-  std::vector<char> few;
-  if (S) few = S->few;
-  for (;;) {
-    if (!S) {
-      S = new CoarseState();
-      S->nodes_target = nodes_target;
-      S->per_mesh = per_mesh;
-      S->fewer = fewer;
-      S->few = few;
-      ++ctx->coarse_gen;
-      ctx->coarse = S;
-      const int st = build_space(ctx, S);
-      if (st) {
-        coarse_release(ctx);
-        return st;
-      }
-      few = S->few;
+  if (!S || S->op_gen != ctx->assemble_gen) {
+    // The matrix at hand decides, not an earlier one: the operator of the default
+    // space is built for every assembly, and a space with fewer subdomains, kept
+    // beside it, takes over where the default one is out of FP32's reach.
+    auto use = [&](CoarseState* A, CoarseState* B) {
+      A->other = B;
+      if (B) B->other = nullptr;
+      ctx->coarse = S = A;
+      ctx->coarse_gen = A->gen;
+      A->op_gen = ctx->assemble_gen;
+    };
+    auto is_few = [](const CoarseState* A) { return std::find(A->few.begin(), A->few.end(), 1) != A->few.end(); };
+    CoarseState *D = S, *F = S ? S->other : nullptr;
+    if (S && is_few(S)) std::swap(D, F);
+    if (S) S->other = nullptr;
+    ctx->coarse = nullptr;  // both are D's and F's until one is in use
+    auto give_up = [&](int st) {
+      if (ctx->stream) cudaStreamSynchronize(ctx->stream);
+      release_state(ctx, D);
+      release_state(ctx, F);
+      return st;
+    };
+    auto make = [&](CoarseState*& A, int fewer, const std::vector<char>& few) {
+      A = new CoarseState();
+      A->nodes_target = nodes_target;
+      A->per_mesh = per_mesh;
+      A->fewer = fewer;
+      A->few = few;
+      A->gen = ++ctx->coarse_count;
+      return build_space(ctx, A);
+    };
+    int st = AXIA_OK;
+    for (int fewer = D ? D->fewer : 0;; ++fewer) {
+      if (!D && (st = make(D, fewer, {}))) return give_up(st);
+      st = build_operator(ctx, D);
+      // a node row reaches more subdomains than an item list holds (very flat
+      // elements, hub nodes): larger ones, with the automatic size
+      if (!D->row_overflow || nodes_target > 0 || fewer >= DEFAULT_SUBDOMAIN_STEPS) break;
+      give_up(st);  // a half-built operator is not reused
+      ctx->last_error.clear();
     }
-    if (S->op_gen == ctx->assemble_gen) break;
-    const int st = build_operator(ctx, S);
-    // The automatic size falls back to larger subdomains where a node row
-    // reaches more of them than an item list holds (very flat elements, hub
-    // nodes) and where the correction is out of FP32's reach.
-    bool retry = false;
-    if (S->row_overflow) {
-      retry = nodes_target == 0 && fewer < DEFAULT_SUBDOMAIN_STEPS;
-      ++fewer;
+    std::vector<char> few(D->reducible.size(), 0);
+    if (D->row_overflow || !mark_few(D, st, few)) {
+      if (st) return give_up(st);
+      use(D, F);
     } else {
-      retry = mark_few(S, st, few);
+      ctx->last_error.clear();
+      if (F && F->few != few) {
+        if (ctx->stream) cudaStreamSynchronize(ctx->stream);
+        release_state(ctx, F);
+      }
+      if (!F && (st = make(F, D->fewer, few))) return give_up(st);
+      if ((st = build_operator(ctx, F))) return give_up(st);
+      use(F, D);
     }
-    if (st == AXIA_OK && !retry) {
-      S->op_gen = ctx->assemble_gen;
-      break;
-    }
-    coarse_release(ctx);  // a half-built operator is not reused
-    S = nullptr;
-    if (!retry) return st;
-    ctx->last_error.clear();
   }
   // arrival counters of the restriction (a stopped solve may leave them set)
   AXIA_CUDA(ctx, cudaMemsetAsync(S->cnt, 0, (size_t)S->args.n_sub * sizeof(int), ctx->stream));

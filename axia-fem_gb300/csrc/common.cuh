@@ -409,7 +409,8 @@ struct axia_ctx {
   int multi_grid = 0, multi_lanes = 0, multi_vec = 0;
   bool multi_coarse = false;          // groups planned for the two-level kernel
   int64_t graph_coarse = -1;    // coarse space the captured graph reads (its coarse_gen; -1: diagonal only)
-  int64_t coarse_gen = 0;       // coarse spaces built so far (a new space gets new device arrays)
+  int64_t coarse_gen = 0;       // number of the coarse space in use (each has device arrays of its own)
+  int64_t coarse_count = 0;     // coarse spaces built so far
   int tuned_lanes = 0, tuned_vec = 0;  // node-block layout chosen by axia_gpu_autotune (0: none)
   int tuned_btc = 0, tuned_btu = 0;    // batched-kernel tile chosen by axia_gpu_autotune_batched (0: none)
   void* multi_graph = nullptr;        // cudaGraphExec_t

@@ -96,3 +96,33 @@ def test_one_slender_mesh_of_a_family(gpu_ctx):
     assert alone[1] <= ms[1].n_nodes / 500 < total
     # the mean row length of the family shifts a count by one box or so
     assert abs(total - sum(alone)) <= 0.35 * sum(alone)
+
+
+def test_each_matrix_decides_for_itself(gpu_ctx):
+    """Density designs of one bar, in reach of FP32 and, with a soft root, out of
+    it: a design's subdomains and solution do not depend on the designs before it."""
+    m = meshgen.simp_beam(48, 8, 8)
+    x = m.coords[:, 0]
+    f = np.zeros(m.ndof)
+    f[0::3] = x > x.max() - 1e-9
+    designs = np.ones((2, m.n_elem))
+    designs[1, m.coords[m.conn].mean(axis=1)[:, 0] < 8.0] = 0.4
+
+    def solve(k):
+        u, _, info = gpu_ctx.compliance_forward(designs[k], 3.0, 1.0, f, **dict(MIXED, rtol=1e-6))
+        return u, info.iters, gpu_ctx.coarse_size()[0]
+
+    def fresh():
+        gpu_ctx.setup(m)
+        gpu_ctx.assemble_ex(_lib.ASM_BSR64 | _lib.ASM_BSR32)
+
+    alone = []
+    for k in (0, 1):
+        fresh()
+        alone.append(solve(k))
+    assert alone[1][2] < alone[0][2]  # the second takes fewer subdomains
+    fresh()
+    for k in (0, 1, 1, 0, 1, 0, 0):
+        u, iters, n_sub = solve(k)
+        assert (iters, n_sub) == alone[k][1:]
+        assert np.array_equal(u, alone[k][0])
